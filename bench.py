@@ -534,8 +534,11 @@ def our_launches_per_step(n, d, m):
     8,192 points) bounds, two x (Morton keys, inverse, coordinate gather), cross positions and
     the seed kernel; the pruned search's planning (21, the index-order fallback's two
     included), a second tile build, two search
-    launches and two merges, or one search launch; the local systems and the final sum."""
+    launches and two merges, or one search launch; the local systems and the final sum.  Below the
+    seeded sizes the direct search: scale and one launch."""
     seeded = n >= 8192
+    if not seeded:
+        return 2 + 2
     levels = 0
     p_ = n
     while seeded and p_ >= 8192:

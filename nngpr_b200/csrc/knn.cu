@@ -27,8 +27,9 @@
 //     exactly at merge time and the insertion sequence equals the exact scan's;
 //   * top-M list: M = num_nn rounded up to 8/16/32/64; the M - num_nn leading slots hold -inf
 //     and never move; prefix (fit) searches are triangular and issue the heaviest blocks first.
-// Generic kernel (any d <= 256, any num_nn, float or double): exact distances, query
-// coordinates in shared memory, sorted lists in the workspace.
+// Searches short in queries, and every FP64 search up to 128 neighbours, take the direct kernel
+// (knn_direct.cu).  Generic kernel (any d <= 256, any num_nn, float or double): exact distances,
+// query coordinates in shared memory, sorted lists in the workspace.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -37,6 +38,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "knn_direct.cuh"
 #include "knn_prune.cuh"
 #include "knn_seed.cuh"
 #include "knn_tc.cuh"
@@ -492,21 +494,46 @@ ScreenVariant pick_screen(int D, int M) {
     return ScreenVariant{};
 }
 
-enum class KnnPath { Tc, Simt, Generic };
+// Where the direct search is the faster one: its time is a cost per query (the selection) and per
+// pair (fitted to B200 times of d = 3..28, 500..434,874 refs, 1..100,000 queries), the others' hardly
+// depends on the number of queries while those do not fill the chip.
+//   * Against the tensor-core search below the query count that turns on its seeds: measured 320
+//     us at 500 refs, 800 at 16,599 and 4,400 at 434,874, for 64 to 4,096 queries alike (direct, d = 18:
+//     67 us for 256 queries of 16,599 refs, 126 for 1,000, 305 for 4,096); from there on it is
+//     seeded and measured 550 to 940 us at 16,384 queries (direct: 202 us at d = 3 for a set of
+//     16,384 points over itself, 306 at d = 8, 974 at d = 24 where it loses to 882).
+//   * A larger set searched over itself stays with the seeded and pruned prefix search.
+//   * Against the SIMT screen (num_nn 33..64 or d > 24) up to a query count that falls with d:
+//     m = 48, d = 3: 1.5 against 3.0 ms at 50,000 points, 5.2 against 5.5 at 100,000, 18 against 15 at
+//     200,000; d = 16: 4.3 against 5.3 ms at 50,000, 16 against 11 at 100,000.
+bool direct_pays(int64_t n_ref, int64_t n_query, int d, bool tc_ok) {
+    const double nr = (double)n_ref, nq = (double)n_query, dp = direct::row_len(d);
+    if (!tc_ok) return nq * (dp + 2.0) <= 600000.0;
+    const bool seeded = n_query >= seed::kMinQueries;
+    if (seeded && n_query == n_ref && n_query > seed::kMinQueries) return false;
+    const double us = nq * (2.0 + 0.35 * dp) * 1e-3 + nq * nr * (0.25 + 0.14 * dp) * 1e-6;
+    // (2,500: a row shard of a large prefix search has few queries too, and is seeded)
+    return us <= (seeded ? 700.0 + 0.002 * nr : std::min(550.0 + 0.0085 * nr, 2500.0));
+}
 
-// Search kernel: the tensor-core screen where the shape has a variant (FP32, d <= 24 apart
-// from 9-11 padded to 12 etc., num_nn <= 32), else the SIMT screen, else the generic kernel.  NNGP_KNN_KERNEL=tc|simt|generic forces a
-// kernel where the shape has one (testing and comparisons); unset or any other value selects
-// automatically.
-KnnPath choose_path(int d, int m, bool is_float) {
+enum class KnnPath { Tc, Simt, Generic, Direct };
+
+// Search kernel: NNGP_KNN_KERNEL=tc|simt|generic|direct forces a kernel where the shape has one
+// (testing and comparisons); unset or any other value selects by the rule at direct_pays, then the
+// tensor-core screen where the shape has a variant (FP32, d <= 24 apart from 9-11 padded to 12
+// etc., num_nn <= 32), else the SIMT screen, else the generic kernel.
+KnnPath choose_path(int64_t n_ref, int64_t n_query, int d, int m, bool is_float) {
     const char *env = std::getenv("NNGP_KNN_KERNEL");
     const std::string want = env ? env : "auto";
     const int M = round_m(m), D = round_d(d);
     const bool tc_ok = is_float && D != 0 && M != 0 && M <= 32 && tc_variant(D, M).fn != nullptr;
     const bool simt_ok = is_float && D != 0 && M != 0 && !(M == 64 && D > 16);
+    const bool direct_ok = m <= direct::kMaxNeighbours && n_ref <= (int64_t)1 << 30;
     if (want == "generic") return KnnPath::Generic;
     if (want == "simt") return simt_ok ? KnnPath::Simt : KnnPath::Generic;
     if (want == "tc" && tc_ok) return KnnPath::Tc;
+    if (want == "direct" && direct_ok) return KnnPath::Direct;
+    if (direct_ok && ((!tc_ok && !simt_ok) || direct_pays(n_ref, n_query, d, tc_ok))) return KnnPath::Direct;
     if (tc_ok) return KnnPath::Tc;  // faster than the SIMT screen at every d measured on B200 (3, 8, 16)
     return simt_ok ? KnnPath::Simt : KnnPath::Generic;
 }
@@ -527,7 +554,7 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same) {
     KnnPlan p;
     const int M = round_m(m);
     const int D = round_d(d);
-    p.path = choose_path(d, m, std::is_same<T, float>::value);
+    p.path = choose_path(n_ref, n_query, d, m, std::is_same<T, float>::value);
     if (p.path == KnnPath::Tc) {
         p.tv = tc_variant(D, M);
         p.dp = p.tv.dp;
@@ -537,7 +564,7 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same) {
         p.dp = p.v.dp;
         p.n_ref_pad = (n_ref + p.v.tj - 1) / p.v.tj * p.v.tj;
     } else {
-        p.dp = d;
+        p.dp = p.path == KnnPath::Direct ? direct::row_len(d) : d;
         p.n_ref_pad = n_ref;
     }
     size_t off = 0;
@@ -545,7 +572,7 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same) {
     off = align_up(off + (size_t)p.n_ref_pad * p.dp * sizeof(T), 256);
     p.off_q = same ? p.off_ref : off;
     if (!same) off = align_up(off + (size_t)n_query * p.dp * sizeof(T), 256);
-    if (p.path != KnnPath::Generic) {
+    if (p.path == KnnPath::Tc || p.path == KnnPath::Simt) {
         p.off_rec = off;
         const size_t rec_bytes = p.path == KnnPath::Tc ? (size_t)(p.n_ref_pad / tc::kTcRefTile) * p.tv.stage_bytes
                                                         : (size_t)p.n_ref_pad * p.v.rec_f4 * 16;
@@ -578,7 +605,9 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same) {
                 off = align_up(off + p.prune_ws_bytes, 256);
             }
         }
-    } else {
+    } else if (p.path == KnnPath::Generic || std::is_same<T, double>::value) {
+        // (an FP64 workspace holds the generic kernel's lists too: NNGP_KNN_KERNEL may select it at
+        // the call)
         p.off_ldist = off;
         off = align_up(off + (size_t)n_query * m * sizeof(T), 256);
         p.off_lidx = off;
@@ -637,6 +666,12 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
         scale_pad_kernel<T><<<grid_for(n_query * p.dp), 256, 0, stream>>>(query, n_query, d, p.dp, n_query, lp,
                                                                           use_ls, ls_dev, n_ls, qsc);
         NNGP_CUDA_TRY(cudaGetLastError());
+    }
+    if (p.path == KnnPath::Direct) {
+        if (const char *dbg = std::getenv("NNGP_KNN_DEBUG"); dbg && dbg[0] == '1')
+            std::fprintf(stderr, "nngp_knn: direct path d=%d m=%d queries=%lld refs=%lld seeded=0 pruned=0\n", d, m,
+                         (long long)n_query, (long long)n_ref);
+        return direct::search<T>(refs, n_ref, qsc, n_query, d, m, has_cut, cut, out, stream);
     }
     if (p.path == KnnPath::Tc) {
         if constexpr (std::is_same<T, float>::value) {
