@@ -20,7 +20,7 @@
 //            storing dK (n m^2 n_theta values in the reference).
 //
 // Two kernels:
-//   * warp kernel (m <= 32): one warp per point, lane i owns row i of the factor in registers;
+//   * warp kernel (m <= 32, local_warp.cuh): 8 or 16 lanes per point, its factor's rows in registers;
 //     FP32 with an FP64 re-solve of the system when a pivot is below the threshold (or FP64
 //     throughout for double inputs);
 //   * block kernel (32 < m <= ~150): one CTA per point, the augmented matrix in shared memory,
@@ -29,561 +29,17 @@
 // kernel (deterministic for a given launch shape).
 #include <algorithm>
 #include <cmath>
+#include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <type_traits>
 
 #include "common.cuh"
+#include "local.cuh"
+#include "local_warp.cuh"
 
 namespace nngp {
-
-constexpr int kMaxDimLocal = 256;
-constexpr int kMaxTheta = kMaxDimLocal + 3;
-constexpr int kWarpM = 32;
-constexpr int kLocWarps = 4;
-constexpr double kHalfLog2Pi = 0.91893853320467274178;
-
-struct LocalArgs {
-    double rbf, cst, noise, alpha;
-    double pivot_abs;  // FP32 systems with a pivot below this are re-solved in FP64
-    int64_t n_rows;    // rows of x_ref / y_ref (neighbour index bound)
-    int64_t n_points;
-    int d, ydim, m;
-    int ard;  // 1: per-feature length scales
-    int family;  // stationary part: NNGP_FAMILY_RBF or a Matern (include/nngp_b200.h)
-    int64_t alpha_below;  // alpha goes on the diagonal slots of neighbours with index < alpha_below
-    int weights_out;      // predict: write w = K_nn^-1 k (a.m per point) to `mean` instead of the mean
-    int idx_rbf, idx_const, idx_noise, idx_ls, n_theta;
-    unsigned long long *fp64_count;  // systems re-solved in FP64 are added here (may be null)
-    // fit step with FP32 inputs: bit p marks point p (counted from the launch's first row), whose
-    // FP32 system needs the FP64 re-solve that local_redo_kernel then runs (predict re-solves in
-    // place and leaves this null)
-    uint32_t *redo_bits;
-    // device block of nngp_theta_params (may be null): [rbf, cst, noise, pivot_abs, 1/l_f ...];
-    // when set, the kernels take these values instead of the fields above
-    const double *dev_params;
-    double inv_ls[kMaxDimLocal];
-};
-
-// The hyperparameter values a kernel works with: from the arguments, or from the device block
-// of a theta that never left the device.
-struct Hyp {
-    double rbf, cst, noise, pivot_abs;
-    const double *inv_ls;
-};
-__device__ __forceinline__ Hyp hyp_of(const LocalArgs &a) {
-    if (a.dev_params) {
-        const double *q = a.dev_params;
-        return Hyp{q[0], q[1], q[2], q[3], q + 4};
-    }
-    return Hyp{a.rbf, a.cst, a.noise, a.pivot_abs, a.inv_ls};
-}
-
-template <typename T> __device__ __forceinline__ T dsqrt(T v) { return sqrt(v); }
-template <typename T> __device__ __forceinline__ T drsqrt(T v) { return rsqrt(v); }
-template <> __device__ __forceinline__ float drsqrt<float>(float v) { return rsqrtf(v); }
-template <typename T> __device__ __forceinline__ T dexp(T v) { return exp(v); }
-template <> __device__ __forceinline__ float dexp<float>(float v) { return expf(v); }
-
-// Unit-amplitude stationary part s of the kernel at squared scaled distance sq (formulas of
-// nngpr/batched_kernels.py:1070-1088 for the Matern kernels; RBF exp(-sq / 2)).
-template <bool MATERN, typename T> __device__ __forceinline__ T kern_s(int family, T sq) {
-    if (!MATERN || family == NNGP_FAMILY_RBF) return dexp<T>(T(-0.5) * sq);
-    if (family == NNGP_FAMILY_MATERN12) return dexp<T>(-dsqrt<T>(sq));
-    if (family == NNGP_FAMILY_MATERN32) {
-        const T r = dsqrt<T>(T(3) * sq);
-        return (T(1) + r) * dexp<T>(-r);
-    }
-    const T r = dsqrt<T>(T(5) * sq);
-    return (T(1) + r + r * r / T(3)) * dexp<T>(-r);
-}
-
-// g with d s / d log l_f = g * t_f^2 (t_f the scaled difference of feature f); isotropic:
-// d s / d log l = g * sq.  `s` is kern_s at the same sq.  Reference gradients:
-// nngpr/batched_kernels.py:1108-1120 (Matern), :895-898 (RBF).
-template <bool MATERN, typename T> __device__ __forceinline__ T kern_g(int family, T sq, T s) {
-    if (!MATERN || family == NNGP_FAMILY_RBF) return s;
-    if (family == NNGP_FAMILY_MATERN12) {
-        const T r = dsqrt<T>(sq);
-        return r > T(0) ? s / r : T(0);  // every t_f is 0 where r is
-    }
-    if (family == NNGP_FAMILY_MATERN32) return T(3) * dexp<T>(-dsqrt<T>(T(3) * sq));
-    const T r = dsqrt<T>(T(5) * sq);
-    return T(5) / T(3) * (T(1) + r) * dexp<T>(-r);
-}
-
-// ---------------------------------------------------------------------------------------
-// Warp kernel
-// ---------------------------------------------------------------------------------------
-// Shared memory per warp (bytes): two Cholesky column slots 2 x kWarpM doubles (16-byte
-// aligned, first) | xs (kWarpM + 1) x ds doubles | P kWarpM x (kWarpM + 1) doubles | inverse
-// diagonal kWarpM doubles | gradient accumulator n_theta doubles.  P holds two triangles: the
-// strictly lower part of the factor, L[i][k] at P[i][k] (k < i), and the fill's kernel values
-// of the lower triangle, E[i][k] at P[k][i + 1] (k <= i, so column i + 1 > row k), which the
-// gradient reuses instead of recomputing them.  One array for both halves the footprint of a
-// warp (more resident warps per SM).
-struct WarpSmem {
-    int ds;  // row stride of xs (d + 1; FP32 systems use whole float4s, see warp_system)
-    size_t c_bytes, xs_bytes, l_bytes, idg_bytes, g_bytes, r_bytes, total;
-    size_t xs_off, l_off, idg_off, g_off, r_off;
-    // f32: FP32 inputs, whose systems also keep the fill's squared distances (kWarpM x (kWarpM + 1)
-    // floats) for the gradient instead of recomputing them
-    // sys4: the warp only ever solves FP32 systems (the fit step's FP32 kernel), so the column
-    // slots, xs, P and the inverse diagonal take 4-byte elements
-    __host__ __device__ static WarpSmem make(int d, int n_theta, bool f32 = false, bool sys4 = false) {
-        WarpSmem s;
-        const size_t e = sys4 ? 4 : 8;
-        s.ds = d + 1;
-        s.c_bytes = (size_t)2 * kWarpM * e;
-        s.xs_bytes = sys4 ? (size_t)(kWarpM + 1) * 4 * (((d + 3) / 4) | 1) * 4 : (size_t)(kWarpM + 1) * s.ds * 8;
-        s.l_bytes = (size_t)kWarpM * (kWarpM + 1) * e;
-        s.idg_bytes = (size_t)kWarpM * e;
-        s.g_bytes = (size_t)(n_theta > 0 ? n_theta : 1) * 8;
-        s.xs_off = s.c_bytes;
-        s.l_off = s.xs_off + s.xs_bytes;
-        s.idg_off = s.l_off + s.l_bytes;
-        s.g_off = s.idg_off + s.idg_bytes;
-        s.r_bytes = f32 ? (size_t)kWarpM * (kWarpM + 1) * 4 : 0;
-        s.r_off = s.g_off + s.g_bytes;
-        s.total = (s.r_off + s.r_bytes + 15) / 16 * 16;
-        return s;
-    }
-};
-
-// Vector of VW elements of TC read with one 16-byte shared-memory load.
-template <typename TC> struct Vec16;
-template <> struct Vec16<double> {
-    static constexpr int VW = 2;
-    using T = double2;
-    __device__ static double get(const double2 &v, int e) { return e == 0 ? v.x : v.y; }
-};
-template <> struct Vec16<float> {
-    static constexpr int VW = 4;
-    using T = float4;
-    __device__ static float get(const float4 &v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
-};
-
-// Solves point p's system in precision TC.  Returns false (and commits nothing) when TC is
-// float and a pivot fell below the FP64 threshold.
-template <typename TC, typename TIn, bool GRAD, bool PRED, bool MATERN>
-__device__ __forceinline__ bool warp_system(const LocalArgs &a, int64_t p, int lane, const TIn *__restrict__ x_ref,
-                                            const TIn *__restrict__ y_ref, const TIn *__restrict__ x_pt,
-                                            const TIn *__restrict__ y_pt, const int32_t *__restrict__ nbr,
-                                            unsigned char *wsm, double &ll_acc, TIn *__restrict__ mean,
-                                            TIn *__restrict__ var, int32_t *__restrict__ flags) {
-    constexpr int M = kWarpM;
-    const Hyp h = hyp_of(a);
-    const unsigned FULL = 0xffffffffu;
-    const WarpSmem lay = WarpSmem::make(a.d, a.n_theta, std::is_same<TIn, float>::value,
-                                        std::is_same<TIn, float>::value && !PRED && std::is_same<TC, float>::value);
-    TC *colbuf = reinterpret_cast<TC *>(wsm);  // two column slots of kWarpM, 16-byte aligned
-    TC *xs = reinterpret_cast<TC *>(wsm + lay.xs_off);
-    TC *Ls = reinterpret_cast<TC *>(wsm + lay.l_off);
-    TC *idg = reinterpret_cast<TC *>(wsm + lay.idg_off);
-    double *gacc = reinterpret_cast<double *>(wsm + lay.g_off);
-    constexpr bool STASH = GRAD && !MATERN;  // RBF gradient: reuse the fill's exponentials
-    // FP32 RBF systems also keep the squared distances (the gradient's only other use of the fill)
-    constexpr bool STASH_R = STASH && std::is_same<TC, float>::value && std::is_same<TIn, float>::value;
-    float *Rs = reinterpret_cast<float *>(wsm + lay.r_off);
-    // FP32 rows of xs are whole float4s, an odd number of them (one 16-byte load per 4 features,
-    // rows of different lanes in distinct bank groups), zero padded: the padding adds (0 - 0)^2
-    // terms, so every sum is the same as over the d features alone
-    constexpr bool VEC4 = std::is_same<TC, float>::value;
-    const int d = a.d;
-    const int ds = VEC4 ? 4 * (((d + 3) / 4) | 1) : lay.ds;
-
-    // ---- neighbour of this lane --------------------------------------------------------
-    int32_t j = -1;
-    if (lane < a.m) {
-        j = __ldg(nbr + p * a.m + lane);
-        if (j < -1 || (int64_t)j >= a.n_rows) {
-            flag_or(flags, NNGP_FLAG_BAD_INDEX);
-            j = -1;
-        }
-    }
-    const bool valid = j >= 0;
-    const unsigned vmask = __ballot_sync(FULL, valid);
-
-    // ---- gather scaled coordinates: rows 0..M-1 neighbours, row M the point ------------
-    __syncwarp();
-    for (int f = 0; f < d; ++f) {
-        const TC s = (TC)h.inv_ls[a.ard ? f : 0];
-        xs[lane * ds + f] = valid ? (TC)x_ref[(int64_t)j * d + f] * s : TC(0);
-    }
-    for (int f = lane; f < d; f += 32) xs[M * ds + f] = (TC)x_pt[p * d + f] * (TC)h.inv_ls[a.ard ? f : 0];
-    if (VEC4) {
-        for (int f = d; f < ds; ++f) xs[lane * ds + f] = TC(0);
-        for (int f = d + lane; f < ds; f += 32) xs[M * ds + f] = TC(0);
-    }
-    __syncwarp();
-
-    // ---- fill: squared scaled distances, then kernel values ------------------------------
-    TC r[M];
-    TC rp = TC(0);
-#pragma unroll
-    for (int k = 0; k < M; ++k) r[k] = TC(0);
-    if constexpr (VEC4) {
-        const float4 *xs4 = reinterpret_cast<const float4 *>(xs);
-        const int ds4 = ds / 4, nf4 = (d + 3) / 4;
-        for (int f4 = 0; f4 < nf4; ++f4) {
-            const float4 xi = xs4[lane * ds4 + f4];
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                const float4 xk = xs4[k * ds4 + f4];
-                float t = xi.x - xk.x;
-                r[k] = fmaf(t, t, r[k]);
-                t = xi.y - xk.y;
-                r[k] = fmaf(t, t, r[k]);
-                t = xi.z - xk.z;
-                r[k] = fmaf(t, t, r[k]);
-                t = xi.w - xk.w;
-                r[k] = fmaf(t, t, r[k]);
-            }
-            const float4 xp = xs4[M * ds4 + f4];
-            float t = xi.x - xp.x;
-            rp = fmaf(t, t, rp);
-            t = xi.y - xp.y;
-            rp = fmaf(t, t, rp);
-            t = xi.z - xp.z;
-            rp = fmaf(t, t, rp);
-            t = xi.w - xp.w;
-            rp = fmaf(t, t, rp);
-        }
-    } else {
-        for (int f = 0; f < d; ++f) {
-            const TC xi = xs[lane * ds + f];
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                const TC t = xi - xs[k * ds + f];
-                r[k] = fma(t, t, r[k]);
-            }
-            const TC t = xi - xs[M * ds + f];
-            rp = fma(t, t, rp);
-        }
-    }
-    const TC rbf = (TC)h.rbf, cst = (TC)h.cst;
-    const TC diag_add = (TC)h.noise + ((int64_t)j < a.alpha_below ? (TC)a.alpha : TC(0));
-#pragma unroll
-    for (int k = 0; k < M; ++k) {
-        const bool vk = (vmask >> k) & 1u;
-        const TC e = rbf * kern_s<MATERN>(a.family, r[k]);
-        if (STASH && k <= lane) Ls[k * (M + 1) + lane + 1] = e;  // E[lane][k], upper triangle of P
-        if (STASH_R) Rs[lane * (M + 1) + k] = (float)r[k];
-        TC kv = (valid && vk) ? e + cst : TC(0);
-        if (k == lane) kv = valid ? kv + diag_add : TC(1);
-        r[k] = kv;
-    }
-    const TC ep0 = rbf * kern_s<MATERN>(a.family, rp);  // kept for the gradient
-    TC kvec = valid ? ep0 + cst : TC(0);                 // K[p][lane]
-    const TC kpp = rbf + cst + (TC)h.noise + (PRED ? TC(0) : (TC)a.alpha);
-
-    // ---- Cholesky of the neighbour block fused with l = L^-1 k ----------------------------
-    // A lane's own results (its pivot's reciprocal, l_lane, z_lane, b_lane, v_lane) are not picked
-    // out of the step that produces them: the running value a lane holds stops changing once
-    // its own step is reached, so each is formed once after the loop, from the same operands.
-    TC minpiv = TC(3.0e38);
-    TC ss = TC(0);
-#pragma unroll
-    for (int k = 0; k < M; ++k) {
-        const TC piv = __shfl_sync(FULL, r[k], k);
-        minpiv = fmin(minpiv, piv);
-        const TC inv = drsqrt<TC>(piv);  // 1 / L_kk
-        r[k] = r[k] * inv;               // L_jk, and L_kk = piv * inv on lane k itself
-        if (lane == k) idg[k] = inv;
-        const TC lk = __shfl_sync(FULL, kvec, k) * inv;
-        if (lane > k) kvec = fma(-r[k], lk, kvec);
-        ss = fma(lk, lk, ss);
-        if (k + 1 < M) {
-            // column k of L to a shared slot (alternating slots: a lane that wrote column k has
-            // finished reading column k - 1), then every lane reads L[jj][k], jj > k, as
-            // broadcast 16-byte loads instead of one shuffle per element
-            TC *col = colbuf + (k & 1) * M;
-            col[lane] = r[k];
-            __syncwarp();
-            using V = Vec16<TC>;
-            const typename V::T *cv = reinterpret_cast<const typename V::T *>(col);
-#pragma unroll
-            for (int q = (k + 1) / V::VW; q < M / V::VW; ++q) {
-                const typename V::T v = cv[q];
-#pragma unroll
-                for (int e = 0; e < V::VW; ++e) {
-                    const int jj = q * V::VW + e;
-                    if (jj > k) r[jj] = fma(-r[k], V::get(v, e), r[jj]);
-                }
-            }
-        }
-    }
-    const TC s2 = kpp - ss;
-    if constexpr (std::is_same<TC, float>::value) {
-        if (!(minpiv >= (TC)h.pivot_abs) || !(s2 >= (TC)h.pivot_abs)) return false;  // NaN-safe
-    }
-    if (!(minpiv > TC(0)) || !(s2 > TC(0))) flag_or(flags, NNGP_FLAG_NOT_PD);
-
-    // L (strictly lower part, the upper part of P keeps E) and inverse diagonal to shared
-    // memory for the backward solves
-#pragma unroll
-    for (int k = 0; k < M; ++k)
-        if (k < lane) Ls[lane * (M + 1) + k] = r[k];
-    const TC l_own = kvec * idg[lane];  // l_lane (this lane's own write of idg)
-    __syncwarp();
-
-    if (PRED && a.weights_out) {
-        // conditioning weights w = L^-T l = K_nn^-1 k and the variance term s2 (no outputs yet:
-        // the full-conditioning recursion combines them with earlier predictions)
-        TC bv = l_own;
-#pragma unroll
-        for (int k = M - 1; k >= 0; --k) {
-            const TC bk = __shfl_sync(FULL, bv, k) * idg[k];
-            const TC lkj = Ls[k * (M + 1) + lane];
-            if (lane < k) bv = fma(-lkj, bk, bv);
-        }
-        const TC b_own = bv * idg[lane];
-        if (lane < a.m) mean[p * a.m + lane] = (TIn)b_own;
-        if (lane == 0) var[p] = (TIn)s2;
-        return true;
-    }
-
-    // ---- outputs ------------------------------------------------------------------------
-    TC zw = TC(0);
-    TC wsum = TC(0);
-    double ll = 0.0;
-    for (int c = 0; c < a.ydim; ++c) {
-        TC yv = valid ? (TC)y_ref[(int64_t)j * a.ydim + c] : TC(0);
-#pragma unroll
-        for (int k = 0; k < M; ++k) {
-            const TC zk = __shfl_sync(FULL, yv, k) * idg[k];
-            if (lane > k) yv = fma(-r[k], zk, yv);
-        }
-        const TC z_own = yv * idg[lane];
-        const TC mu = warp_sum(l_own * z_own);
-        if (PRED) {
-            if (lane == 0) mean[p * a.ydim + c] = (TIn)mu;
-        } else {
-            const TC res = (TC)y_pt[p * a.ydim + c] - mu;
-            const double rd = (double)res, sd = (double)s2;
-            ll += -0.5 * rd * rd / sd - 0.5 * log(sd) - kHalfLog2Pi;
-            if (GRAD) {
-                const TC rs = res / s2;
-                zw = fma(rs, z_own, zw);
-                wsum += (res * rs - TC(1)) / (TC(2) * s2);
-            }
-        }
-    }
-    if (PRED) {
-        if (lane == 0) var[p] = (TIn)s2;
-        return true;
-    }
-    if (!GRAD) {
-        if (lane == 0) ll_acc += ll;
-        return true;
-    }
-
-    // ---- adjoint: b = L^-T l, v = L^-T zw ------------------------------------------------
-    TC bv = l_own, vv = zw;
-#pragma unroll
-    for (int k = M - 1; k >= 0; --k) {
-        const TC ik = idg[k];
-        const TC bk = __shfl_sync(FULL, bv, k) * ik;
-        const TC vk = __shfl_sync(FULL, vv, k) * ik;
-        const TC lkj = Ls[k * (M + 1) + lane];
-        if (lane < k) {
-            bv = fma(-lkj, bk, bv);
-            vv = fma(-lkj, vk, vv);
-        }
-    }
-    const TC b_own = bv * idg[lane], v_own = vv * idg[lane];
-
-    // the fill's squared distances: kept (FP32 RBF), else recomputed (xs is intact); rp still
-    // holds the fill's distance to the point itself
-    if constexpr (STASH_R) {
-#pragma unroll
-        for (int k = 0; k < M; ++k) r[k] = (TC)Rs[lane * (M + 1) + k];
-    } else {
-#pragma unroll
-        for (int k = 0; k < M; ++k) r[k] = TC(0);
-        rp = TC(0);
-        for (int f = 0; f < d; ++f) {
-            const TC xi = xs[lane * ds + f];
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                const TC t = xi - xs[k * ds + f];
-                r[k] = fma(t, t, r[k]);
-            }
-            const TC t = xi - xs[M * ds + f];
-            rp = fma(t, t, rp);
-        }
-    }
-    TC g_amp = TC(0), g_cst = TC(0), g_noise = TC(0), g_iso = TC(0);
-#pragma unroll
-    for (int k = 0; k < M; ++k) {
-        const TC bk = __shfl_sync(FULL, b_own, k);
-        const TC vk = __shfl_sync(FULL, v_own, k);
-        const bool vk_ok = (vmask >> k) & 1u;
-        const TC G = wsum * b_own * bk - TC(0.5) * (b_own * vk + v_own * bk);
-        const TC wgt = (valid && vk_ok) ? (k < lane ? TC(2) : (k == lane ? TC(1) : TC(0))) : TC(0);
-        const TC s = STASH ? TC(0) : kern_s<MATERN>(a.family, r[k]);
-        const TC gw = wgt * G;
-        // E[lane][k] for k <= lane (wgt is 0 above the diagonal, where P holds L)
-        const TC ge = gw * (STASH ? (k <= lane ? Ls[k * (M + 1) + lane + 1] : TC(0)) : rbf * s);
-        const TC gl = MATERN ? gw * (rbf * kern_g<MATERN>(a.family, r[k], s)) : ge;
-        g_amp += ge;
-        g_cst += gw;
-        g_iso = fma(gl, r[k], g_iso);
-        if (k == lane && valid) g_noise += G;
-        r[k] = gl;  // kept for the per-feature length-scale terms
-    }
-    // pair (p, lane), weight 2, and (p, p)
-    const TC Gp = valid ? TC(0.5) * v_own - wsum * b_own : TC(0);
-    const TC sp = MATERN ? kern_s<MATERN>(a.family, rp) : TC(0);
-    const TC gpe = TC(2) * Gp * (MATERN ? rbf * sp : ep0);
-    const TC gpl = MATERN ? TC(2) * Gp * (rbf * kern_g<MATERN>(a.family, rp, sp)) : gpe;
-    g_amp += gpe;
-    g_cst += TC(2) * Gp;
-    g_iso = fma(gpl, rp, g_iso);
-    const double amp_t = (double)warp_sum(g_amp) + (double)wsum * h.rbf;
-    const double cst_t = (double)warp_sum(g_cst) + (double)wsum;
-    const double noi_t = (double)warp_sum(g_noise) + (double)wsum;
-    const double iso_t = (double)warp_sum(g_iso);
-    if (lane == 0) {
-        ll_acc += ll;
-        if (a.idx_rbf >= 0) gacc[a.idx_rbf] += amp_t;
-        if (a.idx_const >= 0) gacc[a.idx_const] += h.cst * cst_t;
-        if (a.idx_noise >= 0) gacc[a.idx_noise] += h.noise * noi_t;
-        if (a.idx_ls >= 0 && !a.ard) gacc[a.idx_ls] += iso_t;
-    }
-    if (a.idx_ls >= 0 && a.ard) {
-        for (int f = 0; f < d; ++f) {
-            const TC xi = xs[lane * ds + f];
-            TC acc = TC(0);
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                const TC t = xi - xs[k * ds + f];
-                acc = fma(r[k] * t, t, acc);
-            }
-            const TC t = xi - xs[M * ds + f];
-            acc = fma(gpl * t, t, acc);
-            const double s = (double)warp_sum(acc);
-            if (lane == 0) gacc[a.idx_ls + f] += s;
-        }
-    }
-    __syncwarp();
-    return true;
-}
-
-// Resident CTAs per SM the register budget is set for: the fit step's FP32 kernel (FP32 systems
-// only, 4-byte warp layout) 4, the others 3.
-template <typename TIn, bool PRED> constexpr int kLocMinBlocks = (std::is_same<TIn, float>::value && !PRED) ? 4 : 3;
-
-template <typename TIn, bool GRAD, bool PRED, bool MATERN>
-__global__ void __launch_bounds__(kLocWarps * 32, (kLocMinBlocks<TIn, PRED>)) local_warp_kernel(
-    const __grid_constant__ LocalArgs a, const TIn *__restrict__ x_ref, const TIn *__restrict__ y_ref,
-    const TIn *__restrict__ x_pt, const TIn *__restrict__ y_pt, const int32_t *__restrict__ nbr,
-    double *__restrict__ block_out, TIn *__restrict__ mean, TIn *__restrict__ var, int32_t *__restrict__ flags) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const WarpSmem lay = WarpSmem::make(a.d, a.n_theta, std::is_same<TIn, float>::value,
-                                        std::is_same<TIn, float>::value && !PRED);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char *wsm = smem_raw + warp * lay.total;
-    double *gacc = reinterpret_cast<double *>(wsm + lay.g_off);
-    for (int t = lane; t < a.n_theta; t += 32) gacc[t] = 0.0;
-    __syncwarp();
-    double ll_acc = 0.0;
-    bool used_fp64 = false;
-    unsigned long long n_fp64 = 0;
-    const int64_t nwarps = (int64_t)gridDim.x * kLocWarps;
-    for (int64_t p = (int64_t)blockIdx.x * kLocWarps + warp; p < a.n_points; p += nwarps) {
-        bool done = false;
-        if constexpr (std::is_same<TIn, float>::value) {
-            done = warp_system<float, TIn, GRAD, PRED, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm, ll_acc, mean,
-                                                       var, flags);
-        }
-        if (!done) {
-            if constexpr (std::is_same<TIn, float>::value) {
-                used_fp64 = true;
-                ++n_fp64;
-            }
-            if constexpr (std::is_same<TIn, float>::value && !PRED) {
-                // the fit step's FP32 kernel carries no FP64 system (registers): the point is
-                // marked for local_redo_kernel
-                if (lane == 0) atomicOr(a.redo_bits + (p >> 5), 1u << (p & 31));
-            } else {
-                warp_system<double, TIn, GRAD, PRED, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm, ll_acc, mean,
-                                                             var, flags);
-            }
-        }
-    }
-    if (used_fp64 && lane == 0) {
-        flag_or(flags, NNGP_FLAG_FP64_FALLBACK);
-        if (a.fp64_count) atomicAdd(a.fp64_count, n_fp64);
-    }
-    if (PRED) return;
-    // CTA reduction in fixed order: warp w's totals -> slot w, then warp 0 sums
-    __shared__ double red[kLocWarps];
-    if (lane == 0) red[warp] = ll_acc;
-    __syncthreads();
-    const int nt = 1 + (GRAD ? a.n_theta : 0);
-    double *o = block_out + (int64_t)blockIdx.x * nt;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < kLocWarps; ++w) s += red[w];
-        o[0] = s;
-    }
-    if (GRAD) {
-        for (int t = threadIdx.x; t < a.n_theta; t += blockDim.x) {
-            double s = 0.0;
-            for (int w = 0; w < kLocWarps; ++w)
-                s += reinterpret_cast<const double *>(smem_raw + w * lay.total + lay.g_off)[t];
-            o[1 + t] = s;
-        }
-    }
-}
-
-// FP64 re-solve of the fit-step systems the FP32 kernel marked (warp per point, the same warp
-// layout); the points of a 32-point word go to one warp, words to warps in a fixed order, so the
-// per-CTA partials are deterministic for a given launch shape.
-template <bool GRAD, bool MATERN>
-__global__ void __launch_bounds__(kLocWarps * 32, 3) local_redo_kernel(
-    const __grid_constant__ LocalArgs a, const float *__restrict__ x_ref, const float *__restrict__ y_ref,
-    const float *__restrict__ x_pt, const float *__restrict__ y_pt, const int32_t *__restrict__ nbr,
-    double *__restrict__ block_out, int32_t *__restrict__ flags) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const WarpSmem lay = WarpSmem::make(a.d, a.n_theta, true);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char *wsm = smem_raw + warp * lay.total;
-    double *gacc = reinterpret_cast<double *>(wsm + lay.g_off);
-    for (int t = lane; t < a.n_theta; t += 32) gacc[t] = 0.0;
-    __syncwarp();
-    double ll_acc = 0.0;
-    const int64_t words = (a.n_points + 31) / 32;
-    const int64_t nwarps = (int64_t)gridDim.x * kLocWarps;
-    for (int64_t w = (int64_t)blockIdx.x * kLocWarps + warp; w < words; w += nwarps) {
-        uint32_t bits = a.redo_bits[w];
-        while (bits) {
-            const int64_t p = w * 32 + (__ffs(bits) - 1);
-            bits &= bits - 1;
-            warp_system<double, float, GRAD, false, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm, ll_acc,
-                                                            nullptr, nullptr, flags);
-        }
-    }
-    __shared__ double red[kLocWarps];
-    if (lane == 0) red[warp] = ll_acc;
-    __syncthreads();
-    const int nt = 1 + (GRAD ? a.n_theta : 0);
-    double *o = block_out + (int64_t)blockIdx.x * nt;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < kLocWarps; ++w) s += red[w];
-        o[0] = s;
-    }
-    if (GRAD) {
-        for (int t = threadIdx.x; t < a.n_theta; t += blockDim.x) {
-            double s = 0.0;
-            for (int w = 0; w < kLocWarps; ++w)
-                s += reinterpret_cast<const double *>(smem_raw + w * lay.total + lay.g_off)[t];
-            o[1 + t] = s;
-        }
-    }
-}
 
 // ---------------------------------------------------------------------------------------
 // Block kernel (32 < m): one CTA per point, FP64, augmented matrix in shared memory
@@ -871,6 +327,47 @@ __global__ void finalize_kernel(const double *__restrict__ block_out, int nblock
 // Host side
 // ---------------------------------------------------------------------------------------
 namespace {
+int num_sms();
+size_t block_smem_limit();
+
+// CTAs of a kernel that one SM holds, asked once per kernel, device and launch shape.
+nngp_status resident_ctas(const void *fn, int threads, size_t smem, int *out) {
+    static std::mutex mu;
+    static std::map<std::tuple<const void *, int, int, size_t>, int> known;
+    int dev = 0;
+    NNGP_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(fn, dev, threads, smem);
+    auto it = known.find(key);
+    if (it == known.end()) {
+        int n = 0;
+        NNGP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem));
+        it = known.emplace(key, std::max(n, 1)).first;
+    }
+    *out = it->second;
+    return NNGP_OK;
+}
+}  // namespace
+
+nngp_status warp_launch(const void *fn, size_t warp_bytes, int64_t need_warps, int grid_limit, WarpLaunch *out) {
+    if (warp_bytes > block_smem_limit())
+        return fail(NNGP_ERR_UNSUPPORTED, "the local systems of this d and m need more shared memory than one CTA has");
+    const int sms = num_sms();
+    // few systems: single-warp CTAs, so that no SM takes two warps while another has none
+    out->warps = need_warps <= (int64_t)sms * 4 || 2 * warp_bytes > block_smem_limit() ? 1 : 2;
+    out->smem = out->warps * warp_bytes;
+    NNGP_CUDA_TRY(ensure_smem_limit(fn, (int)out->smem));
+    int per_sm = 1;
+    nngp_status st = resident_ctas(fn, out->warps * 32, out->smem, &per_sm);
+    if (st != NNGP_OK) return st;
+    int64_t grid = std::min<int64_t>((need_warps + out->warps - 1) / out->warps,
+                                     (int64_t)sms * std::min(per_sm, kLocalGridPerSm));
+    if (grid_limit > 0) grid = std::min<int64_t>(grid, grid_limit);
+    out->grid = (int)std::max<int64_t>(1, grid);
+    return NNGP_OK;
+}
+
+namespace {
 
 int num_sms() {
     static int cached = 0;
@@ -890,35 +387,29 @@ constexpr size_t kCountBytes = 256;  // head of the log-likelihood workspace: th
 
 struct LocalPlan {
     bool warp = true;
-    int grid = 0;
-    int redo_grid = 0;  // CTAs of local_redo_kernel (their partials follow the main kernel's)
-    size_t smem = 0;
+    int grid = 0;       // CTAs of the main kernel: of the block kernel, or at most (warp kernel)
+    size_t smem = 0;    // block kernel
     int nt = 1;
     size_t bits_off = 0;  // byte offset of the FP64 re-solve bitmask from the workspace head
     size_t ws_bytes = 0;
 };
 
-// f32: the launch runs the FP32-input kernels (their warp layout keeps the squared distances);
-// sys4: and only FP32 systems (the fit step: 4-byte warp layout)
-LocalPlan plan_local(int64_t n_points, int d, int m, int n_theta, bool grad, bool f32 = false, bool sys4 = false) {
+LocalPlan plan_local(int64_t n_points, int d, int m, int n_theta, bool grad) {
     LocalPlan p;
     p.warp = m <= kWarpM;
     p.nt = 1 + (grad ? n_theta : 0);
     const int sms = num_sms();
     if (p.warp) {
-        p.smem = WarpSmem::make(d, n_theta, f32, sys4).total * kLocWarps;
-        const int64_t need = (n_points + kLocWarps - 1) / kLocWarps;
-        p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 8));
+        p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(n_points, (int64_t)sms * kLocalGridPerSm));
     } else {
         p.smem = BlockSmem::make(m, d).total;
         p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(n_points, (int64_t)sms * 2));
     }
     // [256 bytes: the count of FP64 re-solves | per-CTA partials of the main kernel, then of the
     // re-solve kernel | the re-solve bitmask, one bit per point], plus 256 of alignment slack
-    // (laid out for FP32 inputs whatever the dtype: the workspace size does not depend on it)
     const int64_t words = (n_points + 31) / 32;
-    p.redo_grid = (int)std::max<int64_t>(1, std::min<int64_t>((words + kLocWarps - 1) / kLocWarps, (int64_t)sms * 8));
-    p.bits_off = kCountBytes + align_up((size_t)(p.grid + p.redo_grid) * p.nt * sizeof(double), 256);
+    const int64_t redo_grid = std::max<int64_t>(1, std::min<int64_t>(words, (int64_t)sms * kLocalGridPerSm));
+    p.bits_off = kCountBytes + align_up((size_t)(p.grid + redo_grid) * p.nt * sizeof(double), 256);
     p.ws_bytes = p.bits_off + align_up((size_t)words * sizeof(uint32_t), 256) + 256;
     return p;
 }
@@ -977,21 +468,34 @@ nngp_status fill_args(LocalArgs &a, const nngp_kernel *k, int d, int ydim, int m
 }
 
 template <typename TIn, bool GRAD, bool PRED>
-nngp_status launch_local(const LocalPlan &pl, const LocalArgs &a, const TIn *x_ref, const TIn *y_ref, const TIn *x_pt,
+nngp_status launch_block(const LocalPlan &pl, const LocalArgs &a, const TIn *x_ref, const TIn *y_ref, const TIn *x_pt,
                          const TIn *y_pt, const int32_t *nbr, double *block_out, TIn *mean, TIn *var, int32_t *flags,
                          cudaStream_t stream) {
-    if (pl.warp) {
-        auto fn = a.family == NNGP_FAMILY_RBF ? local_warp_kernel<TIn, GRAD, PRED, false>
-                                              : local_warp_kernel<TIn, GRAD, PRED, true>;
-        NNGP_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(fn), (int)pl.smem));
-        fn<<<pl.grid, kLocWarps * 32, pl.smem, stream>>>(a, x_ref, y_ref, x_pt, y_pt, nbr, block_out, mean, var, flags);
-    } else {
-        auto fn = local_block_kernel<TIn, GRAD, PRED>;
-        NNGP_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(fn), (int)pl.smem));
-        fn<<<pl.grid, kBlkThreads, pl.smem, stream>>>(a, x_ref, y_ref, x_pt, y_pt, nbr, block_out, mean, var, flags);
-    }
+    auto fn = local_block_kernel<TIn, GRAD, PRED>;
+    NNGP_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(fn), (int)pl.smem));
+    fn<<<pl.grid, kBlkThreads, pl.smem, stream>>>(a, x_ref, y_ref, x_pt, y_pt, nbr, block_out, mean, var, flags);
     NNGP_CUDA_TRY(cudaGetLastError());
     return NNGP_OK;
+}
+
+// The fit step's main kernel: *parts per-CTA partial sums of pl.nt values in block_out.
+template <typename TIn>
+nngp_status run_fit(const LocalPlan &pl, const LocalArgs &a, bool grad, const TIn *x_ref, const TIn *y_ref,
+                    const TIn *x_pt, const TIn *y_pt, const int32_t *nbr, double *block_out, int *parts,
+                    int32_t *flags, cudaStream_t stream) {
+    if (pl.warp) return launch_fit<TIn>(a, grad, x_ref, y_ref, x_pt, y_pt, nbr, block_out, pl.grid, parts, flags, stream);
+    *parts = pl.grid;
+    return grad ? launch_block<TIn, true, false>(pl, a, x_ref, y_ref, x_pt, y_pt, nbr, block_out, nullptr, nullptr, flags,
+                                                 stream)
+                : launch_block<TIn, false, false>(pl, a, x_ref, y_ref, x_pt, y_pt, nbr, block_out, nullptr, nullptr,
+                                                  flags, stream);
+}
+
+template <typename TIn>
+nngp_status run_predict(const LocalPlan &pl, const LocalArgs &a, const TIn *x_ref, const TIn *y_ref, const TIn *x_pt,
+                        const int32_t *nbr, TIn *mean, TIn *var, int32_t *flags, cudaStream_t stream) {
+    if (pl.warp) return launch_predict<TIn>(a, x_ref, y_ref, x_pt, nbr, mean, var, flags, stream);
+    return launch_block<TIn, false, true>(pl, a, x_ref, y_ref, x_pt, nullptr, nbr, nullptr, mean, var, flags, stream);
 }
 
 template <typename TIn>
@@ -1014,8 +518,7 @@ nngp_status loglik_impl(const TIn *x, const TIn *y, int64_t n, int d, int ydim, 
         return NNGP_OK;
     }
     if (!x || !y || (m > 0 && !nbr)) return fail(NNGP_ERR_INVALID_ARGUMENT, "loglik: null input pointer");
-    const LocalPlan pl = plan_local(rows, d, m, a.n_theta, grad, std::is_same<TIn, float>::value,
-                                    std::is_same<TIn, float>::value);
+    const LocalPlan pl = plan_local(rows, d, m, a.n_theta, grad);
     if (!ws || ws_bytes < pl.ws_bytes) return fail(NNGP_ERR_WORKSPACE, "loglik: workspace missing or too small");
     unsigned char *head = reinterpret_cast<unsigned char *>(align_up(reinterpret_cast<uintptr_t>(ws), 256));
     a.fp64_count = reinterpret_cast<unsigned long long *>(head);
@@ -1030,22 +533,16 @@ nngp_status loglik_impl(const TIn *x, const TIn *y, int64_t n, int d, int ydim, 
         a.redo_bits = reinterpret_cast<uint32_t *>(head + pl.bits_off);
         NNGP_CUDA_TRY(cudaMemsetAsync(a.redo_bits, 0, (size_t)((rows + 31) / 32) * sizeof(uint32_t), stream));
     }
-    if (grad)
-        st = launch_local<TIn, true, false>(pl, a, x, y, x_pt, y_pt, nbr, block_out, nullptr, nullptr, flags, stream);
-    else
-        st = launch_local<TIn, false, false>(pl, a, x, y, x_pt, y_pt, nbr, block_out, nullptr, nullptr, flags, stream);
+    int parts = 0;
+    st = run_fit<TIn>(pl, a, grad, x, y, x_pt, y_pt, nbr, block_out, &parts, flags, stream);
     if (st != NNGP_OK) return st;
-    int parts = pl.grid;
     if constexpr (std::is_same<TIn, float>::value) {
         if (redo) {
-            double *redo_out = block_out + (size_t)pl.grid * pl.nt;
-            auto fn = a.family == NNGP_FAMILY_RBF ? (grad ? local_redo_kernel<true, false> : local_redo_kernel<false, false>)
-                                                  : (grad ? local_redo_kernel<true, true> : local_redo_kernel<false, true>);
-            const int redo_smem = (int)(WarpSmem::make(d, a.n_theta, true).total * kLocWarps);  // FP64 systems
-            NNGP_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(fn), redo_smem));
-            fn<<<pl.redo_grid, kLocWarps * 32, redo_smem, stream>>>(a, x, y, x_pt, y_pt, nbr, redo_out, flags);
-            NNGP_CUDA_TRY(cudaGetLastError());
-            parts += pl.redo_grid;
+            int redo_parts = 0;
+            st = launch_redo(a, grad, x, y, x_pt, y_pt, nbr, block_out + (size_t)parts * pl.nt,
+                             num_sms() * kLocalGridPerSm, &redo_parts, flags, stream);
+            if (st != NNGP_OK) return st;
+            parts += redo_parts;
         }
     }
     finalize_kernel<<<1, 256, 0, stream>>>(block_out, parts, pl.nt, out);
@@ -1063,8 +560,8 @@ nngp_status predict_impl(const TIn *xt, const TIn *yt, int64_t nt, const TIn *xq
     if (st != NNGP_OK) return st;
     if (nq == 0) return NNGP_OK;
     if (!xq || !mean || !var || (m > 0 && (!nbr || !xt || !yt))) return fail(NNGP_ERR_INVALID_ARGUMENT, "predict: null pointer");
-    const LocalPlan pl = plan_local(nq, d, m, 0, false, std::is_same<TIn, float>::value);
-    return launch_local<TIn, false, true>(pl, a, xt, yt, xq, nullptr, nbr, nullptr, mean, var, flags, stream);
+    const LocalPlan pl = plan_local(nq, d, m, 0, false);
+    return run_predict<TIn>(pl, a, xt, yt, xq, nbr, mean, var, flags, stream);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1288,8 +785,7 @@ nngp_status predict_full_f64(const double *x_full, const double *y_train, int64_
     a.alpha_below = nt;  // alpha on training neighbours only (base_nngpr.py:952-954)
     a.weights_out = 1;
     const LocalPlan pl = plan_local(nq, d, m, 0, false);
-    st = launch_local<double, false, true>(pl, a, x_full, y_train, x_full + nt * d, nullptr, nbr, nullptr, wts, s2,
-                                           flags, stream);
+    st = run_predict<double>(pl, a, x_full, y_train, x_full + nt * d, nbr, wts, s2, flags, stream);
     if (st != NNGP_OK) return st;
     if (samples) {
         sample_recursion_kernel<<<1, 32, 0, stream>>>(nbr, wts, s2, y_train, nt, nq, m, ydim, want_var, z, mean,
@@ -1387,12 +883,10 @@ nngp_status loglik_f64_noalloc(const double *x, const double *y, int64_t n, int 
     if (st != NNGP_OK) return st;
     LocalPlan pl = plan_local(n, d, m, a.n_theta, grad);
     pl.grid = std::min(pl.grid, kStaticBlocks);  // the kernels stride over the points
-    if (grad)
-        st = launch_local<double, true, false>(pl, a, x, y, x, y, nbr, block_out, nullptr, nullptr, flags, stream);
-    else
-        st = launch_local<double, false, false>(pl, a, x, y, x, y, nbr, block_out, nullptr, nullptr, flags, stream);
+    int parts = 0;
+    st = run_fit<double>(pl, a, grad, x, y, x, y, nbr, block_out, &parts, flags, stream);
     if (st != NNGP_OK) return st;
-    finalize_kernel<<<1, 256, 0, stream>>>(block_out, pl.grid, pl.nt, out);
+    finalize_kernel<<<1, 256, 0, stream>>>(block_out, parts, pl.nt, out);
     NNGP_CUDA_TRY(cudaGetLastError());
     return NNGP_OK;
 }
