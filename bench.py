@@ -547,6 +547,8 @@ def our_launches_per_step(n, d, m):
     from nngpr_b200.sharding import search_is_pruned
     pruned = seeded and search_is_pruned(n, d)
     search = (21 + 1 + 2 + 2) if pruned else 1
+    if pruned and d >= 9 and n >= 131072:  # cells: k-means steps, directions, assignment, two reaches
+        search += 10
     return 3 + 9 * levels + search + 2
 
 

@@ -10,6 +10,14 @@
 // (d = 3, n = 434,874: about 125 tiles per group of 128 rows instead of about 1,700 on average)
 // and checks j < i per candidate.
 //
+// In many dimensions boxes exclude little; from 9 features on the rows and refs are also kept in k-means
+// cells, and a tile is dropped as well when the slab between its cell and the group's is wider than the
+// bound allows (knn_cells.cu).  Inside a cell the rows are ordered by their seed first (16 steps of a
+// ninth of a factor of two in the squared distance, then the curve): a group reaches as far as its
+// largest seed, and the few rows in a cluster's tails would make every group reach far.  At d = 16, n = 1M (mixture of 64):
+// 3,282 listed tiles of 7,813 per group with boxes, 834 with cells, 443 with rows ordered by seed; search 68.5 ->
+// 38.9 -> 33.8 ms (32.2 with tile records written 16 bytes at a time).
+//
 // Exactness: the FP32 squared distance the search compares, ((t0^2 + t1^2) + ...) with every
 // step rounded and t_f = fl(x_jf - x_if), is at least (1 - u)^(D + 2) times the exact squared
 // distance of the same FP32 coordinates (all terms are non-negative), minus at most
@@ -33,6 +41,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "knn_cells.cuh"
 #include "knn_prune.cuh"
 
 namespace nngp {
@@ -40,11 +49,19 @@ namespace prune {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kEarlyShift = 3;       // rows below n / 8 take the index-order search
-constexpr int kBands = kEarlyShift + 1;  // band b: rows [n / 2^(b + 1), n / 2^b) (the last only at rounding edges)
+// Rows below n >> shift take the index-order search: n / 8 with boxes alone, n / 64 with cells, whose lists stay
+// short for sparse prefixes too (d = 16, n = 1M: the rows below n / 8 in index order take 4.5 ms, as much
+// as all the others).
+constexpr int kEarlyShift = 3, kEarlyShiftCells = 6;
+constexpr int kBands = 7;  // band b: rows [n / 2^(b + 1), n / 2^b), b = 0 .. shift (the last only at rounding edges)
 constexpr int kLooseLog2Q = 4 * 256;  // seed > 16 x band geometric mean (log2 in 1/256 units)
-constexpr uint64_t kIndexOrderTag = 1ull << 36;  // above (band << 32 | curve position) for bands < 16
-constexpr uint64_t kOutsideTag = 1ull << 37;     // rows outside the searched range: sorted last, not searched
+// Sort keys, 32 bits: curve positions take 21 bits (n <= kMaxPoints), cells 7, bands 3.  Rows: band | cell |
+// position, then the index-order rows, then the rows outside the searched range.  Refs: cell | class |
+// position.
+constexpr int kPosBits = 21, kCellBits = 7;
+static_assert(kMaxPoints <= (1 << kPosBits) && cells::kMaxCells <= (1 << kCellBits) && kBands <= 7, "sort keys");
+constexpr uint32_t kIndexOrderTag = 0x80000000u;  // above every (band, cell, position) for bands < 7
+constexpr uint32_t kOutsideTag = 0xC0000000u;
 // The pruned rows go back to index order when their tile lists hold more tiles than their
 // index-order groups would stream.  Lists that exclude nothing hold about 4/3 of those tiles
 // (a group in curve order needs the tiles up to its largest index, an index-order group up to
@@ -54,9 +71,9 @@ constexpr double kFallbackFrac = 1.0;
 constexpr int kStats = 3 * kBands + 3;  // per band: seed log sums, counts, pruned counts; index-order
                                         // count; sum of the pruned rows' indices; fallback flag
 
-__device__ __forceinline__ int band_of(int64_t i, int64_t n) {
+__device__ __forceinline__ int band_of(int64_t i, int64_t n, int shift) {
     int b = 0;
-    while (b < kBands - 1 && (i << (b + 1)) < n) ++b;  // i < n / 2^(b + 1)
+    while (b < shift && (i << (b + 1)) < n) ++b;  // i < n / 2^(b + 1)
     return b;
 }
 
@@ -105,14 +122,16 @@ __global__ void __launch_bounds__(kThreads) tile_box_kernel(const float *__restr
     }
 }
 
-// Ref order: points sorted by (index class, curve position), class = 3 - band: [0, n/8),
-// [n/8, n/4), [n/4, n/2), [n/2, n).  A tile then holds refs of one class (up to the one tile at
-// each class boundary), so a group of rows of band b skips whole tiles whose refs all come after
-// its rows, and meets refs j > i only in its own class.
-__global__ void __launch_bounds__(kThreads) ref_keys_kernel(int64_t n, const int32_t *__restrict__ pos0,
-                                                            uint64_t *__restrict__ keys, int32_t *__restrict__ vals) {
+// Ref order: points sorted by (cell, index class, curve position), class = shift - band: [0, n >> shift), ...,
+// [n/4, n/2), [n/2, n).  A tile then holds refs of one cell and class (up to the tiles at their
+// boundaries), so a group of rows of band b skips whole tiles whose refs all come after its rows, and
+// meets refs j > i only in its own class.
+__global__ void __launch_bounds__(kThreads) ref_keys_kernel(int64_t n, int shift, const int32_t *__restrict__ pos0,
+                                                            const uint8_t *__restrict__ cell,
+                                                            uint32_t *__restrict__ keys, int32_t *__restrict__ vals) {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
-        keys[j] = (uint64_t)(kBands - 1 - band_of(j, n)) << 32 | (uint32_t)pos0[j];
+        const uint32_t c = cell ? cell[j] : 0u;
+        keys[j] = ((c * 8u + (uint32_t)(shift - band_of(j, n, shift))) << kPosBits) | (uint32_t)pos0[j];
         vals[j] = (int32_t)j;
     }
 }
@@ -120,7 +139,7 @@ __global__ void __launch_bounds__(kThreads) ref_keys_kernel(int64_t n, const int
 // Per band: sum of log2q(seed) over the finite seeds of the rows [early, row_hi) (early already
 // raised to the shard's first row), and their count (integer sums: the result does not depend on
 // the order of the atomics).
-__global__ void __launch_bounds__(kThreads) band_stats_kernel(int64_t n, int64_t early, int64_t row_hi,
+__global__ void __launch_bounds__(kThreads) band_stats_kernel(int64_t n, int shift, int64_t early, int64_t row_hi,
                                                               const float *__restrict__ seeds,
                                                               unsigned long long *__restrict__ sum,
                                                               unsigned long long *__restrict__ cnt) {
@@ -130,7 +149,7 @@ __global__ void __launch_bounds__(kThreads) band_stats_kernel(int64_t n, int64_t
          i += (int64_t)gridDim.x * blockDim.x) {
         const float tau = seeds[i];
         if (!isinf(tau)) {
-            const int b = band_of(i, n);
+            const int b = band_of(i, n, shift);
             s[b] += log2q(tau);
             c[b] += 1;
         }
@@ -150,15 +169,15 @@ __global__ void __launch_bounds__(kThreads) band_stats_kernel(int64_t n, int64_t
     }
 }
 
-// Sort keys of the rows [row_lo, row_hi): pruned rows (band << 32 | curve position), the others
-// (2^36 | index); rows outside the range (2^37 | index).  Counts of pruned rows per band and of
-// the index-order rows.
-__global__ void __launch_bounds__(kThreads) classify_kernel(int64_t n, int64_t early, int64_t row_lo, int64_t row_hi,
+// Sort keys of the rows [row_lo, row_hi): pruned rows (band, cell, curve position), the others and the
+// rows outside the range (tag | index).  Counts of pruned rows per band and of the index-order rows.
+__global__ void __launch_bounds__(kThreads) classify_kernel(int64_t n, int shift, int by_seed, int64_t early, int64_t row_lo, int64_t row_hi,
                                                             const float *__restrict__ seeds,
                                                             const int32_t *__restrict__ pos0,
+                                                            const uint8_t *__restrict__ cell,
                                                             const unsigned long long *__restrict__ sum,
                                                             const unsigned long long *__restrict__ cnt,
-                                                            uint64_t *__restrict__ keys, int32_t *__restrict__ vals,
+                                                            uint32_t *__restrict__ keys, int32_t *__restrict__ vals,
                                                             unsigned long long *__restrict__ pruned_cnt,
                                                             unsigned long long *__restrict__ index_cnt,
                                                             unsigned long long *__restrict__ pruned_isum) {
@@ -167,20 +186,27 @@ __global__ void __launch_bounds__(kThreads) classify_kernel(int64_t n, int64_t e
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         vals[i] = (int32_t)i;
         if (i < row_lo || i >= row_hi) {
-            keys[i] = kOutsideTag | (uint64_t)i;
+            keys[i] = kOutsideTag | (uint32_t)i;
             continue;
         }
         bool pruned = false;
         int b = 0;
+        uint32_t place = (uint32_t)pos0[i];
         if (i >= early) {
-            b = band_of(i, n);
+            b = band_of(i, n, shift);
             const float tau = seeds[i];
             if (!isinf(tau) && cnt[b] > 0) {
                 const long long mean = (long long)sum[b] / (long long)cnt[b];
-                pruned = log2q(tau) <= mean + kLooseLog2Q;
+                const long long rel = log2q(tau) - mean;
+                pruned = rel <= kLooseLog2Q;
+                if (by_seed) {  // rows of one cell by seed, then by curve position
+                    const long long q = (rel + 256) / 40;
+                    place = (uint32_t)(q < 0 ? 0 : (q > 15 ? 15 : q)) << (kPosBits - 4) | place >> 4;
+                }
             }
         }
-        keys[i] = pruned ? ((uint64_t)b << 32 | (uint32_t)pos0[i]) : (kIndexOrderTag | (uint64_t)i);
+        keys[i] = pruned ? (((uint32_t)b << kCellBits | (cell ? cell[i] : 0u)) << kPosBits) | place
+                         : kIndexOrderTag | (uint32_t)i;
         if (pruned) {
             c[b] += 1;
             si += (unsigned long long)i;
@@ -210,8 +236,9 @@ __device__ __forceinline__ int cell_level(unsigned long long cnt, int d, int bit
     return L;
 }
 
-// headpos[r] = r where a new (band, cell) segment starts among the pruned rows, else 0.
-__global__ void __launch_bounds__(kThreads) segment_kernel(int64_t n, const uint64_t *__restrict__ skeys,
+// headpos[r] = r where a new (band, cell) segment starts among the pruned rows, else 0: cells from the
+// keys, or without them (use_cells 0) octree cells of the curve.
+__global__ void __launch_bounds__(kThreads) segment_kernel(int64_t n, const uint32_t *__restrict__ skeys, int use_cells,
                                                            const int32_t *__restrict__ rows,
                                                            const int32_t *__restrict__ pos0,
                                                            const uint64_t *__restrict__ keys0,
@@ -220,6 +247,7 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(int64_t n, const uint
     unsigned long long total = 0;
     for (int b = 0; b < kBands; ++b) total += pruned_cnt[b];
     auto cell_of = [&](int64_t r, int b) -> uint64_t {
+        if (use_cells) return (skeys[r] >> kPosBits) & ((1u << kCellBits) - 1u);
         const int L = cell_level(pruned_cnt[b], d, bits);
         const int shift = d * (bits - L);
         const uint64_t key = keys0[pos0[rows[r]]];
@@ -228,10 +256,10 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(int64_t n, const uint
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         int32_t h = 0;
         if (r < (int64_t)total) {
-            const int b = (int)(skeys[r] >> 32) & 15;
+            const int b = (int)(skeys[r] >> (kPosBits + kCellBits));
             bool head = r == 0;
             if (!head) {
-                const int bp = (int)(skeys[r - 1] >> 32) & 15;
+                const int bp = (int)(skeys[r - 1] >> (kPosBits + kCellBits));
                 head = bp != b || cell_of(r - 1, b) != cell_of(r, b);
             }
             h = head ? (int32_t)r : 0;
@@ -352,7 +380,14 @@ struct Boxes {
     const int32_t *tmin, *glim;
     int d;
     float shrink;  // 1 - gamma, gamma = (d + 3) 2^-23 (exact in FP32)
+    // cells (K = 0: none): home cell of every tile and group, reach of the tiles (pivot-major: treach[a *
+    // n_tiles + t]) and of the groups (greach[g * K + b]), the pivots' distances
+    int K = 0;
+    const int32_t *thome = nullptr, *ghome = nullptr;
+    const float *treach = nullptr, *greach = nullptr, *apart = nullptr;
 };
+// covers the length of a rounded unit vector (at most 1 + 2^-23)
+constexpr float kSlabScale = 1.0f - 9.5367431640625e-07f;  // 1 - 2^-20
 
 // 32-bit words of one group's tile masks
 __host__ __device__ __forceinline__ int64_t mask_words(int64_t n_tiles) { return (n_tiles + 31) / 32; }
@@ -379,27 +414,29 @@ __device__ __forceinline__ GroupBox load_group(const Boxes &b, int64_t g) {
 
 constexpr int kBoxChunk = 128;  // tiles whose boxes a CTA stages in shared memory at a time
 
-// May ref tile tt of the staged chunk hold a neighbour of a row of the group (need), and does
-// its box meet the group's (overlap)?  slo / shi: the chunk's boxes, feature-major.
-__device__ __forceinline__ void tile_test(const Boxes &b, const GroupBox &q, const float (*slo)[kBoxChunk],
-                                          const float (*shi)[kBoxChunk], int32_t tmin, int tt, bool &need,
+// Does the lower bound lb of the squared distance of two sets exclude the tile (see the top)?
+__device__ __forceinline__ bool excluded(const Boxes &b, const GroupBox &q, float lb) {
+    return !isinf(q.tau) && __fsub_rd(__fmul_rd(lb, b.shrink), 1e-37f) > (float)q.tau;
+}
+
+// May a ref tile of box [tile_lo(f), tile_hi(f)] hold a neighbour of a row of the group (need), and does
+// its box meet the group's (overlap)?
+template <typename Lo, typename Hi>
+__device__ __forceinline__ void tile_test(const Boxes &b, const GroupBox &q, Lo &&tile_lo, Hi &&tile_hi, bool &need,
                                           bool &overlap) {
-    need = false;
-    overlap = false;
-    if (tmin >= q.lim) return;  // every ref of the tile comes after every row
     // lb <= the exact squared box distance: every FP32 operation rounded toward -inf
     float lb = 0.f;
     bool meet = true;
 #pragma unroll
     for (int f = 0; f < kMaxDim; ++f) {
         if (f < b.d) {
-            const float tl = slo[f][tt], th = shi[f][tt];
+            const float tl = tile_lo(f), th = tile_hi(f);
             meet = meet && !(tl > q.hi[f] || q.lo[f] > th);
             const float gap = fmaxf(0.f, fmaxf(__fsub_rd(tl, q.hi[f]), __fsub_rd(q.lo[f], th)));  // NaN -> 0
             lb = __fadd_rd(lb, __fmul_rd(gap, gap));
         }
     }
-    need = isinf(q.tau) || !(__fsub_rd(__fmul_rd(lb, b.shrink), 1e-37f) > (float)q.tau);
+    need = !excluded(b, q, lb);
     overlap = need && meet;
 }
 
@@ -407,13 +444,16 @@ __device__ __forceinline__ void tile_test(const Boxes &b, const GroupBox &q, con
 // CTA stages in shared memory (each box read once per CTA instead of once per group):
 // counts[g] = tiles needed (0 for the slots past the groups), and the group's masks of needed
 // tiles and of needed tiles whose box meets the group's (32 tiles per word:
-// masks[(g * words + w) * 2 + {0, 1}]).
+// masks[(g * words + w) * 2 + {0, 1}]).  CELLS: the slab between two cells decides first, and a tile's
+// box is read (from global memory, nothing staged) only where it does not exclude the tile.
+template <bool CELLS>
 __global__ void __launch_bounds__(kThreads) count_kernel(Boxes b, const DevSizes *__restrict__ pruned,
                                                          int64_t max_groups, int64_t n_tiles,
                                                          int32_t *__restrict__ counts, uint32_t *__restrict__ masks) {
-    __shared__ float slo[kMaxDim][kBoxChunk], shi[kMaxDim][kBoxChunk];
-    __shared__ int32_t smin[kBoxChunk];
     constexpr int kWarps = kThreads / 32;
+    __shared__ float slo[CELLS ? 1 : kMaxDim][kBoxChunk], shi[CELLS ? 1 : kMaxDim][kBoxChunk];
+    __shared__ int32_t smin[kBoxChunk];
+    __shared__ float sslab[CELLS ? kWarps : 1][cells::kMaxCells];  // pivots' distance less the group's reach
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t n_groups = pruned->n_groups;
     const int64_t words = mask_words(n_tiles);
@@ -424,28 +464,61 @@ __global__ void __launch_bounds__(kThreads) count_kernel(Boxes b, const DevSizes
         GroupBox q{};
         if (act) q = load_group(b, g);
         int c = 0;
-        for (int64_t t0 = 0; t0 < n_tiles; t0 += kBoxChunk) {
-            const int nt = (int)min((int64_t)kBoxChunk, n_tiles - t0);
-            __syncthreads();
-            for (int i = threadIdx.x; i < nt * b.d; i += kThreads) {
-                const int tt = i / b.d, f = i - tt * b.d;
-                slo[f][tt] = b.tlo[(t0 + tt) * b.d + f];
-                shi[f][tt] = b.thi[(t0 + tt) * b.d + f];
+        auto put = [&](int64_t w, bool need, bool ov) {
+            const unsigned nm = __ballot_sync(0xFFFFFFFFu, need), om = __ballot_sync(0xFFFFFFFFu, ov);
+            if (lane == 0) {
+                masks[(g * words + w) * 2] = nm;
+                masks[(g * words + w) * 2 + 1] = om;
             }
-            for (int i = threadIdx.x; i < nt; i += kThreads) smin[i] = b.tmin[t0 + i];
-            __syncthreads();
+            c += __popc(nm);
+        };
+        if constexpr (CELLS) {
             if (act) {
-                for (int base = 0; base < nt; base += 32) {
-                    const int tt = base + lane;
-                    bool need = false, ov = false;
-                    if (tt < nt) tile_test(b, q, slo, shi, smin[tt], tt, need, ov);
-                    const unsigned nm = __ballot_sync(0xFFFFFFFFu, need), om = __ballot_sync(0xFFFFFFFFu, ov);
-                    if (lane == 0) {
-                        const int64_t w = (t0 + base) / 32;
-                        masks[(g * words + w) * 2] = nm;
-                        masks[(g * words + w) * 2 + 1] = om;
+                const int home = b.ghome[g];
+                __syncwarp();
+                for (int k = lane; k < b.K; k += 32)
+                    sslab[warp][k] = __fsub_rd(b.apart[home * b.K + k], b.greach[g * b.K + k]);
+                __syncwarp();
+                for (int64_t w = 0; w < words; ++w) {
+                    const int64_t t = w * 32 + lane;
+                    // not if every ref of the tile comes after every row, or the slab excludes it (a NaN
+                    // excludes nothing)
+                    bool may = t < n_tiles && b.tmin[t] < q.lim;
+                    if (may) {
+                        const int th = b.thome[t];
+                        if (th != home) {
+                            const float gap = __fsub_rd(sslab[warp][th], b.treach[(int64_t)home * n_tiles + t]);
+                            const float v = __fmul_rd(fmaxf(gap, 0.f), kSlabScale);
+                            may = !excluded(b, q, __fmul_rd(v, v));
+                        }
                     }
-                    c += __popc(nm);
+                    bool need = false, ov = false;
+                    if (may) {
+                        const float *tl = b.tlo + t * b.d, *th = b.thi + t * b.d;
+                        tile_test(b, q, [&](int f) { return tl[f]; }, [&](int f) { return th[f]; }, need, ov);
+                    }
+                    put(w, need, ov);
+                }
+            }
+        } else {
+            for (int64_t t0 = 0; t0 < n_tiles; t0 += kBoxChunk) {
+                const int nt = (int)min((int64_t)kBoxChunk, n_tiles - t0);
+                __syncthreads();
+                for (int i = threadIdx.x; i < nt * b.d; i += kThreads) {
+                    const int tt = i / b.d, f = i - tt * b.d;
+                    slo[f][tt] = b.tlo[(t0 + tt) * b.d + f];
+                    shi[f][tt] = b.thi[(t0 + tt) * b.d + f];
+                }
+                for (int i = threadIdx.x; i < nt; i += kThreads) smin[i] = b.tmin[t0 + i];
+                __syncthreads();
+                if (act) {
+                    for (int base = 0; base < nt; base += 32) {
+                        const int tt = base + lane;
+                        bool need = false, ov = false;
+                        if (tt < nt && smin[tt] < q.lim)  // else every ref of the tile comes after every row
+                            tile_test(b, q, [&](int f) { return slo[f][tt]; }, [&](int f) { return shi[f][tt]; }, need, ov);
+                        put((t0 + base) / 32, need, ov);
+                    }
                 }
             }
         }
@@ -620,16 +693,20 @@ __global__ void uniform_groups_kernel(int64_t n_rows, int G, int64_t n_groups, i
 struct Layout {
     int64_t n_tiles, max_groups;
     size_t tlo, thi, tmin, stats, keys_a, keys_b, vals_a, vals_b, rvals_a, rvals_b, headpos, seg_start, gh, gid, row_off, sizes, glo,
-        ghi, gtau, glim, counts, offsets, masks, list, cub, cub_bytes, total;
+        ghi, gtau, glim, counts, offsets, masks, list, cub, cub_bytes, cells_ws, cells_bytes, thome, ghome, treach, greach,
+        total;
+    int n_cells;  // 0: none
     int64_t maxg[2], max_items[2];
     size_t cnt[2], cbase[2], K[2], kbase[2], S[2], sbase[2], igroup[2], it0[2], it1[2], islot[2], okey_a[2], okey_b[2],
         oval_a[2], oval_b[2], partial[2];
 };
 
-// Groups: segments per band <= (pruned rows of the band) / 256 or 1, groups per segment
-// <= rows / G + 1, so max_groups = n / G + n / 256 + 2 kBands bounds the count.
+// Groups: segments per band <= (pruned rows of the band) / 256 or 1, or K cells (at most n / 4,096, 32 from
+// 65,536 points on: kBands K <= n / 256), groups per segment <= rows / G + 1, so
+// max_groups = n / G + n / 256 + 2 kBands bounds the count.
 Layout layout(int64_t n, int d, int G) {
     Layout L{};
+    L.n_cells = cells::count(n, d);
     L.n_tiles = (n + kTileRefs - 1) / kTileRefs;
     L.max_groups = n / G + n / 256 + 2 * kBands + 1;
     size_t off = 0;
@@ -680,6 +757,12 @@ Layout layout(int64_t n, int d, int G) {
     L.list = take((size_t)L.max_groups * L.n_tiles * 4);
     L.cub_bytes = align_up((size_t)(4u << 20) + (size_t)n / 2, 256);
     L.cub = take(L.cub_bytes);
+    L.cells_bytes = cells::workspace(n, d);
+    L.cells_ws = take(L.cells_bytes);
+    L.thome = take(L.n_cells > 0 ? (size_t)L.n_tiles * 4 : 0);
+    L.ghome = take(L.n_cells > 0 ? (size_t)L.max_groups * 4 : 0);
+    L.treach = take((size_t)L.n_cells * L.n_tiles * 4);
+    L.greach = take((size_t)L.n_cells * L.max_groups * 4);
     L.total = off + 256;
     return L;
 }
@@ -788,7 +871,7 @@ Layout layout_query(int64_t n_ref, int64_t n_query, int d, int G) {
 
 }  // namespace
 
-int64_t early_rows(int64_t n) { return n >> kEarlyShift; }
+int64_t early_rows(int64_t n, int d) { return n >> (cells::count(n, d) > 0 ? kEarlyShiftCells : kEarlyShift); }
 
 bool enabled() {
     const char *env = std::getenv("NNGP_KNN_PRUNE");
@@ -826,50 +909,62 @@ nngp_status build(const float *xs, int64_t n, int64_t row_lo, int64_t row_hi, in
     int32_t *glim = static_cast<int32_t *>(at(L.glim));
     int32_t *counts = static_cast<int32_t *>(at(L.counts)), *offsets = static_cast<int32_t *>(at(L.offsets));
     int32_t *list = static_cast<int32_t *>(at(L.list));
-    const int64_t early = early_rows(n);
+    const int64_t early = early_rows(n, d);
+    const int shift = L.n_cells > 0 ? kEarlyShiftCells : kEarlyShift;
+    cells::Cells cl;
+    if (L.n_cells > 0) {
+        nngp_status cst = cells::build(xs, n, d, dp, at(L.cells_ws), L.cells_bytes, &cl, stream);
+        if (cst != NNGP_OK) return cst;
+    }
     auto cub_check = [&](size_t need) -> nngp_status {
         return need <= L.cub_bytes ? NNGP_OK
                                    : fail(NNGP_ERR_WORKSPACE, "knn pruning: sort / scan scratch of " +
                                                                   std::to_string(need) + " bytes exceeds the budget");
     };
 
-    // ref order (index class, curve position) and the boxes of its tiles
-    ref_keys_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, pos0, static_cast<uint64_t *>(at(L.keys_a)),
+    // ref order (cell, index class, curve position), the boxes of its tiles and their reach
+    ref_keys_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, shift, pos0, cl.of, static_cast<uint32_t *>(at(L.keys_a)),
                                                          static_cast<int32_t *>(at(L.rvals_a)));
     NNGP_CUDA_TRY(cudaGetLastError());
-    cub::DoubleBuffer<uint64_t> rk(static_cast<uint64_t *>(at(L.keys_a)), static_cast<uint64_t *>(at(L.keys_b)));
+    cub::DoubleBuffer<uint32_t> rk(static_cast<uint32_t *>(at(L.keys_a)), static_cast<uint32_t *>(at(L.keys_b)));
     cub::DoubleBuffer<int32_t> rv(static_cast<int32_t *>(at(L.rvals_a)), static_cast<int32_t *>(at(L.rvals_b)));
     size_t need0 = 0;
-    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need0, rk, rv, (int)n, 0, 36, stream));
+    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need0, rk, rv, (int)n, 0, 31, stream));
     if (need0 > L.cub_bytes) return fail(NNGP_ERR_WORKSPACE, "knn pruning: sort scratch exceeds the budget");
     size_t have0 = L.cub_bytes;
-    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(at(L.cub), have0, rk, rv, (int)n, 0, 36, stream));
+    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(at(L.cub), have0, rk, rv, (int)n, 0, 31, stream));
     const int32_t *ref_order = rv.Current();
     tile_box_kernel<<<grid_of(L.n_tiles * 32), kThreads, 0, stream>>>(xs, n, d, dp, ref_order, L.n_tiles, tlo, thi,
                                                                        tmin);
     NNGP_CUDA_TRY(cudaGetLastError());
+    if (L.n_cells > 0) {
+        nngp_status cst = cells::reach(cl, xs, d, dp, n, ref_order, nullptr, nullptr, L.n_tiles, true,
+                                       static_cast<int32_t *>(at(L.thome)), static_cast<float *>(at(L.treach)), stream);
+        if (cst != NNGP_OK) return cst;
+    }
     NNGP_CUDA_TRY(cudaMemsetAsync(sum, 0, kStats * 8, stream));
-    band_stats_kernel<<<grid_of(n - early), kThreads, 0, stream>>>(n, std::max(early, row_lo), row_hi, seeds, sum,
+    band_stats_kernel<<<grid_of(n - early), kThreads, 0, stream>>>(n, shift, std::max(early, row_lo), row_hi, seeds, sum,
                                                                    cnt);
     NNGP_CUDA_TRY(cudaGetLastError());
-    classify_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, early, row_lo, row_hi, seeds, pos0, sum, cnt,
-                                                         static_cast<uint64_t *>(at(L.keys_a)),
+    classify_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, shift, L.n_cells > 0 ? 1 : 0, early, row_lo, row_hi, seeds, pos0, cl.of, sum, cnt,
+                                                         static_cast<uint32_t *>(at(L.keys_a)),
                                                          static_cast<int32_t *>(at(L.vals_a)), pcnt, icnt, isum);
     NNGP_CUDA_TRY(cudaGetLastError());
 
-    // rows: pruned (band, curve position) first, then the index-order rows ascending
-    cub::DoubleBuffer<uint64_t> dk(static_cast<uint64_t *>(at(L.keys_a)), static_cast<uint64_t *>(at(L.keys_b)));
+    // rows: pruned (band, cell, curve position) first, then the index-order rows ascending
+    cub::DoubleBuffer<uint32_t> dk(static_cast<uint32_t *>(at(L.keys_a)), static_cast<uint32_t *>(at(L.keys_b)));
     cub::DoubleBuffer<int32_t> dv(static_cast<int32_t *>(at(L.vals_a)), static_cast<int32_t *>(at(L.vals_b)));
     size_t need = 0;
-    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, dk, dv, (int)n, 0, 38, stream));
+    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, dk, dv, (int)n, 0, 32, stream));
     nngp_status st = cub_check(need);
     if (st != NNGP_OK) return st;
     size_t have = L.cub_bytes;
-    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(at(L.cub), have, dk, dv, (int)n, 0, 38, stream));
+    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(at(L.cub), have, dk, dv, (int)n, 0, 32, stream));
     int32_t *rows = dv.Current();
 
     // groups: segments of one band and one octree cell, cut every G rows
-    segment_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, dk.Current(), rows, pos0, keys0, pcnt, d, bits, headpos);
+    segment_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, dk.Current(), L.n_cells > 0 ? 1 : 0, rows, pos0, keys0, pcnt, d, bits,
+                                                        headpos);
     NNGP_CUDA_TRY(cudaGetLastError());
     need = 0;
     NNGP_CUDA_TRY(cub::DeviceScan::InclusiveScan(nullptr, need, headpos, seg_start, cub::Max(), (int)n, stream));
@@ -893,10 +988,21 @@ nngp_status build(const float *xs, int64_t n, int64_t row_lo, int64_t row_hi, in
                                                                           glo, ghi, gtau, glim);
     NNGP_CUDA_TRY(cudaGetLastError());
     Boxes b{tlo, thi, glo, ghi, gtau, tmin, glim, d, 1.0f - (float)(d + 3) * 1.1920928955078125e-07f};
+    if (L.n_cells > 0) {
+        b.K = L.n_cells;
+        b.thome = static_cast<int32_t *>(at(L.thome));
+        b.ghome = static_cast<int32_t *>(at(L.ghome));
+        b.treach = static_cast<float *>(at(L.treach));
+        b.greach = static_cast<float *>(at(L.greach));
+        b.apart = cl.apart;
+        nngp_status cst = cells::reach(cl, xs, d, dp, n, rows, row_off, &sizes->n_groups, L.max_groups, false,
+                                       static_cast<int32_t *>(at(L.ghome)), static_cast<float *>(at(L.greach)), stream);
+        if (cst != NNGP_OK) return cst;
+    }
     NNGP_CUDA_TRY(cudaMemsetAsync(counts + L.max_groups, 0, sizeof(int32_t), stream));
     uint32_t *masks = static_cast<uint32_t *>(at(L.masks));
-    count_kernel<<<grid_of(L.max_groups * 32), kThreads, 0, stream>>>(b, sizes, L.max_groups, L.n_tiles, counts,
-                                                                       masks);
+    auto count_fn = b.K > 0 ? count_kernel<true> : count_kernel<false>;
+    count_fn<<<grid_of(L.max_groups * 32), kThreads, 0, stream>>>(b, sizes, L.max_groups, L.n_tiles, counts, masks);
     NNGP_CUDA_TRY(cudaGetLastError());
     need = 0;
     NNGP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, need, counts, offsets, (int)(L.max_groups + 1), stream));
@@ -963,7 +1069,7 @@ nngp_status build_query(const float *xs_ref, int64_t n_ref, const float *xq, int
     Boxes b{tlo, thi, glo, ghi, gtau, tmin, glim, d, 1.0f - (float)(d + 3) * 1.1920928955078125e-07f};
     NNGP_CUDA_TRY(cudaMemsetAsync(counts + L.max_groups, 0, sizeof(int32_t), stream));
     uint32_t *masks = static_cast<uint32_t *>(at(L.masks));
-    count_kernel<<<grid_of(L.max_groups * 32), kThreads, 0, stream>>>(b, sizes, L.max_groups, L.n_tiles, counts,
+    count_kernel<false><<<grid_of(L.max_groups * 32), kThreads, 0, stream>>>(b, sizes, L.max_groups, L.n_tiles, counts,
                                                                        masks);
     NNGP_CUDA_TRY(cudaGetLastError());
     size_t need = 0;

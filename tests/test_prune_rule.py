@@ -147,3 +147,44 @@ def test_round_down_box_bound_never_exceeds_the_exact_bound():
             ok = np.isfinite(exact)
             assert np.all(lhs.astype(np.float64)[ok] <= exact[ok]), (d, scale)
 
+
+
+def test_slab_bound_never_exceeds_the_fp32_distance():
+    """The rule between two cells: with u the FP32 unit vector from pivot a to pivot b, the reach of a set
+    the largest FP32 (x - p) . u plus (d + 8) 2^-23 R, every operation of the gap rounded down, the
+    squared slab times (1 - gamma) less 1e-37 stays below the FP32 squared distance of every pair of
+    points, also for points far from their pivot, on the far side of the other one, or at it."""
+    rng = np.random.default_rng(17)
+    f64 = np.float64
+    tight = 0.0
+    for d in (9, 16, 24):
+        shrink = np.float32(1.0 - (d + 3) * 2.0 ** -23)
+        for scale in (1e-20, 1.0, 1e4, 1e12):
+            for spread in (1e-3, 0.3, 3.0):
+                for _ in range(40):
+                    pa, pb = (rng.normal(size=(2, d)) * scale + rng.normal() * scale * 10).astype(np.float32)
+                    t = pb.astype(f64) - pa.astype(f64)
+                    u = (t / np.sqrt((t * t).sum())).astype(np.float32)
+                    apart = _rd(np.array([(t * u).sum() - 1e-12 * np.abs(t * u).sum()]))[0]
+                    sets, reach = [], []
+                    for p, v in ((pa, u), (pb, -u)):
+                        x = (p + rng.normal(size=(60, d)) * scale * spread).astype(np.float32)
+                        x[:5] = p + np.outer(rng.uniform(0, 1.2, 5), v * np.float32(np.sqrt((t * t).sum())))
+                        s, r2 = np.zeros(60, np.float32), np.zeros(60, np.float32)
+                        for f in range(d):
+                            e = (x[:, f] - p[f]).astype(np.float32)
+                            s = (e.astype(f64) * f64(v[f]) + s).astype(np.float32)
+                            r2 = (e.astype(f64) ** 2 + r2).astype(np.float32)
+                        err = np.float32((d + 8) * 2.0 ** -23) * np.sqrt(r2.max())
+                        up = s.max().astype(f64) + f64(err)
+                        reach.append(np.nextafter(np.float32(up), np.float32(np.inf)))
+                        sets.append(x)
+                    gap = _rd(np.array([f64(apart) - f64(reach[0])]))
+                    gap = np.maximum(_rd(gap.astype(f64) - f64(reach[1])), np.float32(0))
+                    v = _rd(gap.astype(f64) * (1.0 - 2.0 ** -20))
+                    lb = _rd(v.astype(f64) ** 2)
+                    lhs = f64(_rd(_rd(lb.astype(f64) * f64(shrink)).astype(f64) - 1e-37)[0])
+                    d2 = fp32_sqdist(sets[0][:, None], sets[1][None]).astype(f64)
+                    assert lhs <= d2.min(), (d, scale, spread)
+                    tight = max(tight, lhs / d2.min() if d2.min() > 0 and lhs > 0 else 0.0)
+    assert tight > 0.5  # and it does separate sets
