@@ -20,10 +20,10 @@
 //            storing dK (n m^2 n_theta values in the reference).
 //
 // Two kernels:
-//   * warp kernel (m <= 32, local_warp.cuh): 8 or 16 lanes per point, its factor's rows in registers;
+//   * warp kernel (m <= 64, local_warp.cuh): 8, 16 or 32 lanes per point; up to 32 neighbours
 //     FP32 with an FP64 re-solve of the system when a pivot is below the threshold (or FP64
 //     throughout for double inputs);
-//   * block kernel (32 < m <= ~150): one CTA per point, the augmented matrix in shared memory,
+//   * block kernel (64 < m <= ~150): one CTA per point, the augmented matrix in shared memory,
 //     FP64.
 // Per-point terms are summed in FP64: per warp, per CTA, then in fixed order by a finalize
 // kernel (deterministic for a given launch shape).
@@ -42,7 +42,7 @@
 namespace nngp {
 
 // ---------------------------------------------------------------------------------------
-// Block kernel (32 < m): one CTA per point, FP64, augmented matrix in shared memory
+// Block kernel (64 < m): one CTA per point, FP64, augmented matrix in shared memory
 // ---------------------------------------------------------------------------------------
 constexpr int kBlkThreads = 256;
 
@@ -354,7 +354,10 @@ nngp_status warp_launch(const void *fn, size_t warp_bytes, int64_t need_warps, i
         return fail(NNGP_ERR_UNSUPPORTED, "the local systems of this d and m need more shared memory than one CTA has");
     const int sms = num_sms();
     // few systems: single-warp CTAs, so that no SM takes two warps while another has none
-    out->warps = need_warps <= (int64_t)sms * 4 || 2 * warp_bytes > block_smem_limit() ? 1 : 2;
+    // (and where a pair leaves shared memory for one warp more)
+    const int64_t sm_bytes = 228 * 1024, cta_bytes = 1024 + 64;
+    const int64_t one = sm_bytes / ((int64_t)warp_bytes + cta_bytes), two = 2 * (sm_bytes / (2 * (int64_t)warp_bytes + cta_bytes));
+    out->warps = need_warps <= (int64_t)sms * 4 || (one > two && one <= kLocalGridPerSm) ? 1 : 2;
     out->smem = out->warps * warp_bytes;
     NNGP_CUDA_TRY(ensure_smem_limit(fn, (int)out->smem));
     int per_sm = 1;
@@ -396,7 +399,7 @@ struct LocalPlan {
 
 LocalPlan plan_local(int64_t n_points, int d, int m, int n_theta, bool grad) {
     LocalPlan p;
-    p.warp = m <= kWarpM;
+    p.warp = m <= kWarpM;  // else one CTA per point
     p.nt = 1 + (grad ? n_theta : 0);
     const int sms = num_sms();
     if (p.warp) {
@@ -528,7 +531,7 @@ nngp_status loglik_impl(const TIn *x, const TIn *y, int64_t n, int d, int ydim, 
     const TIn *y_pt = y + row_begin * ydim;
     // FP32 warp systems: the points that need the FP64 re-solve are marked, then re-solved by a
     // second kernel (its partials follow the main kernel's; finalize sums both in a fixed order)
-    const bool redo = std::is_same<TIn, float>::value && pl.warp;
+    const bool redo = std::is_same<TIn, float>::value && m <= kRedoM;
     if (redo) {
         a.redo_bits = reinterpret_cast<uint32_t *>(head + pl.bits_off);
         NNGP_CUDA_TRY(cudaMemsetAsync(a.redo_bits, 0, (size_t)((rows + 31) / 32) * sizeof(uint32_t), stream));
@@ -759,6 +762,8 @@ __global__ void __launch_bounds__(kCovThreads) cov_recursion_kernel(const int32_
     }
 }
 
+constexpr int kFullM = 64;  // neighbour slots of the recursions (two per lane)
+
 size_t predict_full_workspace(int64_t nq, int m) { return (size_t)(2 * nq * (int64_t)m + nq) * sizeof(double) + 256; }
 
 // samples == false: predict (mean, and var when want_var; with dense_cov, var receives the
@@ -769,7 +774,7 @@ nngp_status predict_full_f64(const double *x_full, const double *y_train, int64_
                              int32_t *flags, void *ws, size_t ws_bytes, cudaStream_t stream, bool samples = false,
                              const double *z = nullptr, bool dense_cov = false) {
     if (nt < 0 || nq < 0) return fail(NNGP_ERR_INVALID_ARGUMENT, "predict_full: negative size");
-    if (m < 1 || m > 2 * kWarpM) return fail(NNGP_ERR_UNSUPPORTED, "predict_full: num_nn must be in [1, 64]");
+    if (m < 1 || m > kFullM) return fail(NNGP_ERR_UNSUPPORTED, "predict_full: num_nn must be in [1, 64]");
     LocalArgs a;
     nngp_status st = fill_args(a, k, d, ydim, m, nt + nq, nq, 0.0, false);
     if (st != NNGP_OK) return st;

@@ -10,7 +10,8 @@ namespace nngp {
 
 constexpr int kMaxDimLocal = 256;
 constexpr int kMaxTheta = kMaxDimLocal + 3;
-constexpr int kWarpM = 32;
+constexpr int kWarpM = 64;  // neighbours of the warp kernel
+constexpr int kRedoM = 32;  // up to here FP32 inputs are solved in FP32 (FP64 re-solves), above in FP64
 constexpr double kHalfLog2Pi = 0.91893853320467274178;
 
 struct LocalArgs {

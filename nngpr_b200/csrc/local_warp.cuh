@@ -1,13 +1,13 @@
-// Local systems of up to 32 neighbours: 32 / LPP points per warp, LPP lanes per point (local.cu
+// Local systems of up to 64 neighbours: 32 / LPP points per warp, LPP lanes per point (local.cu
 // has the mathematics).
 //
 // Lane `sub` of a point's group owns the rows c * LPP + sub, c = 0 .. C - 1 (C = M / LPP), of the
-// neighbour block, row i in registers up to column (c + 1) * LPP - 1: with the rows of one class
-// c equally long, every loop bound is a compile-time constant and only the diagonal LPP x LPP
-// blocks hold entries above the diagonal.  M is the neighbour count rounded up to 16 or 32; rows past
-// it and missing neighbours are identity rows.
+// neighbour block, row i up to column (c + 1) * LPP - 1: with the rows of one class c equally long,
+// every loop bound is a compile-time constant and only the diagonal LPP x LPP blocks hold
+// entries above the diagonal.  M is the neighbour count rounded up to 16, 32 or 64; rows past it and
+// missing neighbours are identity rows.
 //
-// LPP is 16 at M = 32 and 8 at M = 16: two rows per lane, two or four points per warp.  Why several
+// LPP is M / 2: two rows per lane, one, two or four points per warp.  Why several
 // points per warp: with one row per lane a lane computes whole rows of a symmetric matrix, twice
 // the fill's and three times the factor's work, and the chain of each column (two shuffles, a
 // reciprocal square root, a trip through shared memory) is paid per point.  At M = 32 a warp issues 24
@@ -20,7 +20,9 @@
 // Measured against one row per lane (one B200): FP32 n = 1,000,000, d = 16, m = 32 with gradient 8.66 ->
 // 5.80 ms; FP64 n = 434,874, d = 3 5.11 -> 3.5 ms; FP32 n = 100,000, d = 5, m = 13 0.74 -> 0.17 ms.  Four points per
 // warp at M = 32 (8.3 ms in FP32: 255 registers and 6 warps per SM) and everything unrolled
-// (6.5 ms) were slower.
+// (6.5 ms) were slower.  The factor in two column blocks instead of one sweep: FP32 5.80 -> 5.52 ms, FP64
+// 3.49 -> 3.54 ms.  M = 64 (FP64, kernel values recomputed for the gradient to fit 5 warps per SM): n =
+// 20,000, d = 4 ARD, m = 64, two outputs 15.0 ms with one CTA per system -> 1.40 ms.
 //
 // Shared memory per point (PtLayout): the factor by columns, L[i][k] (i > k) at le[k * lda + i], whose
 // unused upper part keeps the squared distances, R[i][k] (k < i) at le[i * lda + k]; the scaled
@@ -54,13 +56,13 @@ template <> struct Vec16<float> {
 };
 
 // Lanes per point of the systems of type TC (4- or 8-byte) with M rows
-template <typename TC> __host__ __device__ constexpr int lanes_per_point(int M) { return M == 16 ? 8 : 16; }
+template <typename TC> __host__ __device__ constexpr int lanes_per_point(int M) { return M / 2; }
 
-// Resident CTAs (of two warps) per SM the registers are budgeted for.  FP32 and the 16-row systems fit
-// 168 registers, 12 warps per SM.  The 32-row FP64 ones need 240: held to 168 they spill 700 bytes of
-// factor rows into every step (5.2 against 3.5 ms at n = 434,874, d = 3), so they run 8 warps per SM.
+// Resident CTAs (of two warps) per SM the registers are budgeted for: FP32 and the 16-row systems 168
+// registers, 12 warps per SM; the 32- and 64-row FP64 ones are held to 8 and 5 warps by shared memory, so
+// they get the registers they ask for.
 template <typename TIn, int M, bool PRED> constexpr int kWarpMinCtas =
-    PRED ? 1 : (std::is_same<TIn, float>::value || M == 16 ? 6 : 1);
+    !PRED && (M == 16 || (M == 32 && std::is_same<TIn, float>::value)) ? 6 : 1;
 
 // Elements before row i of the packed kernel values: row i holds its columns k < i, rounded up to 4.
 __host__ __device__ inline int packed_row(int i) {
@@ -130,7 +132,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
     using VT = typename V::T;
     constexpr int EV = V::N;
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr bool STASH = GRAD && !MATERN;  // RBF gradient: reuse the fill's kernel values
+    constexpr bool STASH = GRAD && !MATERN && M <= 32;  // RBF gradient: reuse the fill's kernel values
     // (opaque, so that addresses and predicates that depend on the lane are formed where they are used
     // instead of being kept in registers, then in local memory, across the loop over the points)
     int lane_here = lane;
@@ -185,7 +187,8 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
     // ---- neighbours of this lane's rows ----------------------------------------------------
     int32_t j[C];
     bool valid[C];
-    unsigned vmask = 0;  // valid rows of the point
+    using Mask = typename std::conditional<(M > 32), unsigned long long, unsigned>::type;
+    Mask vmask = 0;  // valid rows of the point
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         j[c] = -1;
@@ -200,7 +203,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
     }
 #pragma unroll
     for (int c = 0; c < C; ++c)
-        vmask |= ((__ballot_sync(FULL, valid[c]) >> (grp * LPP)) & (0xffffffffu >> (32 - LPP))) << (c * LPP);
+        vmask |= (Mask)((__ballot_sync(FULL, valid[c]) >> (grp * LPP % 32)) & (0xffffffffu >> (32 - LPP))) << (c * LPP);
 
     // ---- gather scaled coordinates: rows 0..M-1 neighbours, row M the point ------------------
     __syncwarp();
@@ -333,15 +336,12 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
                 if (c > dc || row_of(c) >= k0 + u) LE[(k0 + u) * LDA + row_of(c)] = q[c][u];
     });
     __syncwarp();
-    TC r[C][M];  // row c * LPP + sub up to column (c + 1) * LPP - 1 (past the diagonal: unused values)
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-#pragma unroll
-        for (int k = 0; k < (c + 1) * LPP; ++k) r[c][k] = LE[k * LDA + row_of(c)];
-    __syncwarp();
     const TC kpp = rbf + cst + (TC)h.noise + (PRED ? TC(0) : (TC)a.alpha);
 
     // ---- Cholesky of the neighbour block fused with l = L^-1 k and the first output's z = L^-1 y ----
+    // One block of LPP columns at a time, in registers: the earlier blocks' columns are taken off it
+    // (from shared memory), then its own columns are factored right-looking.  Every entry sees the
+    // columns in ascending order, as in one right-looking sweep, with a third fewer registers.
     // A row's own results (its pivot's reciprocal, l, z, b, v) are formed once after the loops: the
     // running value of a row stops changing at its own step.
     const bool weights = PRED && a.weights_out;
@@ -350,41 +350,65 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
     for (int c = 0; c < C; ++c) yv[c] = (!weights && valid[c]) ? (TC)y_ref[(int64_t)j[c] * a.ydim] : TC(0);
     TC minpiv = TC(3.0e38);
     TC ss = TC(0);
+    auto factor_block = [&](const int dc) {
+        TC r[C][LPP];  // columns dc * LPP .. of the rows of the classes >= dc (past the diagonal: unused values)
+        const int k1 = dc * LPP;
 #pragma unroll
-    for (int k = 0; k < M; ++k) {
-        const int ck = k / LPP, sk = k % LPP;
-        const TC piv = __shfl_sync(FULL, r[ck][k], sk, LPP);
-        minpiv = fmin(minpiv, piv);
-        const TC inv = drsqrt<TC>(piv);  // 1 / L_kk
-        const TC lk = __shfl_sync(FULL, kvec[ck], sk, LPP) * inv;
-        const TC zk = __shfl_sync(FULL, yv[ck], sk, LPP) * inv;
-        if (sub == sk) idg[k] = inv;
-        TC *col = LE + k * LDA;
+        for (int c = dc; c < C; ++c)
 #pragma unroll
-        for (int c = ck; c < C; ++c) {
-            r[c][k] = r[c][k] * inv;  // L_ik
-            if (c > ck || sub > sk) {
-                kvec[c] = fma(-r[c][k], lk, kvec[c]);
-                yv[c] = fma(-r[c][k], zk, yv[c]);
-                col[row_of(c)] = r[c][k];
+            for (int q = 0; q < LPP; ++q) r[c][q] = LE[(k1 + q) * LDA + row_of(c)];
+        __syncwarp();
+#pragma unroll 2
+        for (int k = 0; k < k1; ++k) {
+            const TC *col = LE + k * LDA;
+            TC own[C];
+#pragma unroll
+            for (int c = dc; c < C; ++c) own[c] = -col[row_of(c)];
+#pragma unroll
+            for (int q = 0; q < LPP; q += EV) {
+                const VT v = *reinterpret_cast<const VT *>(col + k1 + q);
+#pragma unroll
+                for (int e = 0; e < EV; ++e)
+#pragma unroll
+                    for (int c = dc; c < C; ++c) r[c][q + e] = fma(own[c], V::get(v, e), r[c][q + e]);
             }
         }
-        ss = fma(lk, lk, ss);
-        if (k + 1 < M) {
+#pragma unroll
+        for (int sk = 0; sk < LPP; ++sk) {
+            const TC piv = __shfl_sync(FULL, r[dc][sk], sk, LPP);
+            minpiv = fmin(minpiv, piv);
+            const TC inv = drsqrt<TC>(piv);  // 1 / L_kk
+            const TC lk = __shfl_sync(FULL, kvec[dc], sk, LPP) * inv;
+            const TC zk = __shfl_sync(FULL, yv[dc], sk, LPP) * inv;
+            if (sub == sk) idg[k1 + sk] = inv;
+            TC *col = LE + (k1 + sk) * LDA;
+#pragma unroll
+            for (int c = dc; c < C; ++c) {
+                r[c][sk] = r[c][sk] * inv;  // L_ik
+                if (c > dc || sub > sk) {
+                    kvec[c] = fma(-r[c][sk], lk, kvec[c]);
+                    yv[c] = fma(-r[c][sk], zk, yv[c]);
+                    col[row_of(c)] = r[c][sk];
+                }
+            }
+            ss = fma(lk, lk, ss);
             __syncwarp();
+            if (sk + 1 < LPP) {
 #pragma unroll
-            for (int q = (k + 1) / EV; q < M / EV; ++q) {
-                const VT v = *reinterpret_cast<const VT *>(col + q * EV);
+                for (int q = (sk + 1) / EV * EV; q < LPP; q += EV) {
+                    const VT v = *reinterpret_cast<const VT *>(col + k1 + q);
 #pragma unroll
-                for (int e = 0; e < EV; ++e) {
-                    const int jj = q * EV + e;
-                    if (jj <= k) continue;
+                    for (int e = 0; e < EV; ++e) {
+                        if (q + e <= sk) continue;
 #pragma unroll
-                    for (int c = jj / LPP; c < C; ++c) r[c][jj] = fma(-r[c][k], V::get(v, e), r[c][jj]);
+                        for (int c = dc; c < C; ++c) r[c][q + e] = fma(-r[c][sk], V::get(v, e), r[c][q + e]);
+                    }
                 }
             }
         }
-    }
+    };
+    factor_block(0);
+    if constexpr (C > 1) factor_block(1);
     const TC s2 = kpp - ss;
     bool ok = true;
     if constexpr (std::is_same<TC, float>::value)
@@ -637,11 +661,11 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_k
                                                          double *__restrict__ block_out, TIn *__restrict__ mean,
                                                          TIn *__restrict__ var, int32_t *__restrict__ flags) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr bool F32 = std::is_same<TIn, float>::value;
-    using T1 = TIn;  // the first attempt's precision
+    using T1 = typename std::conditional<(M > 32), double, TIn>::type;  // the first attempt's precision
+    constexpr bool F32 = std::is_same<T1, float>::value;
     constexpr int LPP = lanes_per_point<T1>(M), GROUPS = 32 / LPP;
     const WarpLayout lay = WarpLayout::make<F32, !F32 || PRED>(M, a.d, a.n_theta, GRAD,
-                                                              GRAD && !MATERN, GRAD && a.ard);
+                                                              GRAD && !MATERN && M <= 32, GRAD && a.ard);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int sub = lane & (LPP - 1), grp = lane / LPP;
     unsigned char *wsm = smem_raw + warp * lay.total;
@@ -697,7 +721,7 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<double, M, false>)) local_re
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int LPP = lanes_per_point<double>(M), GROUPS = 32 / LPP;
     const WarpLayout lay = WarpLayout::make<false, true>(M, a.d, a.n_theta, GRAD,
-                                                        GRAD && !MATERN, GRAD && a.ard);
+                                                        GRAD && !MATERN && M <= 32, GRAD && a.ard);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int sub = lane & (LPP - 1), grp = lane / LPP;
     unsigned char *wsm = smem_raw + warp * lay.total;
@@ -732,7 +756,7 @@ struct WarpLaunch {
 };
 nngp_status warp_launch(const void *fn, size_t warp_bytes, int64_t need_warps, int grid_limit, WarpLaunch *out);
 
-inline int warp_rows(int m) { return m <= 16 ? 16 : 32; }
+inline int warp_rows(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : 64); }
 
 // *parts: CTAs of the launch (the partial sums in block_out)
 template <typename TIn>

@@ -18,9 +18,14 @@ nngp_status launch_fit(const LocalArgs &a, bool grad, const TIn *x_ref, const TI
         return rbf ? (grad ? local_warp_kernel<TIn, R, true, false, false> : local_warp_kernel<TIn, R, false, false, false>)
                    : (grad ? local_warp_kernel<TIn, R, true, false, true> : local_warp_kernel<TIn, R, false, false, true>);
     };
-    auto fn = M == 16 ? pick(std::integral_constant<int, 16>{}) : pick(std::integral_constant<int, 32>{});
+    auto fn = M == 16   ? pick(std::integral_constant<int, 16>{})
+              : M == 32 ? pick(std::integral_constant<int, 32>{})
+                        : pick(std::integral_constant<int, 64>{});
     const int groups = 32 / lanes_per_point<TIn>(M);
-    const size_t bytes = WarpLayout::make<F32, !F32>(M, a.d, a.n_theta, grad, grad && rbf, grad && a.ard).total;
+    const bool keep_e = grad && rbf && M <= 32;
+    const size_t bytes = (F32 && M <= 32 ? WarpLayout::make<true, false>(M, a.d, a.n_theta, grad, keep_e, grad && a.ard)
+                                         : WarpLayout::make<false, true>(M, a.d, a.n_theta, grad, keep_e, grad && a.ard))
+                             .total;
     WarpLaunch w;
     nngp_status st = warp_launch(reinterpret_cast<const void *>(fn), bytes, (a.n_points + groups - 1) / groups,
                                  grid_limit, &w);
@@ -41,9 +46,13 @@ nngp_status launch_predict(const LocalArgs &a, const TIn *x_ref, const TIn *y_re
         constexpr int R = decltype(rows)::value;
         return rbf ? local_warp_kernel<TIn, R, false, true, false> : local_warp_kernel<TIn, R, false, true, true>;
     };
-    auto fn = M == 16 ? pick(std::integral_constant<int, 16>{}) : pick(std::integral_constant<int, 32>{});
+    auto fn = M == 16   ? pick(std::integral_constant<int, 16>{})
+              : M == 32 ? pick(std::integral_constant<int, 32>{})
+                        : pick(std::integral_constant<int, 64>{});
     const int groups = 32 / lanes_per_point<TIn>(M);
-    const size_t bytes = WarpLayout::make<F32, true>(M, a.d, a.n_theta, false, false, false).total;
+    const size_t bytes = (F32 && M <= 32 ? WarpLayout::make<true, true>(M, a.d, 0, false, false, false)
+                                         : WarpLayout::make<false, true>(M, a.d, 0, false, false, false))
+                             .total;
     WarpLaunch w;
     nngp_status st = warp_launch(reinterpret_cast<const void *>(fn), bytes, (a.n_points + groups - 1) / groups, 0, &w);
     if (st != NNGP_OK) return st;

@@ -52,7 +52,31 @@ def test_loglik_row_classes_and_tails(dtype, m, d, ard):
             assert abs(only[0] - want_l) < 1e-10 * abs(want_l)
 
 
-@pytest.mark.parametrize('m', [16, 32])
+@pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
+@pytest.mark.parametrize('m', [33, 47, 63, 64, 65, 80])
+def test_more_than_32_neighbours(dtype, m):
+    """FP64 systems whatever the inputs: one warp per point up to 64 neighbours, one CTA above."""
+    for d, ard, ydim in ((3, False, 1), (6, True, 3)):
+        x, y, p, nbr = problem(m + 37, d, m, ard, ydim, m + d)
+        want_l, want_g = O.log_marginal_likelihood(x, y, nbr, oracle_params(p), 1e-8, True)
+        nt = torch.from_numpy(np.ascontiguousarray(nbr, dtype=np.int32)).cuda()
+        xt, yt = torch.from_numpy(x).to('cuda', dtype), torch.from_numpy(y).to('cuda', dtype)
+        out = ops.loglik(xt, yt, nt, p, 1e-8, True).cpu().numpy()
+        assert abs(out[0] - want_l) < 1e-10 * abs(want_l)
+        assert rel(out[1:], want_g) < 1e-9
+        only = ops.loglik(xt, yt, nt, p, 1e-8, False).cpu().numpy()
+        assert abs(only[0] - want_l) < 1e-10 * abs(want_l)
+        xq = np.random.default_rng(m).uniform(0, 1, (9, d)).astype(np.float32).astype(np.float64)
+        nq = O.knn(x, xq, m, None, p.length_scale)
+        want, std = O.predict(x, y, xq, nq, oracle_params(p), 1e-8)
+        mean, var = ops.predict(xt, yt, torch.from_numpy(xq).to('cuda', dtype),
+                                torch.from_numpy(np.ascontiguousarray(nq, dtype=np.int32)).cuda(), p, 1e-8)
+        lim = 1e-10 if dtype == torch.float64 else 1e-6
+        assert np.max(np.abs(mean.cpu().numpy() - want)) < lim * max(1.0, np.max(np.abs(want)))
+        assert np.max(np.abs(np.sqrt(var.cpu().numpy().astype(np.float64)) - std)) < lim * np.max(std)
+
+
+@pytest.mark.parametrize('m', [16, 32, 50])
 def test_matern_groups(m):
     for nu in (0.5, 2.5):
         x, y, p, nbr = problem(131, 5, m, True, 1, m, nu)
