@@ -13,32 +13,33 @@
 //     The dropped and truncated terms are below 2^-21 |a||b| per product, the FP32 accumulation
 //     adds at most K' ulps; eps = 2^-16 (|qc| + max|rc|)^2 covers both with a margin of 4 or more,
 //     so every ref the exact algorithm inserts still passes the screen;
-//   * persistent CTAs (work items = query tiles handed out heaviest first through a global
-//     counter), 160 threads: warp 4 allocates TMEM (two 128-column accumulators, or one when
-//     three CTAs share the SM) and
-//     one of its lanes issues the TMA bulk copies of ref tiles into a shared-memory ring (operands
-//     and exact coordinates in one copy) and the MMAs; warps 0-3 are the epilogue, warp w owning
-//     query rows 32w..32w+31 (its TMEM lane quadrant).  Up to three CTAs share an SM when shared
-//     memory allows (small d): the epilogue is latency-bound, and every extra warp per scheduler
-//     shows (d = 3: 30.8 ms with two CTAs per SM, 23.1 ms with three, n = 434,874).  For d = 12
-//     and 16, where one CTA fills an SM, a work item is two query tiles: both MMA chains read the
-//     same staged ref tile and 8 epilogue warps share the SM (d = 16, n = 1M: 235 -> 173 ms);
-//   * epilogue: each 32-column chunk of a row is one tcgen05.ld (issued one chunk ahead into a
-//     second register set), screened with three-input min over groups of 8 columns against the
-//     row's threshold into a candidate mask (skipped when no row of the warp has one); the
-//     accumulator buffer is freed as soon as the tile's four chunks are read.  Then each lane
-//     walks the candidates of its row in the whole tile, one per warp iteration (so one
-//     iteration serves every row that has a candidate), and rescores them exactly (exact
-//     coordinates from the same smem stage, the oracle's arithmetic); survivors of the row's
-//     current bound are compacted with ballots into a
-//     per-warp queue.  Once 32 entries are queued the warp drains them into the rows' lists: each
-//     row keeps its best m as a max-heap of 64-bit keys (distance bits << 32 | index) in shared
-//     memory, 32 entries go in per pass, one per lane, entries of one row serialised by match_any.
-//     The key order is (distance, index), so the final sets do not depend on insertion order; at
-//     the end of a work item each heap is sorted across the warp (bitonic) and written out;
-//   * mbarriers: b_full (TMA -> MMA), b_empty (MMA commit + 4 epilogue warps -> producer),
-//     t_full (MMA commit -> epilogue), t_empty (4 epilogue warps -> MMA), a_ready (query operand
-//     written by the epilogue -> MMA).  Every wait is bounded; on a timeout the CTA raises
+//   * persistent CTAs (work items = query tiles handed out heaviest first through a global counter) of
+//     three kinds of warps.  One lane of the MMA warp issues the MMAs and, with two CTAs per SM, the
+//     TMA bulk copies of ref tiles into a shared-memory ring; a CTA alone on its SM has a warp of its
+//     own for the copies.  Screening warp w owns the 32 query rows of TMEM lane quadrant w % 4, and
+//     rescoring warp EPI_WARPS + w the candidates that it finds.  For d = 12 and 16 a work item is two
+//     query tiles: both MMA chains read the same staged ref tile (d = 16, n = 1M: 235 -> 173 ms when
+//     this went in, every tile scanned);
+//   * a screening warp reads its accumulator 16 columns at a time (one load ahead, in a second register set), reduces
+//     groups of 8 columns with three-input minima and compares them with the row's threshold: most tiles
+//     end there, after one vote.  For the others it builds the column mask of each row, releases the
+//     accumulator and appends one entry (mask, tile, row) per row with candidates to a ring in shared
+//     memory;
+//   * a rescoring warp takes up to 32 entries, one per lane; each lane walks its columns, reads their exact
+//     coordinates from the tile's record in global memory, evaluates the oracle's arithmetic, and
+//     inserts what is within the row's bound into the row's list of its best m in shared memory
+//     (list_insert).  The new bound lowers the row's screening threshold, which the screening warp reads
+//     once per stage; an older threshold only lets more through.  Lists are ordered by (distance,
+//     index), so the final sets do not depend on insertion order; at the end of a work item each list
+//     is sorted across the warp (bitonic) and written out.
+//     What bounds it: the screen's and the rescoring's chains of latencies, not a unit's rate (tensor pipe and
+//     issue slots both below half busy).  While one warp did both, the accumulator waited out every
+//     candidate's loads and heap steps, half of the kernel's time at d = 16.  Of one search, one warp for
+//     both -> two: 22.7 -> 20.6 ms (d = 16, n = 1M, clustered), 4.3 -> 3.7 ms (d = 3, n = 434,874), 17.0 -> 15.0 ms
+//     (d = 8, two searches' kernels), 511 -> 368 us (16,384 queries in 50,000, d = 18); from 9.2 to 9.4 ms at d = 24, n = 300,000;
+//   * mbarriers: b_full (TMA -> MMA), b_empty (MMA commit -> producer), t_full (MMA commit ->
+//     screen), t_empty (screening warps -> MMA), a_ready (query operand written by the screening warps
+//     -> MMA); the rings' two counters each are plain words, released and acquired.  Every wait is bounded; on a timeout the CTA raises
 //     NNGP_FLAG_TIMEOUT, drains what it issued (bounded), frees TMEM and returns.
 // No TMA multicast and no cluster launch.
 #include <algorithm>
@@ -53,25 +54,26 @@ namespace tc {
 
 constexpr int QT = kTcQueryTile;  // queries per tile (UMMA M)
 constexpr int RT = kTcRefTile;    // refs per tile (UMMA N)
-static_assert(RT == 128, "the epilogue screens a ref tile as four 32-column chunks");
-constexpr int THREADS = 5 * 32;   // layout self-test: 4 epilogue warps + the MMA warp
+static_assert(RT == 128, "a ref tile is screened as four 32-column chunks");
+constexpr int THREADS = 5 * 32;   // layout self-test: 4 warps that read TMEM + the MMA warp
 constexpr int LIST = 32;       // largest num_nn
-constexpr int HS = 33;         // heap row stride in 64-bit keys (odd: rows of a warp hit distinct banks)
-constexpr int DRAIN_AT = 32;   // queued entries that trigger a drain at the end of a tile (8: +2%, 128: +7% at d = 3)
-constexpr int QCAP = 64;       // key queue entries per epilogue warp (a drain runs before a batch
-                               // that could overflow it)
-constexpr int CQCAP = 96;      // screened candidates queued per epilogue warp for rescoring
+constexpr int DS = 44;         // row of a list: 32 distances, the largest of each 4 of them, padding (16-byte
+                               // loads of 8 rows hit distinct banks)
+constexpr int IS = 33;         // row of its indices (odd: the rows of a warp in distinct banks)
+constexpr int RING = 64;       // candidate entries between a screening warp and its rescoring warp (a tile gives
+                               // at most 32)
+constexpr int RING_MIN = 16;   // entries a rescoring warp waits for (fewer at the end of an item)
+constexpr uint32_t RING_DONE = 0x80000000u, RING_ABORT = 0x40000000u;  // flags beside the pushed count
 constexpr int MAX_STAGES = 8;  // ring stages (mbarrier slots)
 constexpr uint32_t kSelftestCols = 2 * RT;  // TMEM columns of the layout self-test
 constexpr float kEpsTc = 1.52587890625e-05f;       // 2^-16: TF32 x3 split
 constexpr float kEpsBf = 6.103515625e-05f;         // 2^-14: BF16 x3 split
 constexpr float kPadNorm = 1.7014118346046923e38f;  // 2^127: padded refs never pass a finite screen
-// list key: FP32 distance bits (non-negative, so integer order = float order) << 32 | index;
-// an empty slot is (+inf, 0xffffffff), larger than every real entry, read back as index -1
-constexpr uint64_t kEmptyKey = (uint64_t)0x7F800000u << 32 | 0xFFFFFFFFu;
+// a list entry is (distance, index); an empty slot is (+inf, 0xffffffff), larger than every real entry, read back
+// as index -1.  Sorted as FP32 distance bits (non-negative, so integer order = float order) << 32 | index
 
 // D: padded dimension; QTILES: 128-query tiles per work item (their MMAs share each staged ref
-// tile; 4 epilogue warps per query tile, one per TMEM lane quadrant).
+// tile; 4 screening and 4 rescoring warps per query tile, one each per TMEM lane quadrant).
 // Operands: D <= 8 a TF32 x3 split (kind::tf32, K = 8 per MMA, 4-byte elements); D >= 12 a BF16 x3
 // split (kind::f16, K = 16 per MMA, 2-byte elements): half the bytes per ref tile and, at the
 // tensor pipe's doubled BF16 rate, 4 instead of 7 MMA steps per tile at D = 16.
@@ -101,8 +103,8 @@ struct Cfg {
     static constexpr int IX_BYTES = IX_MODE == 2 ? RT * 4 : 0;
     // a ref tile in global memory: [B operand | exact coordinates | indices]; only the B operand
     // is staged in shared memory (the MMAs' input), so a stage is free again as soon as its MMAs
-    // complete.  The screen passes about one pair in 3,000 at d = 16: the epilogue reads those
-    // pairs' exact coordinates and indices from the record in global memory, 32 at a time.
+    // complete.  The screen passes about one pair in 3,000 at d = 16: the rescoring warps
+    // read those pairs' exact coordinates and indices from the record in global memory.
     static constexpr int TILE_BYTES = OP_BYTES + EX_BYTES + IX_BYTES;
     // d = 16: a stage holds two ref tiles, multiplied by one MMA of N = 256 per query tile and K
     // slice (half the MMA instructions and 12 KB of operand reads per 256 x 128 x 16 instead of
@@ -113,29 +115,25 @@ struct Cfg {
     static constexpr int STAGE_BYTES = OP_BYTES * TPS;
     static constexpr int A_TILE = QT * KP * ESZ;    // query operand of one query tile
     static constexpr int A_BYTES = A_TILE * QTILES;
-    static constexpr int LIST_BYTES = ROWS * HS * 8;  // one heap of keys per query
-    static constexpr int QUEUE_BYTES = EPI_WARPS * QCAP * (8 + 1);  // key + row
-    static constexpr int CQ_BYTES = EPI_WARPS * CQCAP * 8;          // ref position << 5 | row
+    static constexpr int LIST_BYTES = ROWS * (DS + IS) * 4;  // the m best of every query, unordered
+    static constexpr int RING_BYTES = EPI_WARPS * (RING * (16 + 4) + 8);  // masks, (tile, row), counters
+    static constexpr int ROW_BYTES = ROWS * 7 * 4;  // per row: threshold, bound, norm, eps, limit, point, largest
     static constexpr int BAR_BYTES = 256;
-    static constexpr int FIXED = ALIGN + A_BYTES + LIST_BYTES + QUEUE_BYTES + CQ_BYTES + BAR_BYTES;  // ALIGN: base slack
-    // as many CTAs per SM (up to 3) as hold at least 2 stages each: more epilogue warps per
-    // scheduler.  Three CTAs share TMEM with one accumulator buffer each (the epilogue frees it
-    // as soon as a tile's scores are in registers); one or two CTAs double-buffer it.
-    static constexpr int ST3 = (75 * 1024 - FIXED) / STAGE_BYTES;
+    static constexpr int FIXED = ALIGN + A_BYTES + LIST_BYTES + RING_BYTES + ROW_BYTES + BAR_BYTES;  // ALIGN: base slack
+    // two CTAs per SM where each holds at least 2 stages: more warps per scheduler
     static constexpr int ST2 = (112 * 1024 - FIXED) / STAGE_BYTES;
-    static constexpr int ST1 = (220 * 1024 - FIXED) / STAGE_BYTES;
-    static constexpr int CTAS_PER_SM = ST3 >= 2 ? 3 : (ST2 >= 2 ? 2 : 1);
-    static constexpr int STN = CTAS_PER_SM == 3 ? ST3 : (CTAS_PER_SM == 2 ? ST2 : ST1);
+    static constexpr int ST1 = (231936 - FIXED) / STAGE_BYTES;  // of 232,448 bytes
+    static constexpr int CTAS_PER_SM = ST2 >= 2 ? 2 : 1;
+    static constexpr int STN = CTAS_PER_SM == 2 ? ST2 : ST1;
     static constexpr int STAGES = STN > MAX_STAGES ? MAX_STAGES : STN;
     // A CTA alone on its SM streams its tiles from a warp of its own: the MMA warp then waits
     // only for a staged tile and a free accumulator buffer, never for a stage to be refilled,
-    // and each copy starts as soon as the MMAs of the stage's previous tile complete.  With 2 or
-    // 3 CTAs per SM the other CTAs fill those gaps, and the register budget has no room for
-    // another warp: the MMA warp issues the copies itself.
+    // and each copy starts as soon as the MMAs of the stage's previous tile complete.  With 2 CTAs
+    // per SM the other CTA fills those gaps, and the MMA warp issues the copies itself.
     static constexpr bool TMA_WARP = CTAS_PER_SM == 1;
-    static constexpr int THREADS = (EPI_WARPS + 1 + (TMA_WARP ? 1 : 0)) * 32;
+    static constexpr int THREADS = (2 * EPI_WARPS + 1 + (TMA_WARP ? 1 : 0)) * 32;
     static constexpr int SMEM = FIXED + STAGES * STAGE_BYTES;
-    static constexpr int NBUF = (CTAS_PER_SM == 3 || PAIR) ? 1 : 2;  // accumulator buffers in TMEM
+    static constexpr int NBUF = PAIR ? 1 : 2;  // accumulator buffers in TMEM
     static constexpr uint32_t BUF_COLS = RS * QTILES;                 // one buffer: a stage per query tile
     static constexpr uint32_t TMEM_COLS = NBUF * BUF_COLS;  // a power of two >= 32, <= 512
     static_assert(TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "TMEM columns");
@@ -272,27 +270,84 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
                  : "memory");
 }
 
-// Max-heap of the m best keys (root = current m-th best): replace the root by x when x is
-// smaller and sift it down.
-__device__ __forceinline__ void heap_insert(uint64_t *h, int m, uint64_t x) {
-    if (!(x < h[0])) return;
-    int i = 0;
+// 16 columns of this thread's TMEM lane, no wait, and the wait with the registers as operands
+__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
+
+// Counters between two warps of a CTA in shared memory
+__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+// Polls *p until ready(value) or limit_ns x waits have passed; false on a timeout.
+template <typename F>
+__device__ __forceinline__ bool poll_bounded(const uint32_t *p, uint64_t limit_ns, uint32_t waits, uint32_t &v, F &&ready) {
+    v = ld_acquire(p);
+    if (ready(v)) return true;
+    const uint64_t t0 = global_timer_ns();
     while (true) {
-        int c = 2 * i + 1;
-        if (c >= m) break;
-        uint64_t kc = h[c];
-        if (c + 1 < m) {
-            const uint64_t k2 = h[c + 1];
-            if (k2 > kc) {
-                kc = k2;
-                ++c;
+        __nanosleep(32);
+        v = ld_acquire(p);
+        if (ready(v)) return true;
+        if ((float)(global_timer_ns() - t0) > (float)limit_ns * (float)waits) return false;
+    }
+}
+
+// A row's m best so far, unordered: distances d[0 .. 31] (slots >= m: -inf), the largest of each four at
+// d[32 .. 39], indices, and the slot of the largest (distance, index).  Replaces that slot by (x, j) when (x, j)
+// is the smaller and finds the new largest through the four-maxima: about 50 instructions, the same in every
+// lane.  A binary heap's sift-down is five dependent steps whose lanes part (one search, n = 1M, d = 16
+// clustered: 33.3 ms with heaps, 32.1 sweeping all 32 slots, 30.1 with the four-maxima).  Returns the largest distance.
+__device__ __forceinline__ float list_insert(float *d, uint32_t *idx, int32_t *largest, float x, uint32_t j) {
+    const int state = *largest, at = state & 31;  // bit 5: the list has held an infinite distance
+    const float top = d[at];
+    if (!(x < top || (x == top && j < idx[at]))) return top;
+    d[at] = x;
+    idx[at] = j;
+    float4 *d4 = reinterpret_cast<float4 *>(d);
+    const float4 own = d4[at >> 2];
+    d[32 + (at >> 2)] = fmaxf(fmaxf(own.x, own.y), fmaxf(own.z, own.w));
+    const float4 a = d4[8], b = d4[9];
+    const float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+    uint32_t fours = (a.x == mx ? 1u : 0u) | (a.y == mx ? 2u : 0u) | (a.z == mx ? 4u : 0u) | (a.w == mx ? 8u : 0u) |
+                     (b.x == mx ? 16u : 0u) | (b.y == mx ? 32u : 0u) | (b.z == mx ? 64u : 0u) | (b.w == mx ? 128u : 0u);
+    auto equal_in = [&](int g) {
+        const float4 t = d4[g];
+        return (t.x == mx ? 1u : 0u) | (t.y == mx ? 2u : 0u) | (t.z == mx ? 4u : 0u) | (t.w == mx ? 8u : 0u);
+    };
+    int g = __ffs((int)fours) - 1;
+    uint32_t eq = equal_in(g);
+    int pos = 4 * g + __ffs((int)eq) - 1;
+    const int held_inf = (state & 32) | (x < pos_inf<float>() ? 0 : 32);
+    // (any of the empty slots will do while there are some and nothing else is infinite)
+    if (((fours & (fours - 1)) | (eq & (eq - 1))) != 0u && (mx < pos_inf<float>() || held_inf)) {
+        for (; fours; fours &= fours - 1) {  // equal distances: the largest index goes first
+            g = __ffs((int)fours) - 1;
+            for (eq = equal_in(g); eq; eq &= eq - 1) {
+                const int k = 4 * g + __ffs((int)eq) - 1;
+                if (idx[k] > idx[pos]) pos = k;
             }
         }
-        if (kc <= x) break;
-        h[i] = kc;
-        i = c;
     }
-    h[i] = x;
+    *largest = pos | held_inf;
+    return mx;
 }
 
 __device__ __forceinline__ float min3f(float a, float b, float c) {
@@ -422,10 +477,21 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
         (reinterpret_cast<uintptr_t>(smem_raw) + (C::ALIGN - 1)) & ~uintptr_t(C::ALIGN - 1));
     unsigned char *sA = sm;
     unsigned char *sB = sA + C::A_BYTES;
-    uint64_t *H = reinterpret_cast<uint64_t *>(sB + S * C::STAGE_BYTES);  // [ROWS][HS] heaps
-    unsigned char *qbase = reinterpret_cast<unsigned char *>(H + C::ROWS * HS);
-    uint64_t *cqbase = reinterpret_cast<uint64_t *>(qbase + C::QUEUE_BYTES);  // [EPI_WARPS][CQCAP] candidates
-    uint64_t *bars = cqbase + EPI_WARPS * CQCAP;
+    float *list_d = reinterpret_cast<float *>(sB + S * C::STAGE_BYTES);           // [ROWS][DS]
+    uint32_t *list_i = reinterpret_cast<uint32_t *>(list_d + C::ROWS * DS);       // [ROWS][IS]
+    uint4 *ring_mask = reinterpret_cast<uint4 *>(list_i + C::ROWS * IS);         // [EPI_WARPS][RING] column masks
+    uint32_t *ring_meta = reinterpret_cast<uint32_t *>(ring_mask + EPI_WARPS * RING);  // tile << 5 | row
+    uint32_t *ring_head = ring_meta + EPI_WARPS * RING;  // entries pushed, with RING_DONE / RING_ABORT
+    uint32_t *ring_tail = ring_head + EPI_WARPS;         // entries taken
+    // per row (slot warp * 32 + lane of its screening warp)
+    float *row_thr = reinterpret_cast<float *>(ring_tail + EPI_WARPS);  // screening threshold, only ever lowered
+    float *row_worst = row_thr + C::ROWS;                // bound of its m-th distance
+    float *row_norm = row_worst + C::ROWS, *row_eps = row_norm + C::ROWS;
+    int32_t *row_limit = reinterpret_cast<int32_t *>(row_eps + C::ROWS);
+    int32_t *row_point = row_limit + C::ROWS;            // -1: past the item's rows
+    int32_t *row_largest = row_point + C::ROWS;          // slot of its list's largest entry (list_insert)
+    uint64_t *bars = reinterpret_cast<uint64_t *>(row_largest + C::ROWS);
+    static_assert((C::LIST_BYTES + C::A_BYTES) % 16 == 0 && (C::RING_BYTES + C::ROW_BYTES) % 8 == 0, "alignment");
     uint64_t *b_full = bars;                    // [S <= MAX_STAGES]
     uint64_t *b_empty = bars + MAX_STAGES;      // [S <= MAX_STAGES]
     uint64_t *t_full = bars + 2 * MAX_STAGES;   // [2]
@@ -437,8 +503,9 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
     static_assert((2 * MAX_STAGES + 8) * 8 <= C::BAR_BYTES, "barrier block");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool producer_warp = warp == EPI_WARPS;                 // MMA issue (and the copies without TMA_WARP)
-    const bool copy_warp = C::TMA_WARP && warp == EPI_WARPS + 1;  // the copies with TMA_WARP
+    // warps 0 .. EPI_WARPS - 1 screen, EPI_WARPS .. 2 EPI_WARPS - 1 rescore what the warp EPI_WARPS below found
+    const bool producer_warp = warp == 2 * EPI_WARPS;                 // MMA issue (and the copies without TMA_WARP)
+    const bool copy_warp = C::TMA_WARP && warp == 2 * EPI_WARPS + 1;  // the copies with TMA_WARP
     // Rows: positions [first_row, first_row + n_rows) of rows_perm (point indices; the positions
     // themselves when rows_perm is null), from dev_sizes = {first_row, n_rows, n_items} on the
     // device or {0, n_query, ceil(n_query / ROWS)}; work item g is positions
@@ -456,11 +523,11 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(&b_full[s], 1);
-            mbar_init(&b_empty[s], 1);  // the MMA commit: the epilogue never reads a stage
+            mbar_init(&b_empty[s], 1);  // the MMA commit: nothing else reads a stage
         }
         // accumulator barriers: one pair per TMEM buffer, or with PAIR one pair per query tile (its
         // 256 columns are released by its own four warps, so the MMAs of one query tile's next
-        // stage overlap the other tile's epilogue)
+        // stage overlap the other tile's screen)
         for (int b = 0; b < (C::PAIR ? QTILES : C::NBUF); ++b) {
             mbar_init(&t_full[b], 1);
             mbar_init(&t_empty[b], C::PAIR ? 4 : EPI_WARPS);
@@ -499,6 +566,10 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
         __syncthreads();
         const int item = *s_item;
         const bool stop = (item >= n_items) || (*s_abort != 0);
+        if (threadIdx.x < EPI_WARPS) {
+            ring_head[threadIdx.x] = 0;
+            ring_tail[threadIdx.x] = 0;
+        }
         __syncthreads();
         if (stop) break;
         const int64_t desc = items.order ? (int64_t)items.order[item] : -1;  // the item's descriptor
@@ -642,166 +713,69 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                 }
             }
             __syncwarp();
-        } else {
-            // ---------------- epilogue warps ----------------
+        } else if (warp < EPI_WARPS) {
+            // ---------------- screening warps ----------------
             // warp w serves query tile w / 4 through TMEM lane quadrant w % 4 (a warp reaches the
             // lanes of its own quadrant only)
             const int qtw = warp >> 2, quad = warp & 3;
             // query row in the work item.  PAIR: the rows are dealt out to the warps in turn (row r
             // to warp r mod EPI_WARPS), so that the candidates of a spatially clustered run of rows
-            // spread over the warps that must release an accumulator together (-1 % at d = 16; the
-            // other shapes keep runs of 32)
+            // spread over the warps that must release an accumulator together (the other shapes keep
+            // runs of 32)
             const int row = C::PAIR ? lane * EPI_WARPS + warp : warp * 32 + lane;
             const bool active = row < n_item_rows;
             const int64_t q = active ? point_of(q0 + row) : 0;  // the point's index
             const int64_t limit = active ? limit_of(q) : 0;
-            float qo[D], qc[D];
-            float nq = 0.f;
+            float *my_thr = row_thr + warp * 32 + lane;
+            {
+                float qc[D];
+                float nq = 0.f;
 #pragma unroll
-            for (int f = 0; f < D; ++f) {
-                qo[f] = active ? qs[q * C::DP + f] : 0.f;
-                const float cf = n_ref > 0 ? (float)(acc[f] / (double)n_ref) : 0.f;
-                qc[f] = qo[f] - cf;
-                nq = fmaf(qc[f], qc[f], nq);
-            }
-            const float span = sqrtf(nq) * 1.0001f + rmax;
-            const float eps = C::EPS * span * span;
-            {  // query operand row: A' = [a_hi | a_hi | a_lo], a = [qc, 1]
+                for (int f = 0; f < D; ++f) {
+                    const float cf = n_ref > 0 ? (float)(acc[f] / (double)n_ref) : 0.f;
+                    qc[f] = (active ? qs[q * C::DP + f] : 0.f) - cf;
+                    nq = fmaf(qc[f], qc[f], nq);
+                }
+                const float span = sqrtf(nq) * 1.0001f + rmax;
+                const float eps = C::EPS * span * span;
+                // query operand row: A' = [a_hi | a_hi | a_lo], a = [qc, 1]
                 float a[C::U];
 #pragma unroll
                 for (int f = 0; f < D; ++f) a[f] = active ? qc[f] : 0.f;
                 a[D] = active ? 1.f : 0.f;
                 put_split_row<C>(sA + qtw * C::A_TILE, quad * 32 + lane, QT, 2, a);
+                fence_proxy_async_smem();
+                mbar_arrive(a_ready);
+                // a proven upper bound of the row's m-th distance (seeded prefix search), else +inf; rows
+                // past the last query never take candidates
+                const float seed = (active && seeds) ? seeds[q] : pos_inf<float>();
+                *my_thr = active ? fminf((seed - nq) + eps, pos_inf<float>()) : neg_inf<float>();  // NaN: +inf
+                const int slot = warp * 32 + lane;
+                row_worst[slot] = seed;
+                row_norm[slot] = nq;
+                row_eps[slot] = eps;
+                row_limit[slot] = (int32_t)limit;
+                row_point[slot] = active ? (int32_t)q : -1;
             }
-            fence_proxy_async_smem();
-            mbar_arrive(a_ready);
-
-            // this warp's rows: row rr's heap at heap[rr * HS .. + m)
-            uint64_t *heap = H + (warp * 32) * HS;
-            for (int rr = 0; rr < 32; ++rr) heap[rr * HS + lane] = kEmptyKey;
-            uint64_t *qk = reinterpret_cast<uint64_t *>(qbase) + warp * QCAP;  // queued keys
-            uint8_t *qr = qbase + EPI_WARPS * QCAP * 8 + warp * QCAP;           // their rows
             __syncwarp();
-            // rows past the last query never take candidates
-            const float tq_off = active ? pos_inf<float>() : neg_inf<float>();
-            // a proven upper bound of the row's m-th distance (seeded prefix search), else +inf
-            const float seed_r = (active && seeds) ? seeds[q] : pos_inf<float>();
-            float worst = seed_r;  // min(seed, distance of the heap root = m-th best so far)
-            float tq = fminf((worst - nq) + eps, tq_off);  // screening threshold of this row
-            int qcount = 0;
-            // insert the queued entries: 32 at a time, each lane into its entry's row heap; entries
-            // of one row go in one after the other (match_any groups), so any order gives the same heap set
-            auto drain = [&]() {
-                __syncwarp();
-                for (int base = 0; base < qcount; base += 32) {
-                    const int e = base + lane;
-                    bool pend = e < qcount;
-                    const int r = pend ? (int)qr[e] : 32 + lane;  // idle lanes: distinct dummy rows
-                    const uint64_t x = pend ? qk[e] : 0;
-                    const unsigned grp = __match_any_sync(FULL, r);
-                    unsigned todo = __ballot_sync(FULL, pend);
-                    while (todo) {
-                        const unsigned g = grp & todo;
-                        if (pend && (g & (0u - g)) == (1u << lane)) {
-                            heap_insert(heap + r * HS, m, x);
-                            pend = false;
-                        }
-                        __syncwarp();
-                        todo = __ballot_sync(FULL, pend);
-                    }
-                }
-                qcount = 0;
-                worst = fminf(__uint_as_float((uint32_t)(heap[lane * HS] >> 32)), seed_r);
-                tq = fminf((worst - nq) + eps, tq_off);
-            };
-
-            // screened candidates waiting for their exact distance: ref position << 5 | row
-            uint64_t *cq = cqbase + warp * CQCAP;
-            int ccount = 0;
-            // rescore queued candidates, one per lane (batches of 32; all of them when `all`, else
-            // the whole batches, the rest moving to the front): the ref's exact coordinates and point
-            // index from its tile record in global memory, the row's query coordinates, bound and
-            // limit by shuffles from the lane that owns the row; survivors of the row's current bound
-            // are queued as keys
-            auto rescore = [&](bool all) {
-                __syncwarp();
-                const int n_do = all ? ccount : (ccount & ~31);
-                for (int base = 0; base < n_do; base += 32) {
-                    if (qcount > QCAP - 32) drain();
-                    const int e = base + lane;
-                    const bool has = e < n_do;
-                    const uint64_t c = has ? cq[e] : 0;
-                    const int r = (int)(c & 31u);
-                    const int64_t jp = (int64_t)(c >> 5);  // the ref's position among the tiles
-                    float qv[D];
-#pragma unroll
-                    for (int f = 0; f < D; ++f) qv[f] = __shfl_sync(FULL, qo[f], r);
-                    const float worst_r = __shfl_sync(FULL, worst, r);
-                    const long long limit_r = __shfl_sync(FULL, (long long)limit, r);
-                    bool keep = false;
-                    uint64_t key = 0;
-                    if (has) {
-                        const int col = (int)(jp & (RT - 1));
-                        const unsigned char *rec = tiles_g + (jp / RT) * C::TILE_BYTES;
-                        // the oracle's arithmetic: ((x0 - q0)^2 + (x1 - q1)^2) + ..., each step rounded
-                        const float4 *rp4 = reinterpret_cast<const float4 *>(rec + C::OP_BYTES) + col * (C::DP / 4);
-                        float rv[C::DP];
-#pragma unroll
-                        for (int f4 = 0; f4 < C::DP / 4; ++f4) {
-                            const float4 t = __ldg(rp4 + f4);
-                            rv[4 * f4] = t.x;
-                            rv[4 * f4 + 1] = t.y;
-                            rv[4 * f4 + 2] = t.z;
-                            rv[4 * f4 + 3] = t.w;
-                        }
-                        int64_t jo = jp;  // index-order tiles: the position is the point index
-                        if (pruned) {
-                            if constexpr (C::IX_MODE == 1) jo = __float_as_int(rv[C::DP - 1]);
-                            else if constexpr (C::IX_MODE == 2)
-                                jo = __ldg(reinterpret_cast<const int32_t *>(rec + C::OP_BYTES + C::EX_BYTES) + col);
-                            else jo = __ldg(ref_perm + jp);
-                        }
-                        const float t0 = sub_rn(rv[0], qv[0]);
-                        float d2 = mul_rn(t0, t0);
-#pragma unroll
-                        for (int f = 1; f < D; ++f) {
-                            const float tf = sub_rn(rv[f], qv[f]);
-                            d2 = add_rn(d2, mul_rn(tf, tf));
-                        }
-                        keep = d2 <= worst_r && jo < (int64_t)limit_r;  // NaN never kept
-                        key = (uint64_t)__float_as_uint(d2) << 32 | (uint32_t)jo;
-                    }
-                    const unsigned mk = __ballot_sync(FULL, keep);
-                    if (keep) {
-                        const int pos = qcount + __popc(mk & ((1u << lane) - 1u));
-                        qk[pos] = key;
-                        qr[pos] = (uint8_t)r;
-                    }
-                    qcount += __popc(mk);
-                }
-                const int rest = ccount - n_do;  // < 32
-                __syncwarp();
-                const uint64_t mv = lane < rest ? cq[n_do + lane] : 0;
-                __syncwarp();
-                if (lane < rest) cq[lane] = mv;
-                __syncwarp();
-                ccount = rest;
-            };
+            uint4 *my_mask = ring_mask + warp * RING;
+            uint32_t *my_meta = ring_meta + warp * RING;
+            uint32_t head = 0, tail = 0;  // warp-uniform; tail: what the rescoring warp is known to have taken
 
             // the next stage's list entries are loaded one stage ahead (global loads that would
             // otherwise sit on the path from the accumulator to the screen)
             int64_t nx[C::TPS];
 #pragma unroll
             for (int h = 0; h < C::TPS; ++h) nx[h] = (pruned && (uint32_t)h < ntiles) ? (int64_t)tl[h] : 0;
-            for (uint32_t u = 0; u < nstg; ++u) {
+            for (uint32_t u = 0; u < nstg && !aborted; ++u) {
                 const uint32_t g = G + u;
                 const uint32_t b = g % C::NBUF;
                 const uint32_t t0 = u * C::TPS;                                  // the stage's first tile
                 const int nh = (int)min((uint32_t)C::TPS, ntiles - t0);           // tiles in the stage
-                int64_t j0[C::TPS];                                               // first ref position of each
+                int64_t tile[C::TPS];                                             // their records
 #pragma unroll
                 for (int h = 0; h < C::TPS; ++h) {
-                    j0[h] = (pruned ? nx[h] : (int64_t)(tfirst + t0 + h)) * RT;
+                    tile[h] = pruned ? nx[h] : (int64_t)(tfirst + t0 + h);
                     const uint32_t tn = t0 + C::TPS + h;
                     if (pruned && tn < ntiles) nx[h] = (int64_t)tl[tn];
                 }
@@ -812,9 +786,11 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                     break;
                 }
                 tc_fence_after();
+                // the rescoring warp lowers the threshold as it goes; an older value passes more
+                const float tq = *reinterpret_cast<volatile float *>(my_thr);
                 // 1) screen each tile of the stage: the minimum of each group of 8 columns (16 per row),
-                //    the accumulator read in four 32-column chunks, each loading while the previous one
-                //    is reduced; one vote per tile, since most tiles give no row of the warp a
+                //    the accumulator read 16 columns at a time, each load in flight while the previous
+                //    one is reduced; one vote per tile, since most tiles give no row of the warp a
                 //    candidate.  A tile that does reads its passing chunks again (the accumulator is
                 //    held until every tile of the stage is screened) for the candidate masks.
                 uint32_t cmk[C::TPS][4];
@@ -828,29 +804,27 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                     const uint32_t taddr =
                         tmem_base + ((uint32_t)(quad * 32) << 16) + b * C::BUF_COLS + qtw * C::RS + h * RT;
                     float gm[16];
-                    auto group_mins = [&](const uint32_t (&v)[32], int c) {
+                    uint32_t va[16], vb[16];
+#define NNGP_V(v, k) __uint_as_float(v[gi * 8 + (k)])
+                    auto group_mins = [&](const uint32_t (&v)[16], int c) {
 #pragma unroll
-                        for (int gi = 0; gi < 4; ++gi) {
-#define NNGP_V(k) __uint_as_float(v[gi * 8 + (k)])
-                            gm[c * 4 + gi] = fminf(min3f(NNGP_V(0), NNGP_V(1), NNGP_V(2)),
-                                                   min3f(NNGP_V(3), NNGP_V(4), fminf(NNGP_V(5), fminf(NNGP_V(6), NNGP_V(7)))));
-#undef NNGP_V
-                        }
+                        for (int gi = 0; gi < 2; ++gi)
+                            gm[c * 2 + gi] =
+                                fminf(min3f(NNGP_V(v, 0), NNGP_V(v, 1), NNGP_V(v, 2)),
+                                      min3f(NNGP_V(v, 3), NNGP_V(v, 4), fminf(NNGP_V(v, 5), fminf(NNGP_V(v, 6), NNGP_V(v, 7)))));
                     };
-                    uint32_t va[32], vb[32];
-                    tmem_ld32_nowait(taddr, va);
+                    tmem_ld16_nowait(taddr, va);
                     tmem_wait_ld(va);
-                    tmem_ld32_nowait(taddr + 32, vb);
-                    group_mins(va, 0);
-                    tmem_wait_ld(vb);
-                    tmem_ld32_nowait(taddr + 64, va);
-                    group_mins(vb, 1);
-                    tmem_wait_ld(va);
-                    tmem_ld32_nowait(taddr + 96, vb);
-                    group_mins(va, 2);
-                    tmem_wait_ld(vb);
-                    group_mins(vb, 3);
-                    float cmin[4];  // minimum of each chunk
+#pragma unroll
+                    for (int c = 0; c < 8; c += 2) {
+                        tmem_ld16_nowait(taddr + 16 * (c + 1), vb);
+                        group_mins(va, c);
+                        tmem_wait_ld(vb);
+                        if (c + 2 < 8) tmem_ld16_nowait(taddr + 16 * (c + 2), va);
+                        group_mins(vb, c + 1);
+                        if (c + 2 < 8) tmem_wait_ld(va);
+                    }
+                    float cmin[4];  // minimum of each 32 columns
 #pragma unroll
                     for (int c = 0; c < 4; ++c) cmin[c] = fminf(fminf(gm[4 * c], gm[4 * c + 1]), fminf(gm[4 * c + 2], gm[4 * c + 3]));
                     has_t[h] = __any_sync(FULL, fminf(fminf(cmin[0], cmin[1]), fminf(cmin[2], cmin[3])) < tq);
@@ -858,30 +832,37 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
                             if (__any_sync(FULL, cmin[c] < tq)) {  // warp-uniform: the load is collective
-                                tmem_ld32_nowait(taddr + 32 * c, va);
+                                tmem_ld16_nowait(taddr + 32 * c, va);
+                                tmem_ld16_nowait(taddr + 32 * c + 16, vb);
                                 tmem_wait_ld(va);
+                                tmem_wait_ld(vb);
                                 uint32_t cm = 0;
 #pragma unroll
-                                for (int gi = 0; gi < 4; ++gi) {
+                                for (int gi = 0; gi < 2; ++gi) {
                                     if (gm[4 * c + gi] < tq) {  // only groups whose minimum passes
 #pragma unroll
-                                        for (int k = 0; k < 8; ++k)
-                                            cm |= (__uint_as_float(va[gi * 8 + k]) < tq ? 1u : 0u) << (gi * 8 + k);
+                                        for (int k = 0; k < 8; ++k) cm |= (NNGP_V(va, k) < tq ? 1u : 0u) << (gi * 8 + k);
+                                    }
+                                    if (gm[4 * c + 2 + gi] < tq) {
+#pragma unroll
+                                        for (int k = 0; k < 8; ++k) cm |= (NNGP_V(vb, k) < tq ? 1u : 0u) << (16 + gi * 8 + k);
                                     }
                                 }
                                 cmk[h][c] = cm;
                             }
                         }
                     }
+#undef NNGP_V
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&t_empty[tb]);
+                // 2) hand the rows with candidates to the rescoring warp: one entry per row and tile
 #pragma unroll
                 for (int h = 0; h < C::TPS; ++h) {
                     if (!has_t[h]) continue;
                     {  // columns with j < limit only (pruned: positions < n_ref; the index test is per candidate)
-                        const int64_t room = (pruned ? n_ref : limit) - j0[h];
+                        const int64_t room = (pruned ? n_ref : limit) - tile[h] * RT;
                         if (room < RT) {
 #pragma unroll
                             for (int c = 0; c < 4; ++c) {
@@ -890,39 +871,182 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                             }
                         }
                     }
-                    // 2) queue the tile's candidates (ref position, row): each lane walks its own
-                    //    (column by column, chunks in order), one per warp iteration; whole batches of
-                    //    32 are rescored as soon as they are queued
-                    uint64_t lo = (uint64_t)cmk[h][0] | (uint64_t)cmk[h][1] << 32;
-                    uint64_t hi = (uint64_t)cmk[h][2] | (uint64_t)cmk[h][3] << 32;
-                    while (__any_sync(FULL, (lo | hi) != 0)) {
-                        if (ccount > CQCAP - 32) rescore(false);
-                        const bool has = (lo | hi) != 0;
-                        int col = 0;
-                        if (has) {
-                            const bool use_lo = lo != 0;  // branch-free pick of the lowest remaining column
-                            const uint64_t w = use_lo ? lo : hi;
-                            col = __ffsll((long long)w) - 1 + (use_lo ? 0 : 64);
-                            const uint64_t w2 = w & (w - 1);
-                            lo = use_lo ? w2 : lo;
-                            hi = use_lo ? hi : w2;
+                    const bool has = (cmk[h][0] | cmk[h][1] | cmk[h][2] | cmk[h][3]) != 0u;
+                    const unsigned mk = __ballot_sync(FULL, has);
+                    const uint32_t cnt = (uint32_t)__popc(mk);
+                    if (cnt == 0) continue;
+                    if (head + cnt - tail > (uint32_t)RING) {  // warp-uniform: wait for places
+                        bool ok = true;
+                        if (lane == 0)
+                            ok = poll_bounded(ring_tail + warp, wait_ns, 1, tail,
+                                              [&](uint32_t v) { return head + cnt - v <= (uint32_t)RING; });
+                        tail = __shfl_sync(FULL, tail, 0);
+                        if (!__shfl_sync(FULL, ok, 0)) {
+                            aborted = true;
+                            break;
                         }
-                        const unsigned mk = __ballot_sync(FULL, has);
-                        if (has) cq[ccount + __popc(mk & ((1u << lane) - 1u))] = (uint64_t)(j0[h] + col) << 5 | (uint32_t)lane;
-                        ccount += __popc(mk);
+                    }
+                    if (has) {
+                        const uint32_t at = (head + (uint32_t)__popc(mk & ((1u << lane) - 1u))) % RING;
+                        my_mask[at] = make_uint4(cmk[h][0], cmk[h][1], cmk[h][2], cmk[h][3]);
+                        my_meta[at] = (uint32_t)tile[h] << 5 | (uint32_t)lane;
+                    }
+                    head += cnt;
+                    __syncwarp();
+                    if (lane == 0) st_release(ring_head + warp, head);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) st_release(ring_head + warp, head | RING_DONE | (aborted ? RING_ABORT : 0u));
+        } else {
+            // ---------------- rescoring warps ----------------
+            // warp EPI_WARPS + w takes the entries of screening warp w: exact distances of the passing columns,
+            // inserted into the rows' lists, whose bounds lower the rows' screening thresholds
+            const int w = warp - EPI_WARPS;
+            float *ld = list_d + w * 32 * DS;
+            uint32_t *li = list_i + w * 32 * IS;
+            for (int rr = 0; rr < 32; ++rr) {
+                ld[rr * DS + lane] = lane < m ? pos_inf<float>() : neg_inf<float>();
+                if (lane < 8) ld[rr * DS + 32 + lane] = 4 * lane < m ? pos_inf<float>() : neg_inf<float>();
+                li[rr * IS + lane] = 0xFFFFFFFFu;
+            }
+            row_largest[w * 32 + lane] = 0;
+            __syncwarp();
+            const uint4 *my_mask = ring_mask + w * RING;
+            const uint32_t *my_meta = ring_meta + w * RING;
+            uint32_t tail = 0, seen = 0;  // entries taken; the last head read
+            while (true) {
+                const bool done = (seen & RING_DONE) != 0u;
+                const uint32_t avail = (seen & ~(RING_DONE | RING_ABORT)) - tail;
+                if (!(avail >= (uint32_t)RING_MIN || (done && avail > 0u))) {
+                    if (done) break;
+                    // the screening warp may find nothing in all of the item's stages: the limit is the sum of
+                    // its own waits, each of which ends in RING_DONE | RING_ABORT when it runs out
+                    bool ok = true;
+                    if (lane == 0)
+                        ok = poll_bounded(ring_head + w, wait_ns, nstg + 2, seen, [&](uint32_t v) {
+                            return (v & RING_DONE) != 0u || (v & ~RING_ABORT) - tail >= (uint32_t)RING_MIN;
+                        });
+                    seen = __shfl_sync(FULL, seen, 0);
+                    if (!__shfl_sync(FULL, ok, 0)) {
+                        aborted = true;
+                        break;
+                    }
+                    continue;
+                }
+                const uint32_t cnt = min(avail, 32u);
+                uint64_t lo = 0, hi = 0;
+                uint32_t meta = 0;
+                if ((uint32_t)lane < cnt) {
+                    const uint32_t at = (tail + (uint32_t)lane) % RING;
+                    const uint4 mk = my_mask[at];
+                    lo = (uint64_t)mk.x | (uint64_t)mk.y << 32;
+                    hi = (uint64_t)mk.z | (uint64_t)mk.w << 32;
+                    meta = my_meta[at];
+                }
+                __syncwarp();
+                tail += cnt;
+                if (lane == 0) st_release(ring_tail + w, tail);  // the places are free again
+                const int r = (int)(meta & 31u), slot = w * 32 + r;
+                const int32_t limit_r = row_limit[slot];
+                const float nq = row_norm[slot], eps = row_eps[slot];
+                float qv[C::DP];
+                {
+                    const float4 *q4 = reinterpret_cast<const float4 *>(qs + (int64_t)max(row_point[slot], 0) * C::DP);
+#pragma unroll
+                    for (int v = 0; v < C::DP / 4; ++v) {
+                        const float4 t = __ldg(q4 + v);
+                        qv[4 * v] = t.x;
+                        qv[4 * v + 1] = t.y;
+                        qv[4 * v + 2] = t.z;
+                        qv[4 * v + 3] = t.w;
                     }
                 }
-                if (ccount >= 32) rescore(false);
-                if (qcount >= DRAIN_AT) drain();
+                const unsigned same_row = __match_any_sync(FULL, (uint32_t)lane < cnt ? r : 32 + lane);
+                const unsigned char *rec = tiles_g + (int64_t)(meta >> 5) * C::TILE_BYTES;
+                // each lane walks its entry's columns, one per iteration.  Up to 8 features the next column's
+                // coordinates and index are asked for before the current one goes into its list; from 20 on
+                // right after that (n = 300,000, d = 24: 9.4 ms against 9.7 either other way); with 12 and 16
+                // at the top of the iteration, where they hold no register across the insertions (d = 16,
+                // n = 200,000: 9.4 ms against 10.2 and 10.7)
+                constexpr bool AT_TOP = QTILES == 2, AHEAD = D <= 8;
+                float rv[C::DP];
+                int64_t jo = 0;
+                bool has = false;
+                auto next_column = [&]() {
+                    has = (lo | hi) != 0;
+                    if (!has) return;
+                    const bool use_lo = lo != 0;  // branch-free pick of the lowest remaining column
+                    const uint64_t wd = use_lo ? lo : hi;
+                    const int col = __ffsll((long long)wd) - 1 + (use_lo ? 0 : 64);
+                    const uint64_t w2 = wd & (wd - 1);
+                    lo = use_lo ? w2 : lo;
+                    hi = use_lo ? hi : w2;
+                    jo = (int64_t)(meta >> 5) * RT + col;  // index-order tiles: the position is the point index
+                    if (pruned) {
+                        if constexpr (C::IX_MODE == 2)
+                            jo = __ldg(reinterpret_cast<const int32_t *>(rec + C::OP_BYTES + C::EX_BYTES) + col);
+                        else if constexpr (C::IX_MODE == 0) jo = __ldg(ref_perm + jo);
+                    }
+                    const float4 *rp4 = reinterpret_cast<const float4 *>(rec + C::OP_BYTES) + col * (C::DP / 4);
+#pragma unroll
+                    for (int v = 0; v < C::DP / 4; ++v) {
+                        const float4 t = __ldg(rp4 + v);
+                        rv[4 * v] = t.x;
+                        rv[4 * v + 1] = t.y;
+                        rv[4 * v + 2] = t.z;
+                        rv[4 * v + 3] = t.w;
+                    }
+                };
+                if constexpr (!AT_TOP) next_column();
+                while (__any_sync(FULL, AT_TOP ? (lo | hi) != 0 : has)) {
+                    if constexpr (AT_TOP) next_column();
+                    bool keep = false;
+                    float d2 = 0.f;
+                    uint32_t jk = 0;
+                    if (has) {
+                        // the oracle's arithmetic: ((x0 - q0)^2 + (x1 - q1)^2) + ..., each step rounded
+                        const float t0 = sub_rn(rv[0], qv[0]);
+                        d2 = mul_rn(t0, t0);
+#pragma unroll
+                        for (int f = 1; f < D; ++f) {
+                            const float tf = sub_rn(rv[f], qv[f]);
+                            d2 = add_rn(d2, mul_rn(tf, tf));
+                        }
+                        if constexpr (C::IX_MODE == 1) {
+                            if (pruned) jo = __float_as_int(rv[C::DP - 1]);
+                        }
+                        jk = (uint32_t)jo;
+                        keep = d2 <= row_worst[slot] && jo < (int64_t)limit_r;  // NaN never kept
+                    }
+                    if constexpr (AHEAD) next_column();
+                    // into the rows' lists; entries of one row go in one after the other, so any order gives
+                    // the same sets
+                    unsigned todo = __ballot_sync(FULL, keep);
+                    while (todo) {
+                        const unsigned grp = same_row & todo;
+                        if (keep && (grp & (0u - grp)) == (1u << lane)) {
+                            const float top = list_insert(list_d + slot * DS, list_i + slot * IS, row_largest + slot, d2, jk);
+                            if (top < row_worst[slot]) {
+                                row_worst[slot] = top;
+                                *reinterpret_cast<volatile float *>(row_thr + slot) = fminf((top - nq) + eps, pos_inf<float>());
+                            }
+                            keep = false;
+                        }
+                        __syncwarp();
+                        todo = __ballot_sync(FULL, keep);
+                    }
+                    if constexpr (!AT_TOP && !AHEAD) next_column();
+                }
             }
-            // write this warp's rows: each heap sorted ascending across the warp (bitonic, keys unique
+            if (seen & RING_ABORT) aborted = true;
+            // write this warp's rows: each list sorted ascending across the warp (bitonic, keys unique
             // except empty slots), index -1 for empty slots
             if (!aborted) {
-                if (ccount > 0) rescore(true);
-                if (qcount > 0) drain();
                 __syncwarp();
                 for (int rr = 0; rr < 32; ++rr) {
-                    uint64_t x = lane < m ? heap[rr * HS + lane] : ~0ull;
+                    uint64_t x = lane < m ? (uint64_t)__float_as_uint(ld[rr * DS + lane]) << 32 | li[rr * IS + lane]
+                                          : ~0ull;
 #pragma unroll
                     for (int k = 2; k <= 32; k <<= 1) {
 #pragma unroll
@@ -932,7 +1056,7 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                             x = take_min ? (o < x ? o : x) : (o > x ? o : x);
                         }
                     }
-                    const int64_t rq = C::PAIR ? rr * EPI_WARPS + warp : warp * 32 + rr;  // item row of row rr
+                    const int64_t rq = C::PAIR ? rr * EPI_WARPS + w : w * 32 + rr;  // item row of row rr
                     if (out_slot >= 0) {
                         items.partial[((int64_t)out_slot * C::ROWS + rq) * 32 + lane] = x;
                     } else if (rq < n_item_rows && lane < m) {
@@ -1036,7 +1160,7 @@ __global__ void __launch_bounds__(THREADS) tc_layout_selftest_kernel(const float
     }
 }
 
-// d 12 and 16 fill an SM with one CTA: two query tiles per work item give it 8 epilogue warps
+// d 12 and 16 fill an SM with one CTA: two query tiles per work item give it 8 screening and 8 rescoring warps
 // and halve the ref-tile stream per query
 template <int D, int QTILES = (D == 12 || D == 16) ? 2 : 1> TcVariant tc_make() {
     using C = Cfg<D, QTILES>;

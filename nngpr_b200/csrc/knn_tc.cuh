@@ -32,7 +32,7 @@ struct TcVariant {
     TcBuildFn build = nullptr;
     int smem = 0, stage_bytes = 0, dp = 0;
     int ctas_per_sm = 1;     // CTAs the shared memory of one SM holds (the kernel's launch bounds)
-    int threads = 160;       // epilogue warps (4 per query tile) + the producer/MMA warp
+    int threads = 352;       // screening and rescoring warps (4 each per query tile) + the MMA warp + the copy warp
     int rows_per_item = 128;  // queries per work item (128 per query tile)
 };
 

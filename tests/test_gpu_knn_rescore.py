@@ -1,0 +1,37 @@
+"""The rescoring warps of the tensor-core search: bit-exact lists against the oracle where every column of every
+tile is a candidate (their rings run full), where equal distances decide, and at the sizes of a tile."""
+import numpy as np
+import pytest
+import torch
+
+from nngpr_b200 import ops
+from oracle import nngp_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def run(monkeypatch, ref, q, m, cut):
+    monkeypatch.setenv('NNGP_KNN_KERNEL', 'tc')
+    r = torch.from_numpy(np.ascontiguousarray(ref, dtype=np.float32)).cuda()
+    qq = r if q is ref else torch.from_numpy(np.ascontiguousarray(q, dtype=np.float32)).cuda()
+    flags = ops.new_flags(r.device)
+    out = ops.knn(r, qq, m, cut, None, flags=flags).cpu().numpy()
+    assert int(flags.item()) == 0
+    return out
+
+
+@pytest.mark.parametrize('d', [1, 3, 4, 8, 10, 16, 18, 24])
+@pytest.mark.parametrize('m', [1, 5, 31, 32])
+def test_rescoring_matches_oracle(monkeypatch, d, m):
+    rng = np.random.default_rng(100 * d + m)
+    # each ref nearer to the origin than the one before it: no bound excludes anything
+    r = rng.normal(size=(2100, d))
+    r *= np.linspace(3, 0.1, len(r))[:, None] / np.linalg.norm(r, axis=1)[:, None]
+    q = rng.normal(scale=1e-3, size=(290, d))
+    for n in (2100, 129, 127):
+        for cut in (None, -40):
+            assert np.array_equal(run(monkeypatch, r[:n], q, m, cut), O.knn(r[:n], q, m, cut, None, np.float32))
+    # lattice points, and all points equal: ties at the m-th distance, the lower indices win
+    x = rng.integers(0, 2, (1500, d)).astype(np.float64)
+    for pts in (x, x[::-1].copy(), np.ones((700, d))):
+        assert np.array_equal(run(monkeypatch, pts, pts, m, 0), O.knn(pts, pts, m, 0, None, np.float32))
