@@ -36,7 +36,7 @@
 //     issue slots both below half busy).  While one warp did both, the accumulator waited out every
 //     candidate's loads and heap steps, half of the kernel's time at d = 16.  Of one search, one warp for
 //     both -> two: 22.7 -> 20.6 ms (d = 16, n = 1M, clustered), 4.3 -> 3.7 ms (d = 3, n = 434,874), 17.0 -> 15.0 ms
-//     (d = 8, two searches' kernels), 511 -> 368 us (16,384 queries in 50,000, d = 18); from 9.2 to 9.4 ms at d = 24, n = 300,000;
+//     (d = 8, two searches' kernels), 511 -> 368 us (16,384 queries in 16,599, d = 18); from 9.2 to 9.4 ms at d = 24, n = 300,000;
 //   * mbarriers: b_full (TMA -> MMA), b_empty (MMA commit -> producer), t_full (MMA commit ->
 //     screen), t_empty (screening warps -> MMA), a_ready (query operand written by the screening warps
 //     -> MMA); the rings' two counters each are plain words, released and acquired.  Every wait is bounded; on a timeout the CTA raises
@@ -120,8 +120,10 @@ struct Cfg {
     static constexpr int ROW_BYTES = ROWS * 7 * 4;  // per row: threshold, bound, norm, eps, limit, point, largest
     static constexpr int BAR_BYTES = 256;
     static constexpr int FIXED = ALIGN + A_BYTES + LIST_BYTES + RING_BYTES + ROW_BYTES + BAR_BYTES;  // ALIGN: base slack
-    // two CTAs per SM where each holds at least 2 stages: more warps per scheduler
-    static constexpr int ST2 = (112 * 1024 - FIXED) / STAGE_BYTES;
+    // two CTAs per SM where each holds at least 2 stages: more warps per scheduler.  113 KB each is all of an SM's
+    // 228 KB but the 1 KB that the system keeps per CTA; a third stage at d = 8 and 20 (112 KB: two) took one search
+    // of n = 434,874, d = 8 from 16.7 to 15.6 ms
+    static constexpr int ST2 = (113 * 1024 - FIXED) / STAGE_BYTES;
     static constexpr int ST1 = (231936 - FIXED) / STAGE_BYTES;  // of 232,448 bytes
     static constexpr int CTAS_PER_SM = ST2 >= 2 ? 2 : 1;
     static constexpr int STN = CTAS_PER_SM == 2 ? ST2 : ST1;
