@@ -531,8 +531,7 @@ def local_flops_per_point(m, d, n_theta):
 def our_launches_per_step(n, d, m):
     """Kernels of this library one fit step launches (CUB's sort and scan kernels not counted):
     scale, centre sums and tile build; per seed level (the prefixes n, n/8, ... of at least
-    8,192 points) bounds, two x (Morton keys, inverse, coordinate gather), cross positions and
-    the seed kernel; the pruned search's planning (21, the index-order fallback's two
+    8,192 points) bounds, Morton keys, places and coordinates, cross positions and the seed kernel; the pruned search's planning (21, the index-order fallback's two
     included), a second tile build, two search
     launches and two merges, or one search launch; the local systems and the final sum.  Below the
     seeded sizes the direct search: scale and one launch."""
@@ -549,7 +548,7 @@ def our_launches_per_step(n, d, m):
     search = (21 + 1 + 2 + 2) if pruned else 1
     if pruned and d >= 9 and n >= 131072:  # cells: k-means steps, directions, assignment, two reaches
         search += 10
-    return 3 + 9 * levels + search + 2
+    return 3 + 5 * levels + search + 2
 
 
 def run_plain(args, torch, x32, y64, xq32, p, flags, flush, lml_ours):

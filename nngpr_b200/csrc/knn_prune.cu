@@ -43,6 +43,7 @@
 #include "common.cuh"
 #include "knn_cells.cuh"
 #include "knn_prune.cuh"
+#include "knn_seed.cuh"
 
 namespace nngp {
 namespace prune {
@@ -243,14 +244,14 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(int64_t n, const uint
                                                            const int32_t *__restrict__ pos0,
                                                            const uint64_t *__restrict__ keys0,
                                                            const unsigned long long *__restrict__ pruned_cnt, int d,
-                                                           int bits, int32_t *__restrict__ headpos) {
+                                                           int bits, int drop, int32_t *__restrict__ headpos) {
     unsigned long long total = 0;
     for (int b = 0; b < kBands; ++b) total += pruned_cnt[b];
     auto cell_of = [&](int64_t r, int b) -> uint64_t {
         if (use_cells) return (skeys[r] >> kPosBits) & ((1u << kCellBits) - 1u);
         const int L = cell_level(pruned_cnt[b], d, bits);
         const int shift = d * (bits - L);
-        const uint64_t key = keys0[pos0[rows[r]]];
+        const uint64_t key = keys0[pos0[rows[r]]] << drop;
         return shift >= 64 ? 0ull : key >> shift;
     };
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
@@ -964,7 +965,7 @@ nngp_status build(const float *xs, int64_t n, int64_t row_lo, int64_t row_hi, in
 
     // groups: segments of one band and one octree cell, cut every G rows
     segment_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, dk.Current(), L.n_cells > 0 ? 1 : 0, rows, pos0, keys0, pcnt, d, bits,
-                                                        headpos);
+                                                        seed::key_drop(d), headpos);
     NNGP_CUDA_TRY(cudaGetLastError());
     need = 0;
     NNGP_CUDA_TRY(cub::DeviceScan::InclusiveScan(nullptr, need, headpos, seg_start, cub::Max(), (int)n, stream));

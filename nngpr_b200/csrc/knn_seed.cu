@@ -17,9 +17,9 @@
 // without seeds; only the number of candidates changes.
 //
 // Steps (all on the caller's stream): per-dimension bounds of the finite coordinates; 64-bit
-// Morton keys (b = min(10, 64 / d) bits per dimension, interleaved) for both grids; a radix sort
-// of each (CUB, key/index pairs); the inverse permutations; then one warp per point, points
-// taken in curve order so that neighbouring warps read the same windows.
+// Morton keys (b = min(10, 64 / d) bits per dimension, interleaved) for both grids; one radix
+// sort of both (CUB, key/index pairs); the inverse permutations and the coordinates in either order; then one
+// warp per point, points taken in curve order so that neighbouring warps read the same windows.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
@@ -70,50 +70,84 @@ __global__ void __launch_bounds__(kThreads) bounds_kernel(const float *__restric
     }
 }
 
-// Morton key of every point on grid `curve` (0: cells aligned with the bounds; 1: shifted by
-// 1.23 % of the extent in every dimension); idx = 0..n-1.
-__global__ void __launch_bounds__(kThreads) keys_kernel(const float *__restrict__ xs, int64_t n, int d, int dp,
-                                                        const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
-                                                        int bits, int curve, uint64_t *__restrict__ keys,
-                                                        int32_t *__restrict__ idx) {
+// The two grids over the bounds: cells aligned with the bounds (curve 0), and shifted by 1.23 % of the extent in
+// every dimension (curve 1).
+struct Grids {
+    float scale, shift1;
+    uint32_t qmax;
+};
+__device__ __forceinline__ Grids grids_of(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi, int d, int bits) {
     float span = 0.f;
     for (int f = 0; f < d; ++f) {
         if (hi[f] >= lo[f]) span = fmaxf(span, from_ord(hi[f]) - from_ord(lo[f]));
     }
     const float cells = (float)(1u << bits);
-    const float scale = span > 0.f && isfinite(span) ? 0.97f * cells / span : 0.f;
-    const float shift = curve == 0 ? 0.f : 0.0123f * cells;
-    const uint32_t qmax = (1u << bits) - 1u;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        uint64_t key = 0;
-        for (int f = 0; f < d; ++f) {
-            const float base = hi[f] >= lo[f] ? from_ord(lo[f]) : 0.f;
-            const float t = (xs[i * dp + f] - base) * scale + shift;
-            const uint32_t q = t > 0.f ? (t < (float)qmax ? (uint32_t)t : qmax) : 0u;  // NaN -> 0
-            for (int b = 0; b < bits; ++b) key |= (uint64_t)((q >> b) & 1u) << (b * d + f);
-        }
-        keys[i] = key;
-        idx[i] = (int32_t)i;
+    return {span > 0.f && isfinite(span) ? 0.97f * cells / span : 0.f, 0.0123f * cells, (1u << bits) - 1u};
+}
+// A point's Morton key on grid `curve`, without its `drop` lowest bits.
+__device__ __forceinline__ uint64_t morton(const float *__restrict__ x, const Grids &g, const uint32_t *__restrict__ lo,
+                                           const uint32_t *__restrict__ hi, int d, int bits, int drop, int curve) {
+    uint64_t key = 0;
+    for (int f = 0; f < d; ++f) {
+        const float base = hi[f] >= lo[f] ? from_ord(lo[f]) : 0.f;
+        const float t = (x[f] - base) * g.scale + (curve == 0 ? 0.f : g.shift1);
+        const uint32_t q = t > 0.f ? (t < (float)g.qmax ? (uint32_t)t : g.qmax) : 0u;  // NaN -> 0
+        for (int b = 0; b < bits; ++b) key |= (uint64_t)((q >> b) & 1u) << (b * d + f);
+    }
+    return key >> drop;
+}
+
+// Sort entries of the points on both grids: keys[c n + i] = c above the key of point i on grid c, idx = i.
+__global__ void __launch_bounds__(kThreads) keys_kernel(const float *__restrict__ xs, int64_t n, int d, int dp,
+                                                        const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
+                                                        int bits, int drop, uint64_t *__restrict__ keys,
+                                                        int32_t *__restrict__ idx) {
+    const Grids g = grids_of(lo, hi, d, bits);
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 2 * n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int c = e >= n ? 1 : 0;
+        const int64_t i = e - c * n;
+        keys[e] = morton(xs + i * dp, g, lo, hi, d, bits, drop, c) | (uint64_t)c << (bits * d - drop);
+        idx[e] = (int32_t)i;
     }
 }
 
-__global__ void __launch_bounds__(kThreads) inverse_kernel(const int32_t *__restrict__ order, int64_t n,
-                                                           int32_t *__restrict__ pos) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-        pos[order[k]] = (int32_t)k;
+// The queries on the refs' grids (their bounds: queries outside them clamp to the edge): their keys as the refs'
+// entries have them, by query, and a sort entry each, 2 above the key on grid 0.
+__global__ void __launch_bounds__(kThreads) qkeys_kernel(const float *__restrict__ xq, int64_t nq, int d, int dp,
+                                                         const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
+                                                         int bits, int drop, uint64_t *__restrict__ k0,
+                                                         uint64_t *__restrict__ k1, uint64_t *__restrict__ keys,
+                                                         int32_t *__restrict__ idx) {
+    const Grids g = grids_of(lo, hi, d, bits);
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 2 * nq; e += (int64_t)gridDim.x * blockDim.x) {
+        const int c = e >= nq ? 1 : 0;
+        const int64_t q = e - c * nq;
+        const uint64_t key = morton(xq + q * dp, g, lo, hi, d, bits, drop, c);
+        if (c == 1) {
+            k1[q] = key | 1ull << (bits * d - drop);
+        } else {
+            k0[q] = key;
+            keys[q] = key | 2ull << (bits * d - drop);
+            idx[q] = (int32_t)q;
+        }
+    }
 }
 
-// Coordinates in a curve's order (row k = point order[k], dp floats) and, for curve 1, the
-// curve-0 position of each of its points: the seed kernel's window reads become contiguous.
-__global__ void __launch_bounds__(kThreads) gather_kernel(const float *__restrict__ xs, int64_t n, int dp,
-                                                          const int32_t *__restrict__ order, float *__restrict__ xs_c) {
-    const int64_t total = n * (dp / 4);
+// Of each curve (entries [0, n) and [n, 2n) of the sorted order): the points' positions, pos[c n + point], and
+// the coordinates in the curve's order (row k = the curve's k-th point, dp floats), so that the seed kernel's window
+// reads are contiguous.
+__global__ void __launch_bounds__(kThreads) place_kernel(const float *__restrict__ xs, int64_t n, int dp,
+                                                         const int32_t *__restrict__ order, int32_t *__restrict__ pos,
+                                                         float *__restrict__ xs_c) {
     const float4 *src = reinterpret_cast<const float4 *>(xs);
     float4 *dst = reinterpret_cast<float4 *>(xs_c);
     const int v4 = dp / 4;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t k = e / v4, v = e - k * v4;
-        dst[e] = src[(int64_t)order[k] * v4 + v];
+    const int64_t total = 2 * n * v4;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = t / v4, v = t - e * v4;
+        const int64_t i = order[e];
+        dst[t] = src[i * v4 + v];
+        if (v == 0) pos[(e >= n ? n : 0) + i] = (int32_t)(e >= n ? e - n : e);
     }
 }
 
@@ -293,11 +327,11 @@ __global__ void __launch_bounds__(kThreads) qseed_kernel(const float *__restrict
 }
 
 struct Layout {
-    size_t keys_a, keys_b, keys0, keys1, idx0_a, idx0_b, idx1_a, idx1_b, pos0, pos1, p0of1, xs0, xs1, bounds, cub,
-        cub_bytes, total;
+    size_t keys_a, keys_b, idx_a, idx_b, pos, p0of1, xs, bounds, cub, cub_bytes, total;
 };
 
-Layout layout(int64_t n, int dp) {
+// of n points on two curves, and nq queries sorted with them
+Layout layout(int64_t n, int dp, int64_t nq = 0) {
     Layout L{};
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -305,21 +339,16 @@ Layout layout(int64_t n, int dp) {
         off = align_up(off + bytes, 256);
         return o;
     };
-    L.keys_a = take((size_t)n * 8);
-    L.keys_b = take((size_t)n * 8);
-    L.keys0 = take((size_t)n * 8);
-    L.keys1 = take((size_t)n * 8);
-    L.idx0_a = take((size_t)n * 4);
-    L.idx0_b = take((size_t)n * 4);
-    L.idx1_a = take((size_t)n * 4);
-    L.idx1_b = take((size_t)n * 4);
-    L.pos0 = take((size_t)n * 4);
-    L.pos1 = take((size_t)n * 4);
+    const size_t entries = 2 * (size_t)n + (size_t)nq;
+    L.keys_a = take(entries * 8);
+    L.keys_b = take(entries * 8);
+    L.idx_a = take(entries * 4);
+    L.idx_b = take(entries * 4);
+    L.pos = take((size_t)n * 2 * 4);
     L.p0of1 = take((size_t)n * 4);
-    L.xs0 = take((size_t)n * dp * 4);
-    L.xs1 = take((size_t)n * dp * 4);
+    L.xs = take((size_t)n * 2 * dp * 4);
     L.bounds = take(2 * 256 * 4);
-    L.cub_bytes = align_up((size_t)(4u << 20) + (size_t)n / 2, 256);  // radix-sort scratch budget
+    L.cub_bytes = align_up((size_t)(4u << 20) + entries / 2, 256);  // radix-sort scratch budget
     L.cub = take(L.cub_bytes);
     L.total = off + 256;
     return L;
@@ -365,89 +394,79 @@ int grid_of(int64_t work) {
 }
 
 
-// One level: seeds of the points [0, n) from the windows of the curves of those points only
-// (combine: keep the smaller of the old and the new bound).
-// seeds == nullptr: only the curves (orders, inverse, sorted keys of both curves, coordinates in
-// curve order), for the query seeds.
-// Only the rows [row_lo, row_hi) get seeds (the others are left as they were).
-nngp_status run_level(const float *xs, int64_t n, int d, int D, int dp, int m, int W, char *base, const Layout &L,
-                      int combine, float *seeds, cudaStream_t stream, const int32_t **order0_out,
-                      const int32_t **pos0_out, const uint64_t **keys0_out, int64_t row_lo = 0,
-                      int64_t row_hi = INT64_MAX) {
+// The curves of n points (left in a workspace region).
+struct Curves {
+    const uint64_t *keys0, *keys1;   // sorted keys (curve 1's with a 1 above them)
+    const int32_t *order0, *order1;  // the points in each curve's order
+    const int32_t *pos0, *pos1;      // and their places in it
+    const int32_t *p0of1;            // curve-0 place of curve 1's k-th point
+    const float *xs0, *xs1;          // coordinates in each curve's order
+    const int32_t *qorder;           // the queries in curve-0 order
+};
+// Both curves, and the queries' order (xq; their keys go to qk0, qk1), come from one radix sort, told apart by the
+// bits above the keys.  A pass over 16,000 to 900,000 entries is bound by latency (8 to 14 us), so sorts of their own
+// took almost as many times as long: the passes for 16,384 queries in 16,599 refs, d = 18, 161 -> 58 us (the
+// whole predict 1.03 -> 0.83 ms), a prefix search of n = 434,874, d = 3 with its n / 8 level 4.97 -> 4.81 ms in all.
+nngp_status make_curves(const float *xs, int64_t n, int d, int dp, char *base, const Layout &L, const float *xq, int64_t nq,
+                        uint64_t *qk0, uint64_t *qk1, Curves &out, cudaStream_t stream) {
     auto at = [&](size_t off) { return reinterpret_cast<void *>(base + off); };
-    uint64_t *keys_a = static_cast<uint64_t *>(at(L.keys_a)), *keys_b = static_cast<uint64_t *>(at(L.keys_b));
-    int32_t *idx[2][2] = {{static_cast<int32_t *>(at(L.idx0_a)), static_cast<int32_t *>(at(L.idx0_b))},
-                          {static_cast<int32_t *>(at(L.idx1_a)), static_cast<int32_t *>(at(L.idx1_b))}};
-    int32_t *pos[2] = {static_cast<int32_t *>(at(L.pos0)), static_cast<int32_t *>(at(L.pos1))};
+    uint64_t *keys = static_cast<uint64_t *>(at(L.keys_a));
+    int32_t *idx = static_cast<int32_t *>(at(L.idx_a)), *pos = static_cast<int32_t *>(at(L.pos));
     uint32_t *lo = static_cast<uint32_t *>(at(L.bounds)), *hi = lo + 256;
-    const int bits = seed::bits(d);
+    const int bits = seed::bits(d), drop = seed::key_drop(d);
+    const int64_t entries = 2 * n + nq;
 
     NNGP_CUDA_TRY(cudaMemsetAsync(lo, 0xFF, 256 * 4, stream));
     NNGP_CUDA_TRY(cudaMemsetAsync(hi, 0x00, 256 * 4, stream));
     bounds_kernel<<<grid_of(n), kThreads, 0, stream>>>(xs, n, d, dp, lo, hi);
     NNGP_CUDA_TRY(cudaGetLastError());
-    const int32_t *order[2] = {nullptr, nullptr};
-    for (int c = 0; c < 2; ++c) {
-        keys_kernel<<<grid_of(n), kThreads, 0, stream>>>(xs, n, d, dp, lo, hi, bits, c, keys_a, idx[c][0]);
-        NNGP_CUDA_TRY(cudaGetLastError());
-        cub::DoubleBuffer<uint64_t> dk(keys_a, keys_b);
-        cub::DoubleBuffer<int32_t> dv(idx[c][0], idx[c][1]);
-        size_t need = 0;
-        NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, dk, dv, (int)n, 0, bits * d, stream));
-        if (need > L.cub_bytes)
-            return fail(NNGP_ERR_WORKSPACE, "knn seeds: radix-sort scratch " + std::to_string(need) +
-                                                " bytes exceeds the budget");
-        size_t have = L.cub_bytes;
-        NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(at(L.cub), have, dk, dv, (int)n, 0, bits * d, stream));
-        order[c] = dv.Current();
-        if ((c == 0 && keys0_out) || !seeds) {  // sorted keys, for cells along the curve or query positions
-            NNGP_CUDA_TRY(cudaMemcpyAsync(at(c ? L.keys1 : L.keys0), dk.Current(), (size_t)n * 8,
-                                          cudaMemcpyDeviceToDevice, stream));
-        }
-        inverse_kernel<<<grid_of(n), kThreads, 0, stream>>>(order[c], n, pos[c]);
-        NNGP_CUDA_TRY(cudaGetLastError());
-        gather_kernel<<<grid_of(n * (dp / 4)), kThreads, 0, stream>>>(xs, n, dp, order[c],
-                                                                      static_cast<float *>(at(c ? L.xs1 : L.xs0)));
+    keys_kernel<<<grid_of(2 * n), kThreads, 0, stream>>>(xs, n, d, dp, lo, hi, bits, drop, keys, idx);
+    NNGP_CUDA_TRY(cudaGetLastError());
+    if (nq > 0) {
+        qkeys_kernel<<<grid_of(2 * nq), kThreads, 0, stream>>>(xq, nq, d, dp, lo, hi, bits, drop, qk0, qk1, keys + 2 * n,
+                                                               idx + 2 * n);
         NNGP_CUDA_TRY(cudaGetLastError());
     }
+    cub::DoubleBuffer<uint64_t> dk(keys, static_cast<uint64_t *>(at(L.keys_b)));
+    cub::DoubleBuffer<int32_t> dv(idx, static_cast<int32_t *>(at(L.idx_b)));
+    const int end_bit = bits * d - drop + (nq > 0 ? 2 : 1);
+    // (a 64-bit count only where 32 bits do not hold it)
+    auto sort = [&](void *scratch, size_t &bytes) {
+        return entries <= INT_MAX
+                   ? cub::DeviceRadixSort::SortPairs(scratch, bytes, dk, dv, (int)entries, 0, end_bit, stream)
+                   : cub::DeviceRadixSort::SortPairs(scratch, bytes, dk, dv, entries, 0, end_bit, stream);
+    };
+    size_t need = 0;
+    NNGP_CUDA_TRY(sort(nullptr, need));
+    if (need > L.cub_bytes)
+        return fail(NNGP_ERR_WORKSPACE,
+                    "knn seeds: radix-sort scratch " + std::to_string(need) + " bytes exceeds the budget");
+    size_t have = L.cub_bytes;
+    NNGP_CUDA_TRY(sort(at(L.cub), have));
+    const int32_t *order = dv.Current();
+    float *xc = static_cast<float *>(at(L.xs));
     int32_t *p0of1 = static_cast<int32_t *>(at(L.p0of1));
-    cross_pos_kernel<<<grid_of(n), kThreads, 0, stream>>>(order[1], pos[0], n, p0of1);
+    place_kernel<<<grid_of(2 * n * (dp / 4)), kThreads, 0, stream>>>(xs, n, dp, order, pos, xc);
     NNGP_CUDA_TRY(cudaGetLastError());
-    if (order0_out) *order0_out = order[0];
-    if (pos0_out) *pos0_out = pos[0];
-    if (keys0_out) *keys0_out = static_cast<const uint64_t *>(at(L.keys0));
-    if (!seeds) return NNGP_OK;
+    cross_pos_kernel<<<grid_of(n), kThreads, 0, stream>>>(order + n, pos, n, p0of1);
+    NNGP_CUDA_TRY(cudaGetLastError());
+    out = Curves{dk.Current(), dk.Current() + n, order, order + n, pos, pos + n, p0of1, xc, xc + n * dp, order + 2 * n};
+    return NNGP_OK;
+}
+
+// One level: seeds of the points [0, n) from the windows of the curves of those points only
+// (combine: keep the smaller of the old and the new bound).
+// Only the rows [row_lo, row_hi) get seeds (the others are left as they were).
+nngp_status run_level(const float *xs, int64_t n, int d, int D, int dp, int m, int W, char *base, const Layout &L,
+                      int combine, float *seeds, cudaStream_t stream, Curves &cv, int64_t row_lo, int64_t row_hi) {
+    nngp_status st = make_curves(xs, n, d, dp, base, L, nullptr, 0, nullptr, nullptr, cv, stream);
+    if (st != NNGP_OK) return st;
     const int grid = (int)std::min<int64_t>((n + kThreads / 32 - 1) / (kThreads / 32), (int64_t)kNumSMsB200 * 16);
-    const SeedArgs sa{static_cast<const float *>(at(L.xs0)), static_cast<const float *>(at(L.xs1)), n, dp, m,
-                      order[0], order[1], p0of1, pos[1], combine, row_lo, row_hi, seeds};
+    const SeedArgs sa{cv.xs0, cv.xs1, n, dp, m, cv.order0, cv.order1, cv.p0of1, cv.pos1, combine, row_lo, row_hi, seeds};
     const bool ok = W == 128 ? dispatch_seed<8>(D, grid, sa, stream) : dispatch_seed<16>(D, grid, sa, stream);
     if (!ok) return fail(NNGP_ERR_UNSUPPORTED, "knn seeds: no kernel for D = " + std::to_string(D));
     NNGP_CUDA_TRY(cudaGetLastError());
     return NNGP_OK;
-}
-
-// Query region of the query-seed workspace.
-struct QLayout {
-    size_t k0, k1, kb, kb2, ia, ib, cub, cub_bytes, total;
-};
-QLayout qlayout(int64_t nq) {
-    QLayout Q{};
-    size_t off = 0;
-    auto take = [&](size_t bytes) {
-        const size_t o = off;
-        off = align_up(off + bytes, 256);
-        return o;
-    };
-    Q.k0 = take((size_t)nq * 8);
-    Q.k1 = take((size_t)nq * 8);
-    Q.kb = take((size_t)nq * 8);
-    Q.kb2 = take((size_t)nq * 8);
-    Q.ia = take((size_t)nq * 4);
-    Q.ib = take((size_t)nq * 4);
-    Q.cub_bytes = align_up((size_t)(4u << 20) + (size_t)nq / 2, 256);
-    Q.cub = take(Q.cub_bytes);
-    Q.total = off + 256;
-    return Q;
 }
 
 template <int D>
@@ -466,7 +485,7 @@ size_t sub_bytes(int64_t n, int dp) { return n / 8 >= kMinPoints ? layout(n / 8,
 
 size_t workspace_query(int64_t n_ref, int64_t n_query, int dp) {
     if (n_ref < kMinPoints || n_query < 1) return 0;
-    return align_up(layout(n_ref, dp).total, 256) + qlayout(n_query).total;
+    return align_up(layout(n_ref, dp, n_query).total, 256) + (size_t)n_query * 16;  // and the queries' keys
 }
 
 nngp_status query_seeds(const float *xs_ref, int64_t n_ref, const float *xq, int64_t n_query, int d, int D, int dp,
@@ -474,51 +493,29 @@ nngp_status query_seeds(const float *xs_ref, int64_t n_ref, const float *xq, int
                         const int32_t **qorder_out) {
     if (n_ref < kMinPoints || n_query < 1 || m < 1 || d < 1 || d > 24 || D < d || dp % 4 != 0 || dp < D)
         return fail(NNGP_ERR_UNSUPPORTED, "knn query seeds: shape outside the seeded search");
-    const Layout L = layout(n_ref, dp);
+    const Layout L = layout(n_ref, dp, n_query);
     if (!ws || ws_bytes < workspace_query(n_ref, n_query, dp))
         return fail(NNGP_ERR_WORKSPACE, "knn query seeds: workspace too small");
     char *base = reinterpret_cast<char *>(align_up(reinterpret_cast<uintptr_t>(ws), 256));
-    const int32_t *order0 = nullptr;
-    nngp_status st = run_level(xs_ref, n_ref, d, D, dp, m, 128, base, L, 0, nullptr, stream, &order0, nullptr, nullptr);
+    uint64_t *qk0 = reinterpret_cast<uint64_t *>(base + align_up(L.total, 256) - 256), *qk1 = qk0 + n_query;
+    Curves cv{};
+    nngp_status st = make_curves(xs_ref, n_ref, d, dp, base, L, xq, n_query, qk0, qk1, cv, stream);
     if (st != NNGP_OK) return st;
-    char *qb = base + align_up(L.total, 256);
-    const QLayout Q = qlayout(n_query);
-    auto qat = [&](size_t off) { return reinterpret_cast<void *>(qb + off); };
-    auto at = [&](size_t off) { return reinterpret_cast<void *>(base + off); };
-    const uint32_t *lo = static_cast<const uint32_t *>(at(L.bounds)), *hi = lo + 256;
-    const int bits = seed::bits(d);
-    uint64_t *qk0 = static_cast<uint64_t *>(qat(Q.k0)), *qk1 = static_cast<uint64_t *>(qat(Q.k1));
-    int32_t *ia = static_cast<int32_t *>(qat(Q.ia));
-    // the queries' keys on the refs' grids (their bounds: queries outside them clamp to the edge)
-    keys_kernel<<<grid_of(n_query), kThreads, 0, stream>>>(xq, n_query, d, dp, lo, hi, bits, 1, qk1, ia);
-    NNGP_CUDA_TRY(cudaGetLastError());
-    keys_kernel<<<grid_of(n_query), kThreads, 0, stream>>>(xq, n_query, d, dp, lo, hi, bits, 0, qk0, ia);
-    NNGP_CUDA_TRY(cudaGetLastError());
-    // query order along curve 0 (sorts a copy of the keys; qk0 stays indexed by query)
-    NNGP_CUDA_TRY(cudaMemcpyAsync(qat(Q.kb), qk0, (size_t)n_query * 8, cudaMemcpyDeviceToDevice, stream));
-    cub::DoubleBuffer<uint64_t> dk(static_cast<uint64_t *>(qat(Q.kb)), static_cast<uint64_t *>(qat(Q.kb2)));
-    cub::DoubleBuffer<int32_t> dv(ia, static_cast<int32_t *>(qat(Q.ib)));
-    size_t need = 0;
-    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, dk, dv, (int)n_query, 0, bits * d, stream));
-    if (need > Q.cub_bytes) return fail(NNGP_ERR_WORKSPACE, "knn query seeds: sort scratch exceeds the budget");
-    size_t have = Q.cub_bytes;
-    NNGP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(qat(Q.cub), have, dk, dv, (int)n_query, 0, bits * d, stream));
-    const int32_t *qorder = dv.Current();
     const int grid = (int)std::min<int64_t>((n_query + kThreads / 32 - 1) / (kThreads / 32), (int64_t)kNumSMsB200 * 16);
-    const float *xs0 = static_cast<const float *>(at(L.xs0)), *xs1 = static_cast<const float *>(at(L.xs1));
-    const uint64_t *k0s = static_cast<const uint64_t *>(at(L.keys0)), *k1s = static_cast<const uint64_t *>(at(L.keys1));
-    const int32_t *p0of1 = static_cast<const int32_t *>(at(L.p0of1));
     switch (D) {
 #define NNGP_QS(DD) \
-    case DD: launch_qseed<DD>(grid, xs0, xs1, k0s, k1s, n_ref, p0of1, xq, n_query, qk0, qk1, qorder, dp, m, seeds, stream); break;
+    case DD:                                                                                                        \
+        launch_qseed<DD>(grid, cv.xs0, cv.xs1, cv.keys0, cv.keys1, n_ref, cv.p0of1, xq, n_query, qk0, qk1, cv.qorder, dp, m, \
+                         seeds, stream);                                                                          \
+        break;
         NNGP_QS(1) NNGP_QS(2) NNGP_QS(3) NNGP_QS(4) NNGP_QS(5) NNGP_QS(6) NNGP_QS(7) NNGP_QS(8) NNGP_QS(12) NNGP_QS(16)
         NNGP_QS(20) NNGP_QS(24)
 #undef NNGP_QS
         default: return fail(NNGP_ERR_UNSUPPORTED, "knn query seeds: no kernel for D = " + std::to_string(D));
     }
     NNGP_CUDA_TRY(cudaGetLastError());
-    if (order0_out) *order0_out = order0;
-    if (qorder_out) *qorder_out = qorder;
+    if (order0_out) *order0_out = cv.order0;
+    if (qorder_out) *qorder_out = cv.qorder;
     return NNGP_OK;
 }
 
@@ -543,15 +540,17 @@ nngp_status prefix_seeds(const float *xs, int64_t n, int d, int D, int dp, int m
     const Layout L = layout(n, dp);
     if (!ws || ws_bytes < workspace(n, dp)) return fail(NNGP_ERR_WORKSPACE, "knn seeds: workspace too small");
     char *base = reinterpret_cast<char *>(align_up(reinterpret_cast<uintptr_t>(ws), 256));
-    nngp_status st = run_level(xs, n, d, D, dp, m, W, base, L, 0, seeds, stream, order0_out, pos0_out, keys0_out,
-                               row_lo, row_hi);
+    Curves cv{};
+    nngp_status st = run_level(xs, n, d, D, dp, m, W, base, L, 0, seeds, stream, cv, row_lo, row_hi);
     if (st != NNGP_OK) return st;
+    if (order0_out) *order0_out = cv.order0;
+    if (pos0_out) *pos0_out = cv.pos0;
+    if (keys0_out) *keys0_out = cv.keys0;
     // rows i < n / 8 see few earlier points in the full windows: bound them again from the
     // curves of the prefix alone (any m earlier points bound a row; the smaller bound is kept)
     char *sub = base + align_up(L.total, 256);
     for (int64_t p = n / 8; p >= kMinPoints && p > row_lo; p /= 8) {
-        st = run_level(xs, p, d, D, dp, m, W, sub, layout(p, dp), 1, seeds, stream, nullptr, nullptr, nullptr, row_lo,
-                       row_hi);
+        st = run_level(xs, p, d, D, dp, m, W, sub, layout(p, dp), 1, seeds, stream, cv, row_lo, row_hi);
         if (st != NNGP_OK) return st;
     }
     return NNGP_OK;

@@ -25,7 +25,7 @@ int window();
 // dimension the search kernel loops over.  Runs on `stream`; ws of workspace(n) bytes.
 // order0 / pos0 / keys0 (optional): the curve-0 order of the points (a permutation of 0..n-1),
 // its inverse and the curve-0 Morton keys in that order (key of point i = keys0[pos0[i]];
-// bits() bits per dimension, interleaved), left in ws for the caller.
+// bits() bits per dimension, interleaved, without the key_drop() lowest), left in ws for the caller.
 // row_lo / row_hi: only the rows [row_lo, row_hi) get seeds (a row shard; -1: up to n).
 nngp_status prefix_seeds(const float *xs, int64_t n, int d, int D, int dp, int m, void *ws, size_t ws_bytes,
                          float *seeds, cudaStream_t stream, const int32_t **order0 = nullptr,
@@ -50,6 +50,8 @@ nngp_status query_seeds(const float *xs_ref, int64_t n_ref, const float *xq, int
 
 // Bits per dimension of the Morton keys for d features.
 inline int bits(int d) { return d < 7 ? 10 : 64 / d; }
+// Lowest bits left off the keys, so that two bits that tell curves and queries apart fit above them.
+inline int key_drop(int d) { return bits(d) * d > 62 ? bits(d) * d - 62 : 0; }
 
 }  // namespace seed
 }  // namespace nngp

@@ -35,3 +35,22 @@ def test_rescoring_matches_oracle(monkeypatch, d, m):
     x = rng.integers(0, 2, (1500, d)).astype(np.float64)
     for pts in (x, x[::-1].copy(), np.ones((700, d))):
         assert np.array_equal(run(monkeypatch, pts, pts, m, 0), O.knn(pts, pts, m, 0, None, np.float32))
+
+
+@pytest.mark.parametrize('d', [2, 6, 7, 8, 9, 16, 21, 24])
+def test_curves_of_one_sort_match_the_direct_search(monkeypatch, d):
+    """Seeds of a prefix search and of queries (both curves and the queries in one sort; from d = 7 on some shapes
+    drop a key's lowest bits for the two that tell them apart), with points on one spot and a far outlier."""
+    rng = np.random.default_rng(d)
+    r = rng.normal(size=(9001, d)).astype(np.float32)
+    r[100:400] = r[100]
+    r[8200] = 1e6
+    q = rng.normal(size=(16385, d)).astype(np.float32)
+    q[5] = r[100]
+    rt, qt = torch.from_numpy(r).cuda(), torch.from_numpy(q).cuda()
+    for a, cut in ((rt, 0), (qt, None)):
+        lists = []
+        for kernel in ('tc', 'direct'):
+            monkeypatch.setenv('NNGP_KNN_KERNEL', kernel)
+            lists.append(ops.knn(rt, a, 32, cut, None))
+        assert torch.equal(lists[0], lists[1])
