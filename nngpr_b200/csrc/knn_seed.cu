@@ -47,26 +47,49 @@ __device__ __forceinline__ float from_ord(uint32_t o) {
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
 }
 
+// Bounds of the finite coordinates of every feature, as ord_of images.  A thread keeps to one 4-feature column of the
+// rows, so that a warp reads whole sectors (a thread per row, feature after feature, took 20.5 against
+// 9.4 us at n = 434,874, d = 3, 8.5 against 3.3 at n = 16,599, d = 18).
 __global__ void __launch_bounds__(kThreads) bounds_kernel(const float *__restrict__ xs, int64_t n, int d, int dp,
                                                           uint32_t *__restrict__ lo, uint32_t *__restrict__ hi) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    for (int f = 0; f < d; ++f) {
-        uint32_t mn = 0xFFFFFFFFu, mx = 0u;
-        for (int64_t i = i0; i < n; i += stride) {
-            const float v = xs[i * dp + f];
+    __shared__ uint32_t slo[256], shi[256];
+    slo[threadIdx.x] = 0xFFFFFFFFu;
+    shi[threadIdx.x] = 0u;
+    __syncthreads();
+    const int v4 = dp / 4;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x / v4 * v4;
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const float4 *src = reinterpret_cast<const float4 *>(xs);
+    if (t0 < stride && t0 < n * v4) {
+        uint32_t mn[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[4] = {0u, 0u, 0u, 0u};
+        auto take = [&](int c, float v) {
             if (isfinite(v)) {
                 const uint32_t o = ord_of(v);
-                mn = min(mn, o);
-                mx = max(mx, o);
+                mn[c] = min(mn[c], o);
+                mx[c] = max(mx[c], o);
+            }
+        };
+#pragma unroll 4
+        for (int64_t t = t0; t < n * v4; t += stride) {
+            const float4 r = __ldg(src + t);
+            take(0, r.x);
+            take(1, r.y);
+            take(2, r.z);
+            take(3, r.w);
+        }
+        const int f0 = 4 * (int)(t0 % v4);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (f0 + c < d && mn[c] <= mx[c]) {
+                atomicMin(slo + f0 + c, mn[c]);
+                atomicMax(shi + f0 + c, mx[c]);
             }
         }
-        mn = __reduce_min_sync(0xFFFFFFFFu, mn);
-        mx = __reduce_max_sync(0xFFFFFFFFu, mx);
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(lo + f, mn);
-            atomicMax(hi + f, mx);
-        }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < d && slo[threadIdx.x] <= shi[threadIdx.x]) {
+        atomicMin(lo + threadIdx.x, slo[threadIdx.x]);
+        atomicMax(hi + threadIdx.x, shi[threadIdx.x]);
     }
 }
 
@@ -133,21 +156,29 @@ __global__ void __launch_bounds__(kThreads) qkeys_kernel(const float *__restrict
     }
 }
 
+// float4 index of the v-th 4 features of place k in a curve's coordinates
+__host__ __device__ __forceinline__ int64_t coords_at(int64_t k, int v, int v4) {
+    return ((k >> 5) * v4 + v) * 32 + (k & 31);
+}
+__host__ __device__ __forceinline__ int64_t blocks_of(int64_t n) { return (n + 31) / 32; }
+
 // Of each curve (entries [0, n) and [n, 2n) of the sorted order): the points' positions, pos[c n + point], and
-// the coordinates in the curve's order (row k = the curve's k-th point, dp floats), so that the seed kernel's window
-// reads are contiguous.
+// the coordinates in the curve's order, so that the seed kernels' window reads are contiguous: blocks of 32 places,
+// in each block 4 features of all 32 after one another (coords_at), 512 bytes for a warp's load of them (by rows of
+// dp floats a load touched 4 times as many lines at d = 16).
 __global__ void __launch_bounds__(kThreads) place_kernel(const float *__restrict__ xs, int64_t n, int dp,
                                                          const int32_t *__restrict__ order, int32_t *__restrict__ pos,
                                                          float *__restrict__ xs_c) {
     const float4 *src = reinterpret_cast<const float4 *>(xs);
     float4 *dst = reinterpret_cast<float4 *>(xs_c);
     const int v4 = dp / 4;
-    const int64_t total = 2 * n * v4;
+    const int64_t total = 2 * n * v4, curve = blocks_of(n) * 32 * v4;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t e = t / v4, v = t - e * v4;
         const int64_t i = order[e];
-        dst[t] = src[i * v4 + v];
-        if (v == 0) pos[(e >= n ? n : 0) + i] = (int32_t)(e >= n ? e - n : e);
+        const int64_t k = e >= n ? e - n : e;
+        dst[(e >= n ? curve : 0) + coords_at(k, (int)v, v4)] = src[i * v4 + v];
+        if (v == 0) pos[(e >= n ? n : 0) + i] = (int32_t)k;
     }
 }
 
@@ -158,21 +189,26 @@ __global__ void __launch_bounds__(kThreads) cross_pos_kernel(const int32_t *__re
         p0_of1[k] = pos0[order1[k]];
 }
 
-// Squared distance bits of the ref row r and the query coordinates qv in the search's exact
-// arithmetic: ((r0 - q0)^2 + (r1 - q1)^2) + ..., every step rounded, over the D padded features.
+// Coordinates of place k of a curve.
 template <int D>
-__device__ __forceinline__ uint32_t dist_bits(const float *__restrict__ row, const float (&qv)[D]) {
-    constexpr int V = (D + 3) / 4;
-    const float4 *r4 = reinterpret_cast<const float4 *>(row);
-    float r[4 * V];
+__device__ __forceinline__ void load_coords(const float4 *__restrict__ xs_c, int64_t k, int v4, float (&r)[(D + 3) / 4 * 4]) {
+    const float4 *p = xs_c + coords_at(k, 0, v4);
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-        const float4 t = __ldg(r4 + v);
+    for (int v = 0; v < (D + 3) / 4; ++v) {
+        const float4 t = __ldg(p + 32 * v);
         r[4 * v] = t.x;
         r[4 * v + 1] = t.y;
         r[4 * v + 2] = t.z;
         r[4 * v + 3] = t.w;
     }
+}
+
+// Squared distance bits of the ref at place k and the query coordinates qv in the search's exact
+// arithmetic: ((r0 - q0)^2 + (r1 - q1)^2) + ..., every step rounded, over the D padded features.
+template <int D>
+__device__ __forceinline__ uint32_t dist_bits(const float4 *__restrict__ xs_c, int64_t k, int v4, const float (&qv)[D]) {
+    float r[(D + 3) / 4 * 4];
+    load_coords<D>(xs_c, k, v4, r);
     const float t0 = sub_rn(r[0], qv[0]);
     float d2 = mul_rn(t0, t0);
 #pragma unroll
@@ -183,9 +219,10 @@ __device__ __forceinline__ uint32_t dist_bits(const float *__restrict__ row, con
     return __float_as_uint(d2);  // NaN bits lie above kInfBits and are never counted
 }
 
-// The m-th smallest of the warp's values (each lane holds N; 0xFFFFFFFF = none, NaN bits above
-// kInfBits never count): bisection on the bit patterns, stopped within kTolBits above it, so
-// at least m values are <= the result; kInfBits when fewer than m values are finite.
+// The m-th smallest of the warp's values (each lane holds N; 0xFFFFFFFF = none, NaN bits above kInfBits never
+// count), or within kTolBits above it: bisection on the bit patterns until a bound has exactly m values at or
+// below it, whose largest is the answer, or the bounds meet; kInfBits when fewer than m values are finite.  Where every
+// lane has a value and m <= 32 the largest of the lanes' smallest bounds it from the start.
 template <int N>
 __device__ __forceinline__ uint32_t mth_smallest_bits(const uint32_t (&v)[N], int m) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -195,22 +232,28 @@ __device__ __forceinline__ uint32_t mth_smallest_bits(const uint32_t (&v)[N], in
         for (int e = 0; e < N; ++e) c += v[e] <= bound ? 1 : 0;
         return (int)__reduce_add_sync(FULL, (unsigned)c);
     };
-    if (count_le(kInfBits) < m) return kInfBits;
-    uint32_t mn = 0xFFFFFFFFu, mx = 0u;
+    uint32_t mn = 0xFFFFFFFFu;
 #pragma unroll
-    for (int e = 0; e < N; ++e) {
-        if (v[e] <= kInfBits) {
-            mn = min(mn, v[e]);
-            mx = max(mx, v[e]);
-        }
+    for (int e = 0; e < N; ++e) mn = min(mn, v[e]);
+    uint32_t lo = __reduce_min_sync(FULL, mn), hi = __reduce_max_sync(FULL, mn);
+    if (m > 32 || hi > kInfBits) {
+        if (count_le(kInfBits) < m) return kInfBits;
+        hi = kInfBits;
     }
-    uint32_t lo = __reduce_min_sync(FULL, mn), hi = __reduce_max_sync(FULL, mx);  // count_le(hi) >= m
     while (hi - lo > kTolBits) {  // invariant: count_le(hi) >= m; warp-uniform
         const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (count_le(mid) >= m) hi = mid;
-        else lo = mid + 1;
+        const int c = count_le(mid);
+        if (c >= m) {
+            hi = mid;
+            if (c == m) break;
+        } else {
+            lo = mid + 1;
+        }
     }
-    return hi;
+    uint32_t mx = 0u;  // the largest value at or below hi
+#pragma unroll
+    for (int e = 0; e < N; ++e) mx = max(mx, v[e] <= hi ? v[e] : 0u);
+    return __reduce_max_sync(FULL, mx);
 }
 
 // One warp per point (taken in curve-0 order).  Lane values: squared-distance bits of the refs
@@ -218,15 +261,17 @@ __device__ __forceinline__ uint32_t mth_smallest_bits(const uint32_t (&v)[N], in
 // so every ref counts once); 0xFFFFFFFF for the other slots.  The row's seed is the m-th
 // smallest value (bisection on the bit patterns, stopped within kTolBits above it), or +inf.
 // xs0 / xs1: the coordinates in curve order; p0_of1[k] = curve-0 position of order1[k].
+// Bound by the window reads (half of each window is j >= i) and the bisection's counts.  Coordinates by rows -> in blocks
+// of 32 places, and a bisection that ends when its count is m, from the lanes' smallest values: 930 -> 807 us (n =
+// 434,874, d = 3, two levels), 1,243 -> 989 us (d = 8), 3,734 -> 3,451 us (n = 1M, d = 16, three levels).
 template <int D, int VPL>
-__global__ void __launch_bounds__(kThreads) seed_kernel(const float *__restrict__ xs0, const float *__restrict__ xs1,
-                                                        int64_t n, int dp, int m, const int32_t *__restrict__ order0,
+__global__ void __launch_bounds__(kThreads) seed_kernel(const float4 *__restrict__ xs0,
+                                                        const float4 *__restrict__ xs1, int64_t n, int v4, int m, const int32_t *__restrict__ order0,
                                                         const int32_t *__restrict__ order1,
                                                         const int32_t *__restrict__ p0_of1,
                                                         const int32_t *__restrict__ pos1, int combine,
                                                         int64_t row_lo, int64_t row_hi, float *__restrict__ seeds) {
     constexpr int W = VPL * 16;
-    constexpr unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < n; k += nwarps) {
@@ -236,9 +281,10 @@ __global__ void __launch_bounds__(kThreads) seed_kernel(const float *__restrict_
             if (lane == 0 && !combine) seeds[i] = __uint_as_float(kInfBits);
             continue;
         }
-        float qv[D];
+        float row[(D + 3) / 4 * 4], qv[D];
+        load_coords<D>(xs0, k, v4, row);
 #pragma unroll
-        for (int f = 0; f < D; ++f) qv[f] = xs0[k * dp + f];
+        for (int f = 0; f < D; ++f) qv[f] = row[f];
         uint32_t v[2 * VPL];
 #pragma unroll
         for (int t = 0; t < VPL; ++t) {
@@ -246,7 +292,7 @@ __global__ void __launch_bounds__(kThreads) seed_kernel(const float *__restrict_
             uint32_t val = 0xFFFFFFFFu;
             if (pk >= 0 && pk < n) {
                 const int64_t j = order0[pk];
-                if (j < i) val = dist_bits<D>(xs0 + pk * dp, qv);
+                if (j < i) val = dist_bits<D>(xs0, pk, v4, qv);
             }
             v[t] = val;
         }
@@ -259,7 +305,7 @@ __global__ void __launch_bounds__(kThreads) seed_kernel(const float *__restrict_
                 const int64_t j = order1[pk];
                 if (j < i) {
                     const int64_t pj = p0_of1[pk];
-                    if (pj < k - W || pj >= k + W) val = dist_bits<D>(xs1 + pk * dp, qv);
+                    if (pj < k - W || pj >= k + W) val = dist_bits<D>(xs1, pk, v4, qv);
                 }
             }
             v[VPL + t] = val;
@@ -286,7 +332,8 @@ __device__ __forceinline__ int64_t lower_bound_u64(const uint64_t *__restrict__ 
 // within W positions on either side (curve 1 skips refs inside curve 0's window), the m-th
 // smallest squared distance in the search's exact arithmetic.
 template <int D>
-__global__ void __launch_bounds__(kThreads) qseed_kernel(const float *__restrict__ xs0, const float *__restrict__ xs1,
+__global__ void __launch_bounds__(kThreads) qseed_kernel(const float4 *__restrict__ xs0,
+                                                         const float4 *__restrict__ xs1,
                                                          const uint64_t *__restrict__ keys0s,
                                                          const uint64_t *__restrict__ keys1s, int64_t n_ref,
                                                          const int32_t *__restrict__ p0_of1,
@@ -296,7 +343,7 @@ __global__ void __launch_bounds__(kThreads) qseed_kernel(const float *__restrict
                                                          const int32_t *__restrict__ qorder, int dp, int m,
                                                          float *__restrict__ seeds) {
     constexpr int VPL = 8, W = VPL * 16;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, v4 = dp / 4;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < n_query; k += nwarps) {
         const int64_t q = qorder[k];
@@ -309,7 +356,7 @@ __global__ void __launch_bounds__(kThreads) qseed_kernel(const float *__restrict
 #pragma unroll
         for (int t = 0; t < VPL; ++t) {
             const int64_t pk = c0 - W + lane + 32 * t;
-            v[t] = (pk >= 0 && pk < n_ref) ? dist_bits<D>(xs0 + pk * dp, qv) : 0xFFFFFFFFu;
+            v[t] = (pk >= 0 && pk < n_ref) ? dist_bits<D>(xs0, pk, v4, qv) : 0xFFFFFFFFu;
         }
 #pragma unroll
         for (int t = 0; t < VPL; ++t) {
@@ -317,7 +364,7 @@ __global__ void __launch_bounds__(kThreads) qseed_kernel(const float *__restrict
             uint32_t val = 0xFFFFFFFFu;
             if (pk >= 0 && pk < n_ref) {
                 const int64_t pj = p0_of1[pk];
-                if (pj < c0 - W || pj >= c0 + W) val = dist_bits<D>(xs1 + pk * dp, qv);
+                if (pj < c0 - W || pj >= c0 + W) val = dist_bits<D>(xs1, pk, v4, qv);
             }
             v[VPL + t] = val;
         }
@@ -346,7 +393,7 @@ Layout layout(int64_t n, int dp, int64_t nq = 0) {
     L.idx_b = take(entries * 4);
     L.pos = take((size_t)n * 2 * 4);
     L.p0of1 = take((size_t)n * 4);
-    L.xs = take((size_t)n * 2 * dp * 4);
+    L.xs = take((size_t)blocks_of(n) * 32 * 2 * dp * 4);
     L.bounds = take(2 * 256 * 4);
     L.cub_bytes = align_up((size_t)(4u << 20) + entries / 2, 256);  // radix-sort scratch budget
     L.cub = take(L.cub_bytes);
@@ -355,7 +402,7 @@ Layout layout(int64_t n, int dp, int64_t nq = 0) {
 }
 
 struct SeedArgs {
-    const float *xs0, *xs1;
+    const float4 *xs0, *xs1;
     int64_t n;
     int dp, m;
     const int32_t *o0, *o1, *p0of1, *p1;
@@ -366,7 +413,7 @@ struct SeedArgs {
 
 template <int D, int VPL>
 void launch_seed(int grid, const SeedArgs &a, cudaStream_t stream) {
-    seed_kernel<D, VPL><<<grid, kThreads, 0, stream>>>(a.xs0, a.xs1, a.n, a.dp, a.m, a.o0, a.o1, a.p0of1, a.p1,
+    seed_kernel<D, VPL><<<grid, kThreads, 0, stream>>>(a.xs0, a.xs1, a.n, a.dp / 4, a.m, a.o0, a.o1, a.p0of1, a.p1,
                                                        a.combine, a.row_lo, a.row_hi, a.seeds);
 }
 
@@ -400,7 +447,7 @@ struct Curves {
     const int32_t *order0, *order1;  // the points in each curve's order
     const int32_t *pos0, *pos1;      // and their places in it
     const int32_t *p0of1;            // curve-0 place of curve 1's k-th point
-    const float *xs0, *xs1;          // coordinates in each curve's order
+    const float4 *xs0, *xs1;         // coordinates in each curve's order (coords_at)
     const int32_t *qorder;           // the queries in curve-0 order
 };
 // Both curves, and the queries' order (xq; their keys go to qk0, qk1), come from one radix sort, told apart by the
@@ -450,7 +497,9 @@ nngp_status make_curves(const float *xs, int64_t n, int d, int dp, char *base, c
     NNGP_CUDA_TRY(cudaGetLastError());
     cross_pos_kernel<<<grid_of(n), kThreads, 0, stream>>>(order + n, pos, n, p0of1);
     NNGP_CUDA_TRY(cudaGetLastError());
-    out = Curves{dk.Current(), dk.Current() + n, order, order + n, pos, pos + n, p0of1, xc, xc + n * dp, order + 2 * n};
+    out = Curves{dk.Current(), dk.Current() + n, order, order + n, pos, pos + n, p0of1,
+                 reinterpret_cast<const float4 *>(xc), reinterpret_cast<const float4 *>(xc) + blocks_of(n) * 32 * (dp / 4),
+                 order + 2 * n};
     return NNGP_OK;
 }
 
@@ -470,7 +519,7 @@ nngp_status run_level(const float *xs, int64_t n, int d, int D, int dp, int m, i
 }
 
 template <int D>
-void launch_qseed(int grid, const float *xs0, const float *xs1, const uint64_t *k0s, const uint64_t *k1s, int64_t n_ref,
+void launch_qseed(int grid, const float4 *xs0, const float4 *xs1, const uint64_t *k0s, const uint64_t *k1s, int64_t n_ref,
                   const int32_t *p0of1, const float *xq, int64_t nq, const uint64_t *qk0, const uint64_t *qk1,
                   const int32_t *qorder, int dp, int m, float *seeds, cudaStream_t stream) {
     qseed_kernel<D><<<grid, kThreads, 0, stream>>>(xs0, xs1, k0s, k1s, n_ref, p0of1, xq, nq, qk0, qk1, qorder, dp, m,
