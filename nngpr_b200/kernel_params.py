@@ -77,13 +77,46 @@ def _unsupported(msg: str):
     return NotImplementedError("Cannot accelerate this kernel: " + msg)
 
 
-def _values(kernel) -> dict:
+def _held(kernel, name):
+    """The value of a leaf's hyperparameter, as the kernel holds it."""
+    return getattr(kernel, name)
+
+
+class _Probe:
+    """The values of a tree's hyperparameters at another ``theta``, taken in the order of
+    ``kernel.theta`` (first operand first): what ``kernel.clone_with_theta(theta)`` would hold, without
+    the clone (a kernel with 18 length scales: ``extract`` 759 -> 399 us on one CPU; a predict
+    call of 1,000 points 1,100 -> 690 us)."""
+
+    def __init__(self, theta):
+        self.theta, self.used = theta, 0
+
+    def __call__(self, kernel, name):
+        h = getattr(kernel, 'hyperparameter_' + name)
+        if h.fixed:
+            return getattr(kernel, name)
+        v = np.exp(self.theta[self.used:self.used + h.n_elements])
+        self.used += h.n_elements
+        return v if h.n_elements > 1 else (v[0] if v.size else np.nan)
+
+
+def _plain_tree(kernel) -> bool:
+    """Whether every node keeps scikit-learn's own ``theta`` and ``clone_with_theta``."""
+    if type(kernel).clone_with_theta is not skk.Kernel.clone_with_theta:
+        return False
+    if isinstance(kernel, (skk.Sum, skk.Product)):
+        return (type(kernel).theta is skk.KernelOperator.theta and _plain_tree(kernel.k1)
+                and _plain_tree(kernel.k2))
+    return type(kernel).theta is skk.Kernel.theta
+
+
+def _values(kernel, value=_held) -> dict:
     """Parameter dictionary of a kernel tree (keys ``noise_level``, ``constant_value``,
-    ``length_scale``, ``rbf_level``)."""
+    ``length_scale``, ``rbf_level``); ``value(leaf, name)`` gives a leaf's hyperparameter."""
     if isinstance(kernel, skk.WhiteKernel):
-        return {'noise_level': float(kernel.noise_level)}
+        return {'noise_level': float(value(kernel, 'noise_level'))}
     if isinstance(kernel, skk.ConstantKernel):
-        return {'constant_value': float(kernel.constant_value)}
+        return {'constant_value': float(value(kernel, 'constant_value'))}
     if isinstance(kernel, skk.Matern):
         # Matern subclasses RBF in scikit-learn (and in nngpr.batched_kernels), so it is tested
         # first; the reference's generic path evaluates nu = 1/2, 3/2, 5/2 and inf
@@ -92,17 +125,17 @@ def _values(kernel) -> dict:
         family = 0 if np.isinf(nu) else MATERN_FAMILY.get(nu)
         if family is None:
             raise _unsupported(f"Matern with nu = {nu} (only 0.5, 1.5, 2.5 and inf)")
-        ls = kernel.length_scale
+        ls = value(kernel, 'length_scale')
         if isinstance(ls, numbers.Number) or np.ndim(ls) == 0:
             return {'length_scale': float(ls), 'family': family}
         return {'length_scale': np.asarray(ls, dtype=np.float64).reshape(-1).copy(), 'family': family}
     if isinstance(kernel, skk.RBF):
-        ls = kernel.length_scale
+        ls = value(kernel, 'length_scale')
         if isinstance(ls, numbers.Number) or np.ndim(ls) == 0:
             return {'length_scale': float(ls)}
         return {'length_scale': np.asarray(ls, dtype=np.float64).reshape(-1).copy()}
     if isinstance(kernel, skk.Sum):
-        a, b = _values(kernel.k1), _values(kernel.k2)
+        a, b = _values(kernel.k1, value), _values(kernel.k2, value)
         a_rbf = bool(set(a) - {'noise_level', 'constant_value'})
         b_rbf = bool(set(b) - {'noise_level', 'constant_value'})
         if a_rbf and b_rbf:
@@ -115,7 +148,7 @@ def _values(kernel) -> dict:
                 b[key] = a.get(key, 0.0) + b.get(key, 0.0)
         return b
     if isinstance(kernel, skk.Product):
-        a, b = _values(kernel.k1), _values(kernel.k2)
+        a, b = _values(kernel.k1, value), _values(kernel.k2, value)
         a_const = not (set(a) - {'constant_value'})
         b_const = not (set(b) - {'constant_value'})
         if not a_const and not b_const:
@@ -138,7 +171,7 @@ def _base_kernel(kernel):
     return getattr(kernel, 'base_kernel', kernel)
 
 
-def theta_map(kernel) -> dict:
+def theta_map(kernel, n=None) -> dict:
     """Position of each parameter in ``kernel.theta``.
 
     Same rule as ``get_kernel_theta_mapping`` (``cuda_kernel_accelerators.py:583-649``):
@@ -153,25 +186,28 @@ def theta_map(kernel) -> dict:
     and removes the collision.
     """
     kernel = _base_kernel(kernel)
-    n = len(kernel.theta)
+    n = len(kernel.theta) if n is None else n
     eps = 1e-15
     maps = []
+    plain = _plain_tree(kernel)
     for a_, b_ in ((0.5, 0.1 * np.sqrt(2.0)), (0.3 * np.sqrt(3.0), -0.2 * np.sqrt(5.0))):
         probe_theta = a_ * np.arange(1, n + 1, dtype=np.float64) + b_
         expected = np.exp(probe_theta)
-        vals = _values(kernel.clone_with_theta(probe_theta))
+        probe = _Probe(probe_theta)
+        vals = _values(kernel, probe) if plain else {}
+        if not plain or probe.used != n:  # a subclass with a theta of its own, or more hyperparameters
+            vals = _values(kernel.clone_with_theta(probe_theta))
+        below, above = expected * (1 + eps), expected * (1 - eps)
 
         def hits(v):
-            return np.flatnonzero((v < expected * (1 + eps)) & (v > expected * (1 - eps)))
+            return np.flatnonzero((v < below) & (v > above))
 
         out = {}
         for key, v in vals.items():
             if key == 'length_scale' and np.ndim(v) > 0:
-                found = []
-                for comp in np.asarray(v).reshape(-1):
-                    h = hits(comp)
-                    if h.size == 1:
-                        found.append(int(h[0]))
+                comps = np.asarray(v).reshape(-1, 1)
+                at = (comps < below) & (comps > above)
+                found = [int(k) for k in at[at.sum(axis=1) == 1].argmax(axis=1)] if n > 0 else []
                 if not found:
                     continue
                 found = sorted(set(found))
@@ -199,7 +235,8 @@ def extract(kernel) -> RbfParams:
     for every other kernel."""
     kernel = _base_kernel(kernel)
     vals = _values(kernel)
-    tmap = theta_map(kernel)
+    n_theta = len(kernel.theta)
+    tmap = theta_map(kernel, n_theta)
     p = RbfParams()
     p.noise_level = float(vals.get('noise_level', 0.0))
     p.const_value = float(vals.get('constant_value', 0.0))
@@ -215,7 +252,7 @@ def extract(kernel) -> RbfParams:
     p.idx_rbf_level = tmap.get('rbf_level', -1)
     ls_idx = tmap.get('length_scale', -1)
     p.idx_ls = ls_idx[0] if isinstance(ls_idx, list) else ls_idx
-    p.n_theta = len(kernel.theta)
+    p.n_theta = n_theta
     return p
 
 
