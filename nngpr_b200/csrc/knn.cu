@@ -497,11 +497,13 @@ ScreenVariant pick_screen(int D, int M) {
 // Where the direct search is the faster one: its time is a cost per query (the selection) and per
 // pair (fitted to B200 times of d = 3..28, 500..434,874 refs, 1..100,000 queries), the others' hardly
 // depends on the number of queries while those do not fill the chip.
-//   * Against the tensor-core search below the query count that turns on its seeds: measured 320
-//     us at 500 refs, 800 at 16,599 and 4,400 at 434,874, for 64 to 4,096 queries alike (direct, d = 18:
-//     67 us for 256 queries of 16,599 refs, 126 for 1,000, 305 for 4,096); from there on it is
-//     seeded and measured 550 to 940 us at 16,384 queries (direct: 202 us at d = 3 for a set of
-//     16,384 points over itself, 306 at d = 8, 974 at d = 24 where it loses to 882).
+//   * Against the tensor-core search below the query count that turns on its seeds: measured 390
+//     us at 500 refs, 780 at 16,599 (d = 18), 1,220 at 100,000 and 2,900 at 434,874 (d = 3), for 64 to 8,192 queries
+//     alike.  Direct at 16,599 refs, d = 18: 67 us for 256 queries, 125 for 1,000, 303 for 4,096, 1,046 for 16,383;
+//     at 434,874, d = 3: 608 for 1,024, 2,104 for 4,096, 3,507 for 8,192.
+//   * From there on it is seeded: 600 us for 16,384 queries of 50,000 refs at d = 3 (direct 890), 750 at d = 8 (1,390),
+//     660 of 16,599 refs at d = 18 (1,035).  A set of 16,384 points over itself has half the pairs: direct 202 us at
+//     d = 3 (480), 308 at d = 8 (590), 517 at d = 16 (750), 977 at d = 24 (740).
 //   * A larger set searched over itself stays with the seeded and pruned prefix search.
 //   * Against the SIMT screen (num_nn 33..64 or d > 24) up to a query count that falls with d:
 //     m = 48, d = 3: 1.5 against 3.0 ms at 50,000 points, 5.2 against 5.5 at 100,000, 18 against 15 at
@@ -513,7 +515,8 @@ bool direct_pays(int64_t n_ref, int64_t n_query, int d, bool tc_ok) {
     if (seeded && n_query == n_ref && n_query > seed::kMinQueries) return false;
     const double us = nq * (2.0 + 0.35 * dp) * 1e-3 + nq * nr * (0.25 + 0.14 * dp) * 1e-6;
     // (2,500: a row shard of a large prefix search has few queries too, and is seeded)
-    return us <= (seeded ? 700.0 + 0.002 * nr : std::min(550.0 + 0.0085 * nr, 2500.0));
+    if (seeded) return us <= (n_query == n_ref ? 700.0 : 450.0) + 0.002 * nr;
+    return us <= std::min(550.0 + 0.0085 * nr, 2500.0);
 }
 
 enum class KnnPath { Tc, Simt, Generic, Direct };
