@@ -466,8 +466,8 @@ def read_profile_traffic():
 
 
 def tensor_peak_tflops(bf16_operands):
-    """Dense tensor rate of the search's operand type: the BF16 dense rate measured on this
-    pool's B200s (MEASURED_PEAKS.json, burst) for BF16 operands, half of it for TF32 (the ratio
+    """Dense tensor rate of the search's operand type: the BF16 dense rate measured on
+    B200s of this kind (MEASURED_PEAKS.json, burst) for BF16 operands, half of it for TF32 (the ratio
     of NVIDIA's dense figures, 1.1 vs 2.25 PFLOP/s)."""
     try:
         with open(os.path.join(ROOT, 'MEASURED_PEAKS.json')) as f:

@@ -5,7 +5,7 @@
 // nngpr/base_nngpr.py:530-535).  The tensor-core kernel streams the refs in index order and
 // screens each against the row's current bound, the m-th best distance found so far; in random
 // input order a row meets about m ln(i/m) list updates, and every one costs an exact rescoring
-// and a heap insert.  That candidate work, not the screen, dominates the kernel at small d.
+// and a list insert.  That candidate work, not the screen, dominates the kernel at small d.
 //
 // Any m distinct refs j < i bound the row from above: the m-th smallest of their distances is
 // >= the m-th smallest over all j < i.  This file finds such refs cheaply: two space-filling
