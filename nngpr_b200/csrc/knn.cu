@@ -498,11 +498,12 @@ ScreenVariant pick_screen(int D, int M) {
 // pair (fitted to B200 times of d = 3..28, 500..434,874 refs, 1..100,000 queries), the others' hardly
 // depends on the number of queries while those do not fill the chip.
 //   * Against the tensor-core search below the query count that turns on its seeds: measured 390
-//     us at 500 refs, 780 at 16,599 (d = 18), 1,220 at 100,000 and 2,900 at 434,874 (d = 3), for 64 to 8,192 queries
-//     alike.  Direct at 16,599 refs, d = 18: 67 us for 256 queries, 125 for 1,000, 303 for 4,096, 1,046 for 16,383;
-//     at 434,874, d = 3: 608 for 1,024, 2,104 for 4,096, 3,507 for 8,192.
-//   * From there on it is seeded: 600 us for 16,384 queries of 50,000 refs at d = 3 (direct 890), 750 at d = 8 (1,390),
-//     660 of 16,599 refs at d = 18 (1,035).  A set of 16,384 points over itself has half the pairs: direct 202 us at
+//     us at 500 refs, 550 to 600 at 16,599 (d = 18, to 4,096 queries; 784 for 16,383), 560 for 1,000 and 842 for 8,192 queries of
+//     100,000 and 920, 1,170 and 1,610 for 1,024, 4,096 and 8,192 of 434,874 (d = 3).  Direct at 16,599 refs, d = 18:
+//     67 us for 256 queries, 125 for 1,000, 303 for 4,096, 1,042 for 16,383; at 100,000, d = 3: 173 for 1,000, 927
+//     for 8,192; at 434,874: 614 for 1,024, 2,077 for 4,096.
+//   * From there on it is seeded: 454 us for 16,384 queries of 50,000 refs at d = 3 (direct 890), 620 at d = 8 (1,380),
+//     597 of 16,599 refs at d = 18 (1,033).  A set of 16,384 points over itself has half the pairs: direct 202 us at
 //     d = 3 (480), 308 at d = 8 (590), 517 at d = 16 (750), 977 at d = 24 (740).
 //   * A larger set searched over itself stays with the seeded and pruned prefix search.
 //   * Against the SIMT screen (num_nn 33..64 or d > 24) up to a query count that falls with d:
@@ -514,12 +515,43 @@ bool direct_pays(int64_t n_ref, int64_t n_query, int d, bool tc_ok) {
     const bool seeded = n_query >= seed::kMinQueries;
     if (seeded && n_query == n_ref && n_query > seed::kMinQueries) return false;
     const double us = nq * (2.0 + 0.35 * dp) * 1e-3 + nq * nr * (0.25 + 0.14 * dp) * 1e-6;
-    // (2,500: a row shard of a large prefix search has few queries too, and is seeded)
-    if (seeded) return us <= (n_query == n_ref ? 700.0 : 450.0) + 0.002 * nr;
-    return us <= std::min(550.0 + 0.0085 * nr, 2500.0);
+    if (seeded) return us <= (n_query == n_ref ? 700.0 + 0.002 * nr : 400.0);
+    return us <= 450.0 + 0.0006 * nr;
 }
 
 enum class KnnPath { Tc, Simt, Generic, Direct };
+
+// Items that each group of queries of an unpruned tensor-core search is split into, so that few groups fill the
+// chip's CTAs in one wave: 16,384 queries of 16,599 refs, d = 18, 659 -> 597 us (129 groups, two parts); of 50,000, d = 3,
+// 603 -> 454 us; 1,000 queries of 434,874, d = 3, 2,900 -> 940 us (8 parts).  A part starts its lists anew from the seeds,
+// so a set searched over itself, whose groups are uneven but start heaviest first, is not split (50,000 points, d =
+// 20, 1,567 us; 1,834 in two parts; 30,000, d = 3, 617; 696).
+int tc_parts(int64_t n_ref, int64_t n_query, const tc::TcVariant &tv, bool has_cut) {
+    if (has_cut && 2 * n_query > n_ref) return 1;
+    const int64_t groups = (n_query + tv.rows_per_item - 1) / tv.rows_per_item;
+    const int64_t slots = (int64_t)kNumSMsB200 * tv.ctas_per_sm, tiles = (n_ref + tc::kTcRefTile - 1) / tc::kTcRefTile;
+    return (int)std::max<int64_t>(1, std::min<int64_t>({slots / groups, tiles / 16, 8}));
+}
+
+// Lists of queries from the sorted lists of their parts (32 keys each: distance bits << 32 | index), one warp each.
+__global__ void __launch_bounds__(256) merge_parts_kernel(const unsigned long long *__restrict__ partial, int parts, int G,
+                                                          int64_t n_query, int m, int32_t *__restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t q = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (q >= n_query) return;
+    const int64_t g = q / G, r = q - g * G;
+    unsigned long long cur = partial[((g * parts) * G + r) * 32 + lane];
+    for (int k = 1; k < parts; ++k) {
+        const unsigned long long nx = partial[((g * parts + k) * G + r) * 32 + (31 - lane)];
+        cur = nx < cur ? nx : cur;  // the 32 smallest of both lists, a bitonic sequence
+#pragma unroll
+        for (int j = 16; j > 0; j >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, cur, j);
+            cur = ((lane & j) == 0) ? (o < cur ? o : cur) : (o > cur ? o : cur);
+        }
+    }
+    if (lane < m) out[q * m + lane] = (int32_t)(uint32_t)cur;
+}
 
 // Search kernel: NNGP_KNN_KERNEL=tc|simt|generic|direct forces a kernel where the shape has one
 // (testing and comparisons); unset or any other value selects by the rule at direct_pays, then the
@@ -545,7 +577,7 @@ struct KnnPlan {
     KnnPath path = KnnPath::Generic;
     int dp = 0;  // padded row length of the scaled arrays
     int64_t n_ref_pad = 0;
-    size_t off_ref = 0, off_q = 0, off_rec = 0, off_acc = 0, off_r2 = 0, off_ctr = 0, off_ldist = 0, off_lidx = 0,
+    size_t off_parts = 0, parts_bytes = 0, off_ref = 0, off_q = 0, off_rec = 0, off_acc = 0, off_r2 = 0, off_ctr = 0, off_ldist = 0, off_lidx = 0,
            off_seed = 0, off_seed_ws = 0, seed_ws_bytes = 0, off_tiles2 = 0, off_prune_ws = 0, prune_ws_bytes = 0,
            total = 0;
     ScreenVariant v{};
@@ -586,6 +618,13 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same) {
         off = align_up(off + 16, 256);
         p.off_ctr = off;
         off = align_up(off + 16, 256);
+        if (p.path == KnnPath::Tc) {  // partial lists of an unpruned search's parts
+            const int64_t groups = (n_query + p.tv.rows_per_item - 1) / p.tv.rows_per_item;
+            const int parts = std::max(tc_parts(n_ref, n_query, p.tv, false), tc_parts(n_ref, n_query, p.tv, true));
+            p.parts_bytes = parts > 1 ? (size_t)groups * parts * p.tv.rows_per_item * 32 * 8 : 0;
+            p.off_parts = off;
+            off = align_up(off + p.parts_bytes, 256);
+        }
         // seeds and pruned lists: of the prefix search (same) or, for other queries, of the query
         // search (the size query plans with same = false and takes the larger of the two)
         const size_t seed_ws = p.path != KnnPath::Tc ? 0
@@ -820,10 +859,19 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
                 lst = prune::merge(lists, 0, G, m, 0, out, stream);
             } else {
                 // rows are query rows (limit = row + cut); a seeded shard's seeds are indexed by point
-                const int64_t items = (n_query + p.tv.rows_per_item - 1) / p.tv.rows_per_item;
-                const tc::TcItems whole{};
+                const int64_t groups = (n_query + p.tv.rows_per_item - 1) / p.tv.rows_per_item;
+                tc::TcItems whole{};
+                whole.parts = tc_parts(n_ref, n_query, p.tv, has_cut != 0);
+                if (p.parts_bytes == 0) whole.parts = 1;
+                whole.partial = reinterpret_cast<unsigned long long *>(base + p.off_parts);
                 const float *seeds_rows = seeds_c ? seeds_c + row_lo : nullptr;
-                lst = launch(tiles, items, none, none, no_sizes, whole, none, none, none, ctr, seeds_rows, cut, 0, q_c);
+                lst = launch(tiles, groups * whole.parts, none, none, no_sizes, whole, none, none, none, ctr, seeds_rows, cut, 0,
+                             q_c);
+                if (lst == NNGP_OK && whole.parts > 1) {
+                    merge_parts_kernel<<<(int)((n_query + 7) / 8), 256, 0, stream>>>(whole.partial, whole.parts, G, n_query, m,
+                                                                                     out);
+                    NNGP_CUDA_TRY(cudaGetLastError());
+                }
             }
             if (lst != NNGP_OK) return lst;
         }

@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
     const bool pruned = tile_list != nullptr;
     const int64_t first_row = dev_sizes ? dev_sizes[0] : 0;
     const int64_t n_rows = dev_sizes ? dev_sizes[1] : n_query;
-    const int64_t n_items = dev_sizes ? dev_sizes[2] : (n_query + C::ROWS - 1) / C::ROWS;
+    const int64_t n_items = dev_sizes ? dev_sizes[2] : (n_query + C::ROWS - 1) / C::ROWS * items.parts;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
@@ -575,8 +575,10 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
         __syncthreads();
         if (stop) break;
         const int64_t desc = items.order ? (int64_t)items.order[item] : -1;  // the item's descriptor
-        const int64_t qtile = desc >= 0 ? (int64_t)items.group[desc] : (has_cut ? (n_items - 1 - item) : item);
-        const int32_t out_slot = desc >= 0 ? items.slot[desc] : -1;  // >= 0: partial lists for a merge
+        const int64_t place = has_cut ? n_items - 1 - item : item;  // without descriptors: group, then part of it
+        const int64_t qtile = desc >= 0 ? (int64_t)items.group[desc] : place / items.parts;
+        // >= 0: partial lists for a merge
+        const int32_t out_slot = desc >= 0 ? items.slot[desc] : (items.parts > 1 ? (int32_t)place : -1);
         int64_t q0, n_item_rows;  // the item's first row position and its row count
         if (row_off) {
             q0 = row_off[qtile];
@@ -594,7 +596,10 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
             ntiles = (uint32_t)(tile_off[qtile + 1] - tile_off[qtile]);
         } else {
             const int64_t block_limit = limit_of(point_of(q0 + n_item_rows - 1));
-            ntiles = (uint32_t)((block_limit + RT - 1) / RT);
+            const uint32_t all = (uint32_t)((block_limit + RT - 1) / RT), parts = (uint32_t)items.parts;
+            const uint32_t part = (uint32_t)(place % items.parts);
+            tfirst = (uint32_t)((uint64_t)all * part / parts);
+            ntiles = (uint32_t)((uint64_t)all * (part + 1) / parts) - tfirst;
         }
         const int32_t *tl = pruned ? tile_list + tile_off[qtile] + tfirst : nullptr;  // this item's ref tiles
         // the item's stages: its tiles one per stage, or two (PAIR: tiles 2u and 2u + 1 in stage u,

@@ -18,6 +18,8 @@ constexpr int kTcQueryTile = 128;  // queries per tile (UMMA M)
 struct TcItems {
     const int32_t *group = nullptr, *t0 = nullptr, *t1 = nullptr, *slot = nullptr, *order = nullptr;
     unsigned long long *partial = nullptr;
+    // All null but partial: each group's tiles in this many items, part p of group g writing slot g parts + p
+    int parts = 1;
 };
 
 using TcFn = void (*)(const unsigned char *, const float *, const double *, const unsigned int *, const float *,

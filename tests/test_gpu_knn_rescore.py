@@ -54,3 +54,19 @@ def test_curves_of_one_sort_match_the_direct_search(monkeypatch, d):
             monkeypatch.setenv('NNGP_KNN_KERNEL', kernel)
             lists.append(ops.knn(rt, a, 32, cut, None))
         assert torch.equal(lists[0], lists[1])
+
+
+@pytest.mark.parametrize('d', [3, 8, 16, 20])
+@pytest.mark.parametrize('n,nq', [(9001, 0), (2047, 130), (4096, 700), (20001, 0), (16600, 16500)])
+def test_parts_of_an_unpruned_search_match_the_direct_search(monkeypatch, d, n, nq):
+    """Groups split into parts of their tiles (several in number, down to none where a prefix is short) and merged."""
+    rng = np.random.default_rng(n + d)
+    rt = torch.from_numpy(rng.normal(size=(n, d)).astype(np.float32)).cuda()
+    rt[n // 2] = rt[n // 3]
+    q = rt if nq == 0 else torch.from_numpy(rng.normal(size=(nq, d)).astype(np.float32)).cuda()
+    for m, cut in ((32, 0), (5, 0)) if nq == 0 else ((32, None), (7, -100), (32, 1000)):
+        lists = []
+        for kernel in ('tc', 'direct'):
+            monkeypatch.setenv('NNGP_KNN_KERNEL', kernel)
+            lists.append(ops.knn(rt, q, m, cut, None))
+        assert torch.equal(lists[0], lists[1])
