@@ -311,6 +311,19 @@ __device__ __forceinline__ bool poll_bounded(const uint32_t *p, uint64_t limit_n
         if ((float)(global_timer_ns() - t0) > (float)limit_ns * (float)waits) return false;
     }
 }
+// The same for a whole warp: lane 0 polls, every lane gets the value.  A shuffle orders no memory, so what lane
+// 0's acquire load makes visible reaches the other lanes (their reads of entries, their writes to places that are
+// free again) through the barrier after it.
+template <typename F>
+__device__ __forceinline__ bool warp_poll(int lane, const uint32_t *p, uint64_t limit_ns, uint32_t waits, uint32_t &v,
+                                          F &&ready) {
+    bool ok = true;
+    if (lane == 0) ok = poll_bounded(p, limit_ns, waits, v, ready);
+    v = __shfl_sync(0xffffffffu, v, 0);
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok;
+}
 
 // A row's m best so far, unordered: distances d[0 .. 31] (slots >= m: -inf), the largest of each four at
 // d[32 .. 39], indices, and the slot of the largest (distance, index).  Replaces that slot by (x, j) when (x, j)
@@ -883,12 +896,8 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                     const uint32_t cnt = (uint32_t)__popc(mk);
                     if (cnt == 0) continue;
                     if (head + cnt - tail > (uint32_t)RING) {  // warp-uniform: wait for places
-                        bool ok = true;
-                        if (lane == 0)
-                            ok = poll_bounded(ring_tail + warp, wait_ns, 1, tail,
-                                              [&](uint32_t v) { return head + cnt - v <= (uint32_t)RING; });
-                        tail = __shfl_sync(FULL, tail, 0);
-                        if (!__shfl_sync(FULL, ok, 0)) {
+                        if (!warp_poll(lane, ring_tail + warp, wait_ns, 1, tail,
+                                       [&](uint32_t v) { return head + cnt - v <= (uint32_t)RING; })) {
                             aborted = true;
                             break;
                         }
@@ -929,13 +938,9 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                     if (done) break;
                     // the screening warp may find nothing in all of the item's stages: the limit is the sum of
                     // its own waits, each of which ends in RING_DONE | RING_ABORT when it runs out
-                    bool ok = true;
-                    if (lane == 0)
-                        ok = poll_bounded(ring_head + w, wait_ns, nstg + 2, seen, [&](uint32_t v) {
+                    if (!warp_poll(lane, ring_head + w, wait_ns, nstg + 2, seen, [&](uint32_t v) {
                             return (v & RING_DONE) != 0u || (v & ~RING_ABORT) - tail >= (uint32_t)RING_MIN;
-                        });
-                    seen = __shfl_sync(FULL, seen, 0);
-                    if (!__shfl_sync(FULL, ok, 0)) {
+                        })) {
                         aborted = true;
                         break;
                     }
