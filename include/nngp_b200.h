@@ -135,14 +135,20 @@ uint64_t nngp_set_wait_limit_ns(uint64_t ns);
  * per operation, so the lists equal those of an exact search in that precision.
  *
  * The fit step's search of a set over itself (ref == query, n_ref == n_query, has_ref_cut with
- * ref_cut_index 0, FP32, n >= 8,192) starts every row from a proven bound of its num_nn-th
- * distance (Morton-window seeds) and, for d <= 24 and 65,536 <= n <= 2,000,000, visits per group
- * of rows only the ref tiles bounding boxes cannot exclude; the lists are the same.
+ * ref_cut_index 0, FP32, n >= 8,192), where it takes the tensor-core kernel (nngp_knn_path: sets
+ * up to 16,384 points mostly take the direct one), starts every row from a proven bound of its
+ * num_nn-th distance (Morton-window seeds) and, for d <= 24 and 65,536 <= n <= 2,000,000, visits per
+ * group of rows only the ref tiles that boxes (and, from 9 features and 131,072 points on, slabs
+ * between k-means cells) cannot exclude; the lists are the same.
  * A search of other queries without a cut (predict: n_ref >= 8,192, n_query >= 16,384) seeds
  * every query from the refs' curve windows around it and, for d <= 24, prunes the same way.
  * NNGP_KNN_SEED_W=0 / NNGP_KNN_PRUNE=0 switch these off (testing).  The workspace covers them.
  * ------------------------------------------------------------------------------------- */
 size_t nngp_knn_workspace_size_f32(int64_t n_ref, int64_t n_query, int32_t d, int32_t num_nn);
+/* The kernel that a search takes: 0 tensor-core, 1 SIMT screen, 2 generic, 3 direct; -1 for an empty one.
+ * (f64: nngp_knn_f64.  Host only.) */
+int32_t nngp_knn_path(int64_t n_ref, int64_t n_query, int32_t d, int32_t num_nn, int32_t has_ref_cut,
+                      int64_t ref_cut_index, int32_t f64);
 nngp_status nngp_knn_f32(const float *ref, int64_t n_ref, const float *query, int64_t n_query,
                          int32_t d, const double *length_scale, int32_t n_ls, int32_t num_nn,
                          int32_t has_ref_cut, int64_t ref_cut_index, int32_t *out_idx,

@@ -30,6 +30,7 @@ EXPORTED = (
     'nngp_plain_knn_f32', 'nngp_knn_reuse_prepare_f32', 'nngp_knn_reuse_rank_f32',
     'nngp_predict_full_workspace_size', 'nngp_predict_full_f64', 'nngp_sample_full_f64',
     'nngp_predict_cov_full_f64', 'nngp_theta_params', 'nngp_knn_f32_ls_device', 'nngp_knn_f64_ls_device',
+    'nngp_knn_path',
 )
 
 
@@ -70,6 +71,7 @@ _SIGS = {
     'nngp_check_device': ([], ctypes.c_int),
     'nngp_knn_workspace_size_f32': ([_i64, _i64, _i32, _i32], _sz),
     'nngp_knn_workspace_size_f64': ([_i64, _i64, _i32, _i32], _sz),
+    'nngp_knn_path': ([_i64, _i64, _i32, _i32, _i32, _i64, _i32], _i32),
     'nngp_knn_f32': ([_vp, _i64, _vp, _i64, _i32, _dp, _i32, _i32, _i32, _i64, _vp, _vp, _vp, _sz, _vp], ctypes.c_int),
     'nngp_knn_f64': ([_vp, _i64, _vp, _i64, _i32, _dp, _i32, _i32, _i32, _i64, _vp, _vp, _vp, _sz, _vp], ctypes.c_int),
     'nngp_knn_f32_ls_device': ([_vp, _i64, _vp, _i64, _i32, _vp, _i32, _i32, _i32, _i64, _vp, _vp, _vp, _sz, _vp],

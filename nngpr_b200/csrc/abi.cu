@@ -16,6 +16,7 @@ namespace nngp {
 
 // implemented in knn.cu / local.cu
 size_t knn_workspace_f32(int64_t n_ref, int64_t n_query, int d, int m);
+int knn_path(int64_t n_ref, int64_t n_query, int d, int m, int has_cut, int64_t cut, int f64);
 size_t knn_workspace_f64(int64_t n_ref, int64_t n_query, int d, int m);
 nngp_status knn_f32(const float *, int64_t, const float *, int64_t, int, const double *, int, int, int, int64_t,
                     int32_t *, int32_t *, void *, size_t, cudaStream_t);
@@ -162,6 +163,12 @@ size_t nngp_knn_workspace_size_f32(int64_t n_ref, int64_t n_query, int32_t d, in
 }
 size_t nngp_knn_workspace_size_f64(int64_t n_ref, int64_t n_query, int32_t d, int32_t num_nn) {
     return knn_workspace_f64(n_ref, n_query, d, num_nn);
+}
+
+int32_t nngp_knn_path(int64_t n_ref, int64_t n_query, int32_t d, int32_t num_nn, int32_t has_ref_cut,
+                      int64_t ref_cut_index, int32_t f64) {
+    if (n_ref <= 0 || n_query <= 0 || d <= 0 || num_nn <= 0) return -1;
+    return knn_path(n_ref, n_query, d, num_nn, has_ref_cut, ref_cut_index, f64);
 }
 
 nngp_status nngp_knn_f32(const float *ref, int64_t n_ref, const float *query, int64_t n_query, int32_t d,

@@ -494,38 +494,45 @@ ScreenVariant pick_screen(int D, int M) {
     return ScreenVariant{};
 }
 
-// Where the direct search is the faster one: its time is a cost per query (the selection) and per
-// pair (fitted to B200 times of d = 3..28, 500..434,874 refs, 1..100,000 queries), the others' hardly
-// depends on the number of queries while those do not fill the chip.
-//   * Against the tensor-core search below the query count that turns on its seeds: measured 390
-//     us at 500 refs, 550 to 600 at 16,599 (d = 18, to 4,096 queries; 784 for 16,383), 560 for 1,000 and 842 for 8,192 queries of
-//     100,000 and 920, 1,170 and 1,610 for 1,024, 4,096 and 8,192 of 434,874 (d = 3).  Direct at 16,599 refs, d = 18:
-//     67 us for 256 queries, 125 for 1,000, 303 for 4,096, 1,042 for 16,383; at 100,000, d = 3: 173 for 1,000, 927
-//     for 8,192; at 434,874: 614 for 1,024, 2,077 for 4,096.
-//   * From there on it is seeded: 454 us for 16,384 queries of 50,000 refs at d = 3 (direct 890), 620 at d = 8 (1,380),
-//     597 of 16,599 refs at d = 18 (1,033).  A set of 16,384 points over itself has half the pairs: direct 202 us at
-//     d = 3 (480), 308 at d = 8 (590), 517 at d = 16 (750), 977 at d = 24 (740).
-//   * A larger set searched over itself stays with the seeded and pruned prefix search.
-//   * Against the SIMT screen (num_nn 33..64 or d > 24) up to a query count that falls with d:
-//     m = 48, d = 3: 1.5 against 3.0 ms at 50,000 points, 5.2 against 5.5 at 100,000, 18 against 15 at
-//     200,000; d = 16: 4.3 against 5.3 ms at 50,000, 16 against 11 at 100,000.
-bool direct_pays(int64_t n_ref, int64_t n_query, int d, bool tc_ok) {
+// (query, ref) pairs of a search: with a cut, query q has the refs below clamp(q + cut, 0, n_ref).
+double pairs_of(int64_t n_ref, int64_t n_query, bool has_cut, int64_t cut) {
+    const double nr = (double)n_ref, nq = (double)n_query, c = (double)cut;
+    if (!has_cut) return nr * nq;
+    const double a = std::min(std::max(-c, 0.0), nq), b = std::min(std::max(nr - c, a), nq);
+    return (b - a) * (c + 0.5 * (a + b - 1.0)) + (nq - b) * nr;
+}
+
+// Where the direct search is the faster one.  `us` fits its time: a cost per query (the selection) and per pair.
+// The tensor-core search's hardly depends on the number of queries while those do not fill the chip; each
+// line is its time at the sizes where the two meet (B200, 32 neighbours; direct / tensor-core, us):
+//   * a cut, in practice a set over itself, which has half the pairs: d = 8 275 / 582, 16 499 / 759, 20 556 / 710 and
+//     24 892 / 730 for 16,384 points, d = 24 517 / 687 for 12,000.  Larger sets stay with the seeded and
+//     pruned prefix search, to which its tests hold them (at d = 3 the direct one would win up to about 30,000
+//     points: 277 / 533 for 20,000);
+//   * few queries, without seeds: d = 3 476 / 679 for 4,096 of 100,000 refs, 790 / 843 for 8,192, 1,038 / 939 for
+//     2,048 of 434,874; d = 18 501 / 679 for 8,192 of 16,599, 730 / 724 for 12,000; d = 16 677 / 708 for 16,383
+//     of 12,000;
+//   * from seed::kMinQueries queries and kMinPoints refs on it is seeded, and faster: for 16,384 queries
+//     d = 3 280 / 284 at 12,000 refs, 310 / 292 at 14,000; d = 8 429 / 426 at 14,000; d = 16 519 / 514 at 8,192.
+// Against the SIMT screen (num_nn 33..64 or d > 24) up to a query count that falls with d: m = 48, a set over
+// itself, d = 3: 1.5 against 3.0 ms at 50,000 points, 5.2 against 5.5 at 100,000, 18 against 15 at 200,000; d = 16: 4.3
+// against 5.3 ms at 50,000, 16 against 11 at 100,000.
+bool direct_pays(int64_t n_ref, int64_t n_query, int d, bool tc_ok, bool has_cut, double pairs) {
     const double nr = (double)n_ref, nq = (double)n_query, dp = direct::row_len(d);
     if (!tc_ok) return nq * (dp + 2.0) <= 600000.0;
-    const bool seeded = n_query >= seed::kMinQueries;
-    if (seeded && n_query == n_ref && n_query > seed::kMinQueries) return false;
-    const double us = nq * (2.0 + 0.35 * dp) * 1e-3 + nq * nr * (0.25 + 0.14 * dp) * 1e-6;
-    if (seeded) return us <= (n_query == n_ref ? 700.0 + 0.002 * nr : 400.0);
-    return us <= 450.0 + 0.0006 * nr;
+    const double us = nq * (2.0 + 0.35 * dp) * 1e-3 + pairs * (0.25 + 0.14 * dp) * 1e-6;
+    if (has_cut) return n_query <= seed::kMinQueries && us <= 380.0 + 10.0 * dp + 0.0006 * nr;
+    if (n_query >= seed::kMinQueries && n_ref >= seed::kMinPoints) return us <= std::min(120.0 + 30.0 * dp, 560.0);
+    return us <= 430.0 + 0.0006 * nr + 0.01 * nq;
 }
 
 enum class KnnPath { Tc, Simt, Generic, Direct };
 
 // Items that each group of queries of an unpruned tensor-core search is split into, so that few groups fill the
-// chip's CTAs in one wave: 16,384 queries of 16,599 refs, d = 18, 659 -> 597 us (129 groups, two parts); of 50,000, d = 3,
-// 603 -> 454 us; 1,000 queries of 434,874, d = 3, 2,900 -> 940 us (8 parts).  A part starts its lists anew from the seeds,
-// so a set searched over itself, whose groups are uneven but start heaviest first, is not split (50,000 points, d =
-// 20, 1,567 us; 1,834 in two parts; 30,000, d = 3, 617; 696).
+// chip's CTAs in one wave: 16,384 queries of 16,599 refs, d = 18, 659 -> 597 us (129 groups, two parts); of 50,000,
+// d = 3, 603 -> 454 us; 1,000 queries of 434,874, d = 3, 2,900 -> 940 us (8 parts).  A part starts its lists anew from
+// the seeds, so a set searched over itself, whose groups are uneven but start heaviest first, is not split
+// (50,000 points, d = 20, 1,567 us; 1,834 in two parts; 30,000, d = 3, 617; 696).
 int tc_parts(int64_t n_ref, int64_t n_query, const tc::TcVariant &tv, bool has_cut) {
     if (has_cut && 2 * n_query > n_ref) return 1;
     const int64_t groups = (n_query + tv.rows_per_item - 1) / tv.rows_per_item;
@@ -553,43 +560,51 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const unsigned long lo
     if (lane < m) out[q * m + lane] = (int32_t)(uint32_t)cur;
 }
 
+// The search of a shape without the direct kernel: the tensor-core screen where the shape has a variant (FP32, d <= 24
+// apart from 9-11 padded to 12 etc., num_nn <= 32), else the SIMT screen, else the generic kernel.
+KnnPath screened_path(int d, int m, bool is_float) {
+    const int M = round_m(m), D = round_d(d);
+    if (!is_float || D == 0 || M == 0) return KnnPath::Generic;
+    if (M <= 32 && tc_variant(D, M).fn != nullptr) return KnnPath::Tc;
+    return M == 64 && D > 16 ? KnnPath::Generic : KnnPath::Simt;
+}
+
+bool direct_ok(int64_t n_ref, int m) { return m <= direct::kMaxNeighbours && n_ref <= (int64_t)1 << 30; }
+
 // Search kernel: NNGP_KNN_KERNEL=tc|simt|generic|direct forces a kernel where the shape has one
-// (testing and comparisons); unset or any other value selects by the rule at direct_pays, then the
-// tensor-core screen where the shape has a variant (FP32, d <= 24 apart from 9-11 padded to 12
-// etc., num_nn <= 32), else the SIMT screen, else the generic kernel.
-KnnPath choose_path(int64_t n_ref, int64_t n_query, int d, int m, bool is_float) {
+// (testing and comparisons); unset or any other value selects by the rule at direct_pays, then as screened_path.
+KnnPath choose_path(int64_t n_ref, int64_t n_query, int d, int m, bool is_float, bool has_cut, double pairs) {
     const char *env = std::getenv("NNGP_KNN_KERNEL");
     const std::string want = env ? env : "auto";
-    const int M = round_m(m), D = round_d(d);
-    const bool tc_ok = is_float && D != 0 && M != 0 && M <= 32 && tc_variant(D, M).fn != nullptr;
-    const bool simt_ok = is_float && D != 0 && M != 0 && !(M == 64 && D > 16);
-    const bool direct_ok = m <= direct::kMaxNeighbours && n_ref <= (int64_t)1 << 30;
+    const KnnPath other = screened_path(d, m, is_float);
     if (want == "generic") return KnnPath::Generic;
-    if (want == "simt") return simt_ok ? KnnPath::Simt : KnnPath::Generic;
-    if (want == "tc" && tc_ok) return KnnPath::Tc;
-    if (want == "direct" && direct_ok) return KnnPath::Direct;
-    if (direct_ok && ((!tc_ok && !simt_ok) || direct_pays(n_ref, n_query, d, tc_ok))) return KnnPath::Direct;
-    if (tc_ok) return KnnPath::Tc;  // faster than the SIMT screen at every d measured on B200 (3, 8, 16)
-    return simt_ok ? KnnPath::Simt : KnnPath::Generic;
+    if (want == "simt") {
+        const int M = round_m(m), D = round_d(d);
+        return is_float && D != 0 && M != 0 && !(M == 64 && D > 16) ? KnnPath::Simt : KnnPath::Generic;
+    }
+    if (want == "tc" && other == KnnPath::Tc) return other;
+    if (!direct_ok(n_ref, m)) return other;
+    if (want == "direct" || other == KnnPath::Generic) return KnnPath::Direct;
+    return direct_pays(n_ref, n_query, d, other == KnnPath::Tc, has_cut, pairs) ? KnnPath::Direct : other;
 }
 
 struct KnnPlan {
     KnnPath path = KnnPath::Generic;
     int dp = 0;  // padded row length of the scaled arrays
     int64_t n_ref_pad = 0;
-    size_t off_parts = 0, parts_bytes = 0, off_ref = 0, off_q = 0, off_rec = 0, off_acc = 0, off_r2 = 0, off_ctr = 0, off_ldist = 0, off_lidx = 0,
-           off_seed = 0, off_seed_ws = 0, seed_ws_bytes = 0, off_tiles2 = 0, off_prune_ws = 0, prune_ws_bytes = 0,
-           total = 0;
+    size_t off_parts = 0, parts_bytes = 0, off_ref = 0, off_q = 0, off_rec = 0, off_acc = 0, off_r2 = 0, off_ctr = 0,
+           off_ldist = 0, off_lidx = 0, off_seed = 0, off_seed_ws = 0, seed_ws_bytes = 0, off_tiles2 = 0,
+           off_prune_ws = 0, prune_ws_bytes = 0, total = 0;
     ScreenVariant v{};
     tc::TcVariant tv{};
 };
 
 template <typename T>
-KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same) {
+KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same, KnnPath path) {
     KnnPlan p;
     const int M = round_m(m);
     const int D = round_d(d);
-    p.path = choose_path(n_ref, n_query, d, m, std::is_same<T, float>::value);
+    p.path = path;
     if (p.path == KnnPath::Tc) {
         p.tv = tc_variant(D, M);
         p.dp = p.tv.dp;
@@ -691,7 +706,9 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
         return NNGP_OK;
     }
     const bool same = (ref == query) && (n_ref == n_query);
-    KnnPlan p = make_plan<T>(n_ref, n_query, d, m, same);
+    const KnnPath path = choose_path(n_ref, n_query, d, m, std::is_same<T, float>::value, has_cut != 0,
+                                     pairs_of(n_ref, n_query, has_cut != 0, cut));
+    const KnnPlan p = make_plan<T>(n_ref, n_query, d, m, same, path);
     if (!ws || ws_bytes < p.total) return fail(NNGP_ERR_WORKSPACE, "knn: workspace missing or too small");
     char *base = reinterpret_cast<char *>(align_up(reinterpret_cast<uintptr_t>(ws), 1024));
     T *refs = reinterpret_cast<T *>(base + p.off_ref);
@@ -909,15 +926,32 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
     return NNGP_OK;
 }
 
+// Bytes for a search with or without a cut, which the size functions are not told: the path of either at the most
+// pairs that it can have, and the direct one, which a cut that leaves fewer pairs may take.
+template <typename T>
+size_t workspace_bytes(int64_t n_ref, int64_t n_query, int d, int m) {
+    if (n_ref <= 0 || n_query <= 0 || d <= 0 || m <= 0) return 256;
+    const double pairs = pairs_of(n_ref, n_query, false, 0);
+    size_t bytes = 0;
+    for (bool has_cut : {false, true}) {
+        const KnnPath path = choose_path(n_ref, n_query, d, m, std::is_same<T, float>::value, has_cut, pairs);
+        bytes = std::max(bytes, make_plan<T>(n_ref, n_query, d, m, false, path).total);
+    }
+    if (direct_ok(n_ref, m)) bytes = std::max(bytes, make_plan<T>(n_ref, n_query, d, m, false, KnnPath::Direct).total);
+    return bytes;
+}
+
 }  // namespace
 
 size_t knn_workspace_f32(int64_t n_ref, int64_t n_query, int d, int m) {
-    if (n_ref <= 0 || n_query <= 0 || d <= 0 || m <= 0) return 256;
-    return make_plan<float>(n_ref, n_query, d, m, false).total;
+    return workspace_bytes<float>(n_ref, n_query, d, m);
 }
 size_t knn_workspace_f64(int64_t n_ref, int64_t n_query, int d, int m) {
-    if (n_ref <= 0 || n_query <= 0 || d <= 0 || m <= 0) return 256;
-    return make_plan<double>(n_ref, n_query, d, m, false).total;
+    return workspace_bytes<double>(n_ref, n_query, d, m);
+}
+
+int knn_path(int64_t n_ref, int64_t n_query, int d, int m, int has_cut, int64_t cut, int f64) {
+    return (int)choose_path(n_ref, n_query, d, m, f64 == 0, has_cut != 0, pairs_of(n_ref, n_query, has_cut != 0, cut));
 }
 
 nngp_status knn_f32(const float *ref, int64_t n_ref, const float *query, int64_t n_query, int d, const double *ls,
