@@ -230,7 +230,9 @@ __global__ void __launch_bounds__(kKnnThreads) knn_screen_kernel(const float4 *_
         int64_t l = qq + cut;
         return l < 0 ? 0 : (l > n_ref ? n_ref : l);
     };
-    const int64_t limit = active ? limit_of(q) : 0;
+    // (threads past the last query follow its limit: with 0 their warp took the boundary form on every tile, and one
+    // such block held the whole search up: 8,000 queries of 100,000, d = 16, 48 neighbours, 8.5 -> 5.2 ms)
+    const int64_t limit = limit_of(active ? q : n_query - 1);
     const int64_t block_limit = limit_of(min(q0 + kKnnThreads, n_query) - 1);
     const int64_t ntiles = (block_limit + TJ - 1) / TJ;
 
@@ -514,12 +516,17 @@ double pairs_of(int64_t n_ref, int64_t n_query, bool has_cut, int64_t cut) {
 //     of 12,000;
 //   * from seed::kMinQueries queries and kMinPoints refs on it is seeded, and faster: for 16,384 queries
 //     d = 3 280 / 284 at 12,000 refs, 310 / 292 at 14,000; d = 8 429 / 426 at 14,000; d = 16 519 / 514 at 8,192.
-// Against the SIMT screen (num_nn 33..64 or d > 24) up to a query count that falls with d: m = 48, a set over
-// itself, d = 3: 1.5 against 3.0 ms at 50,000 points, 5.2 against 5.5 at 100,000, 18 against 15 at 200,000; d = 16: 4.3
-// against 5.3 ms at 50,000, 16 against 11 at 100,000.
+// The SIMT screen (num_nn 33..64 or d > 24) takes one thread per query, so that its time goes in steps of 18,944
+// queries; both times grow with the refs, and the line lies at a number of queries (of half the points of a set
+// over itself), direct / SIMT in ms with 48 neighbours:
+//   * d = 3 3.6 / 4.4 for 40,000 queries of 100,000, 13.2 / 14.6 of 434,874, 32.4 / 28.8 for 100,000; 1.9 / 2.4 for
+//     60,000 points over themselves, 4.8 / 4.7 for 100,000; d = 8 5.6 / 8.6 for 40,000 of 100,000, 54.7 / 52.8 for
+//     100,000 of 434,874;
+//   * d = 16 5.0 / 7.2 for 20,000 of 100,000, 7.5 / 7.2 for 30,000; 2.5 / 2.9 for 40,000 over themselves, 3.7 / 3.5 for
+//     50,000; d = 26 (32 neighbours) 5.3 / 6.5 for 10,000 of 100,000, 8.4 / 6.5 for 16,000.
 bool direct_pays(int64_t n_ref, int64_t n_query, int d, bool tc_ok, bool has_cut, double pairs) {
     const double nr = (double)n_ref, nq = (double)n_query, dp = direct::row_len(d);
-    if (!tc_ok) return nq * (dp + 2.0) <= 600000.0;
+    if (!tc_ok) return pairs / nr * (std::max(dp, 8.0) - 2.0) <= 300000.0;
     const double us = nq * (2.0 + 0.35 * dp) * 1e-3 + pairs * (0.25 + 0.14 * dp) * 1e-6;
     if (has_cut) return n_query <= seed::kMinQueries && us <= 380.0 + 10.0 * dp + 0.0006 * nr;
     if (n_query >= seed::kMinQueries && n_ref >= seed::kMinPoints) return us <= std::min(120.0 + 30.0 * dp, 560.0);

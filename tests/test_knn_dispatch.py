@@ -47,6 +47,15 @@ def test_more_queries_never_turn_a_search_back_to_direct(d, cut):
         assert set(kinds[:first]) <= {DIRECT} and set(kinds[first:]) <= {TC}
 
 
+@pytest.mark.parametrize('d,m,below,above', [(3, 48, 45000, 60000), (8, 64, 45000, 60000), (16, 48, 20000, 25000),
+                                             (26, 32, 11000, 13000), (32, 32, 9500, 11000)])
+def test_against_the_simt_screen_queries_count_by_their_refs(d, m, below, above):
+    """The same line for any number of refs; a set over itself has half the pairs, so twice the points."""
+    for n_ref in (20000, 100000, 434874):
+        assert path(n_ref, below, d, m) == DIRECT and path(n_ref, above, d, m) == SIMT
+    assert path(2 * below, 2 * below, d, m, cut=0) == DIRECT and path(2 * above, 2 * above, d, m, cut=0) == SIMT
+
+
 def test_fp64_and_other_shapes():
     assert path(434874, 434874, 3, cut=0, f64=True) == DIRECT and path(1000, 10, 3, 200, f64=True) == GENERIC
     assert path(100000, 50, 40) == DIRECT and path(100000, 50, 3, 200) == GENERIC
