@@ -142,7 +142,8 @@ uint64_t nngp_set_wait_limit_ns(uint64_t ns);
  * between k-means cells) cannot exclude; the lists are the same.
  * A search of other queries without a cut (predict: n_ref >= 8,192, n_query >= 16,384) seeds
  * every query from the refs' curve windows around it and, for d <= 24, prunes the same way.
- * NNGP_KNN_SEED_W=0 / NNGP_KNN_PRUNE=0 switch these off (testing).  The workspace covers them.
+ * NNGP_KNN_SEED_W=0 / NNGP_KNN_PRUNE=0 switch these off (testing).  The workspace covers them, with and
+ * without a cut, and a workspace for n_query queries serves any smaller number of them.
  * ------------------------------------------------------------------------------------- */
 size_t nngp_knn_workspace_size_f32(int64_t n_ref, int64_t n_query, int32_t d, int32_t num_nn);
 /* The kernel that a search takes: 0 tensor-core, 1 SIMT screen, 2 generic, 3 direct; -1 for an empty one.

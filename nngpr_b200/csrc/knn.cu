@@ -546,6 +546,15 @@ int tc_parts(int64_t n_ref, int64_t n_query, const tc::TcVariant &tv, bool has_c
     const int64_t slots = (int64_t)kNumSMsB200 * tv.ctas_per_sm, tiles = (n_ref + tc::kTcRefTile - 1) / tc::kTcRefTile;
     return (int)std::max<int64_t>(1, std::min<int64_t>({slots / groups, tiles / 16, 8}));
 }
+size_t parts_bytes(int64_t slots, const tc::TcVariant &tv) { return (size_t)slots * tv.rows_per_item * 32 * 8; }
+// Room that covers the partial lists of n_query queries and of any smaller number, which may be split into more
+// parts: a workspace for the largest batch serves the smaller ones.
+size_t parts_room(int64_t n_ref, int64_t n_query, const tc::TcVariant &tv) {
+    const int64_t groups = (n_query + tv.rows_per_item - 1) / tv.rows_per_item;
+    const int64_t slots = (int64_t)kNumSMsB200 * tv.ctas_per_sm, tiles = (n_ref + tc::kTcRefTile - 1) / tc::kTcRefTile;
+    const int64_t parts = std::min<int64_t>(tiles / 16, 8);
+    return parts < 2 ? 0 : parts_bytes(std::min(groups * parts, slots), tv);
+}
 
 // Lists of queries from the sorted lists of their parts (32 keys each: distance bits << 32 | index), one warp each.
 __global__ void __launch_bounds__(256) merge_parts_kernel(const unsigned long long *__restrict__ partial, int parts, int G,
@@ -599,9 +608,10 @@ struct KnnPlan {
     KnnPath path = KnnPath::Generic;
     int dp = 0;  // padded row length of the scaled arrays
     int64_t n_ref_pad = 0;
-    size_t off_parts = 0, parts_bytes = 0, off_ref = 0, off_q = 0, off_rec = 0, off_acc = 0, off_r2 = 0, off_ctr = 0,
-           off_ldist = 0, off_lidx = 0, off_seed = 0, off_seed_ws = 0, seed_ws_bytes = 0, off_tiles2 = 0,
-           off_prune_ws = 0, prune_ws_bytes = 0, total = 0;
+    size_t off_ref = 0, off_q = 0, off_rec = 0, off_acc = 0, off_r2 = 0, off_ctr = 0, off_ldist = 0, off_lidx = 0,
+           off_seed = 0, off_seed_ws = 0, seed_ws_bytes = 0, off_tiles2 = 0, off_prune_ws = 0, prune_ws_bytes = 0,
+           off_parts = 0;
+    size_t needed = 0, total = 0;  // bytes: without and with room for the partial lists of split groups
     ScreenVariant v{};
     tc::TcVariant tv{};
 };
@@ -640,13 +650,6 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same, KnnPa
         off = align_up(off + 16, 256);
         p.off_ctr = off;
         off = align_up(off + 16, 256);
-        if (p.path == KnnPath::Tc) {  // partial lists of an unpruned search's parts
-            const int64_t groups = (n_query + p.tv.rows_per_item - 1) / p.tv.rows_per_item;
-            const int parts = std::max(tc_parts(n_ref, n_query, p.tv, false), tc_parts(n_ref, n_query, p.tv, true));
-            p.parts_bytes = parts > 1 ? (size_t)groups * parts * p.tv.rows_per_item * 32 * 8 : 0;
-            p.off_parts = off;
-            off = align_up(off + p.parts_bytes, 256);
-        }
         // seeds and pruned lists: of the prefix search (same) or, for other queries, of the query
         // search (the size query plans with same = false and takes the larger of the two)
         const size_t seed_ws = p.path != KnnPath::Tc ? 0
@@ -677,7 +680,10 @@ KnnPlan make_plan(int64_t n_ref, int64_t n_query, int d, int m, bool same, KnnPa
         p.off_lidx = off;
         off = align_up(off + (size_t)n_query * m * sizeof(int32_t), 256);
     }
-    p.total = off + 1024;  // slack for base alignment
+    p.needed = off + 1024;  // slack for base alignment
+    p.off_parts = off;
+    if (p.path == KnnPath::Tc) off += parts_room(n_ref, n_query, p.tv);
+    p.total = off + 1024;
     return p;
 }
 
@@ -716,7 +722,7 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
     const KnnPath path = choose_path(n_ref, n_query, d, m, std::is_same<T, float>::value, has_cut != 0,
                                      pairs_of(n_ref, n_query, has_cut != 0, cut));
     const KnnPlan p = make_plan<T>(n_ref, n_query, d, m, same, path);
-    if (!ws || ws_bytes < p.total) return fail(NNGP_ERR_WORKSPACE, "knn: workspace missing or too small");
+    if (!ws || ws_bytes < p.needed) return fail(NNGP_ERR_WORKSPACE, "knn: workspace missing or too small");
     char *base = reinterpret_cast<char *>(align_up(reinterpret_cast<uintptr_t>(ws), 1024));
     T *refs = reinterpret_cast<T *>(base + p.off_ref);
     T *qsc = reinterpret_cast<T *>(base + p.off_q);
@@ -886,7 +892,8 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
                 const int64_t groups = (n_query + p.tv.rows_per_item - 1) / p.tv.rows_per_item;
                 tc::TcItems whole{};
                 whole.parts = tc_parts(n_ref, n_query, p.tv, has_cut != 0);
-                if (p.parts_bytes == 0) whole.parts = 1;
+                // (a workspace without room for them: unsplit, the same lists)
+                if (p.needed + parts_bytes(groups * whole.parts, p.tv) > ws_bytes) whole.parts = 1;
                 whole.partial = reinterpret_cast<unsigned long long *>(base + p.off_parts);
                 const float *seeds_rows = seeds_c ? seeds_c + row_lo : nullptr;
                 lst = launch(tiles, groups * whole.parts, none, none, no_sizes, whole, none, none, none, ctr, seeds_rows, cut, 0,
