@@ -316,6 +316,9 @@ nngp_status nngp_fma_probe(float *out, int64_t iters, int32_t blocks, void *stre
 /* FP64 FMA-rate probe (measurement only): blocks x 256 threads, 8 FMA chains of 8 x iters
  * steps each; out receives blocks x 256 doubles. */
 nngp_status nngp_fma_probe_f64(double *out, int64_t iters, int32_t blocks, void *stream);
+/* out[i] = e^x[i], x[i] <= 0, by the exponential that the FP64 local systems use (its error bound is
+ * stated and tested for it alone).  n <= 2^30. */
+nngp_status nngp_exp_neg_probe(const double *x, double *out, int64_t n, void *stream);
 
 /* Plain FP32 GPU form of the neighbour search: the comparator the optimised search is measured
  * against (no counterpart in the reference's plugin interface; it restates the structure of the

@@ -30,7 +30,7 @@ EXPORTED = (
     'nngp_plain_knn_f32', 'nngp_knn_reuse_prepare_f32', 'nngp_knn_reuse_rank_f32',
     'nngp_predict_full_workspace_size', 'nngp_predict_full_f64', 'nngp_sample_full_f64',
     'nngp_predict_cov_full_f64', 'nngp_theta_params', 'nngp_knn_f32_ls_device', 'nngp_knn_f64_ls_device',
-    'nngp_knn_path',
+    'nngp_knn_path', 'nngp_exp_neg_probe',
 )
 
 
@@ -93,6 +93,7 @@ _SIGS = {
     'nngp_predict_f64': ([_vp, _vp, _i64, _vp, _i64, _i32, _i32, _vp, _i32, _kp, _f64, _vp, _vp, _vp, _vp], ctypes.c_int),
     'nngp_fma_probe': ([_vp, _i64, _i32, _vp], ctypes.c_int),
     'nngp_fma_probe_f64': ([_vp, _i64, _i32, _vp], ctypes.c_int),
+    'nngp_exp_neg_probe': ([_vp, _vp, _i64, _vp], ctypes.c_int),
     'nngp_tc_layout_selftest': ([_vp, _vp, _i32, _vp, _vp, _vp], ctypes.c_int),
     'nngp_tc_layout_selftest_bf16': ([_vp, _vp, _i32, _vp, _vp, _vp], ctypes.c_int),
     'nngp_plain_knn_f32': ([_vp, _i64, _vp, _i64, _i32, _i32, _i32, _i64, _vp, _vp], ctypes.c_int),

@@ -1,8 +1,9 @@
 // FMA-rate probes (FP32 and FP64): the denominators of the roofline fractions of the kernels
 // here that are bound by a SIMT pipe.  Each thread runs 8 independent FMA chains of `iters`
 // steps (16 flops per step); the sum is written out so nothing is eliminated.  The caller times
-// the launch.
+// the launch.  And the exponential of the FP64 local systems on its own, for its error bound.
 #include "common.cuh"
+#include "local.cuh"
 
 namespace nngp {
 
@@ -32,7 +33,22 @@ __global__ void __launch_bounds__(256) fma_probe_f64_kernel(double *out, int64_t
     out[blockIdx.x * blockDim.x + threadIdx.x] = v0 + v1 + v2 + v3 + v4 + v5 + v6 + v7;
 }
 
+__global__ void __launch_bounds__(256) exp_neg_probe_kernel(const double *__restrict__ x, double *__restrict__ out, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = exp_neg(x[i]);
+}
+
 }  // namespace nngp
+
+extern "C" nngp_status nngp_exp_neg_probe(const double *x, double *out, int64_t n, void *stream) {
+    using namespace nngp;
+    set_error("");
+    if (!x || !out || n <= 0 || n > (int64_t)1 << 30)
+        return fail(NNGP_ERR_INVALID_ARGUMENT, "exp_neg_probe: bad arguments");
+    exp_neg_probe_kernel<<<(unsigned)((n + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(x, out, n);
+    NNGP_CUDA_TRY(cudaGetLastError());
+    return NNGP_OK;
+}
 
 extern "C" nngp_status nngp_fma_probe(float *out, int64_t iters, int32_t blocks, void *stream) {
     using namespace nngp;
