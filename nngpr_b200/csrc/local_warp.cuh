@@ -1,13 +1,13 @@
 // Local systems of up to 64 neighbours: 32 / LPP points per warp, LPP lanes per point (local.cu
 // has the mathematics).
 //
-// Lane `sub` of a point's group owns the rows c * LPP + sub, c = 0 .. C - 1 (C = M / LPP), of the
+// Lane `sub` of a point's group owns the rows c * LPP + sub, c = 0, 1 (two rows per lane), of the
 // neighbour block, row i up to column (c + 1) * LPP - 1: with the rows of one class c equally long,
 // every loop bound is a compile-time constant and only the diagonal LPP x LPP blocks hold
 // entries above the diagonal.  M is the neighbour count rounded up to 16, 32 or 64; rows past it and
 // missing neighbours are identity rows.
 //
-// LPP is M / 2: two rows per lane, one, two or four points per warp.  Why several
+// LPP is M / 2: one, two or four points per warp.  Why several
 // points per warp: with one row per lane a lane computes whole rows of a symmetric matrix, twice
 // the fill's and three times the factor's work, and the chain of each column (two shuffles, a
 // reciprocal square root, a trip through shared memory) is paid per point.  At M = 32 a warp issues 24
@@ -55,8 +55,8 @@ template <> struct Vec16<float> {
     __device__ static float4 make(const float *p) { return make_float4(p[0], p[1], p[2], p[3]); }
 };
 
-// Lanes per point of the systems of type TC (4- or 8-byte) with M rows
-template <typename TC> __host__ __device__ constexpr int lanes_per_point(int M) { return M / 2; }
+// Lanes per point of the systems with M rows: two rows per lane
+__host__ __device__ constexpr int lanes_per_point(int M) { return M / 2; }
 
 // Resident CTAs (of two warps) per SM the registers are budgeted for: FP32 and the 16-row systems 168
 // registers, 12 warps per SM; the 32- and 64-row FP64 ones are held to 8 and 5 warps by shared memory, so
@@ -97,18 +97,12 @@ struct PtLayout {
 struct WarpLayout {
     size_t g, total;
     template <bool F32, bool F64> __host__ __device__ static WarpLayout make(int M, int d, int n_theta, bool grad, bool keep_e, bool keep_x) {
+        const int groups = 32 / lanes_per_point(M);
         size_t b = 0;
-        int groups = 0;
-        if (F32) {
-            const int n = 32 / lanes_per_point<float>(M);
-            b = n * PtLayout::make<float>(M, d, grad, keep_e, keep_x).total;
-            groups = n;
-        }
+        if (F32) b = groups * PtLayout::make<float>(M, d, grad, keep_e, keep_x).total;
         if (F64) {
-            const int n = 32 / lanes_per_point<double>(M);
-            const size_t q = n * PtLayout::make<double>(M, d, grad, keep_e, keep_x).total;
+            const size_t q = groups * PtLayout::make<double>(M, d, grad, keep_e, keep_x).total;
             b = q > b ? q : b;
-            groups = n > groups ? n : groups;
         }
         WarpLayout w;
         w.g = (b + 15) / 16 * 16;
@@ -127,7 +121,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
                                              const int32_t *__restrict__ nbr, unsigned char *wsm, double *gacc,
                                              double &ll_acc, TIn *__restrict__ mean, TIn *__restrict__ var,
                                              int32_t *__restrict__ flags) {
-    constexpr int LPP = lanes_per_point<TC>(M), C = M / LPP;
+    constexpr int LPP = lanes_per_point(M), C = 2;  // C: rows per lane
     using V = Vec16<TC>;
     using VT = typename V::T;
     constexpr int EV = V::N;
@@ -156,20 +150,15 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
         for (int o = LPP / 2; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
         return v;
     };
-    auto rows_sum = [&](const TC (&w)[C]) -> TC {
-        if constexpr (C == 2) return lanes_sum(add_rn(w[0], w[1]));
-        else return lanes_sum(w[0]);
-    };
+    auto rows_sum = [&](const TC (&w)[C]) -> TC { return lanes_sum(add_rn(w[0], w[1])); };
     // f(dc, k0) for every 4 columns k0 .. k0 + 3 of the lower triangle: dc is the class of their rows'
     // diagonal block (a constant once inlined), the rows of the classes c >= dc reach them.  Loops,
     // not unrolled code: a kernel of 4,000 straight instructions waits for its instructions.
     auto for_columns = [&](auto &&f) {
 #pragma unroll 1
         for (int k0 = 0; k0 < LPP; k0 += 4) f(0, k0);
-        if constexpr (C > 1) {
 #pragma unroll 1
-            for (int k0 = LPP; k0 < 2 * LPP; k0 += 4) f(1, k0);
-        }
+        for (int k0 = LPP; k0 < 2 * LPP; k0 += 4) f(1, k0);
     };
     auto store4 = [&](TC *at, const TC (&w)[4]) {
 #pragma unroll
@@ -408,7 +397,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
         }
     };
     factor_block(0);
-    if constexpr (C > 1) factor_block(1);
+    factor_block(1);
     const TC s2 = kpp - ss;
     bool ok = true;
     if constexpr (std::is_same<TC, float>::value)
@@ -433,7 +422,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
             for (int u = 3; u >= 0; --u) {
                 const int k = k0 + u;
                 auto step = [&](TC(&b)[C]) {
-                    const TC bc = C == 1 || k0 < LPP ? b[0] : b[C - 1];
+                    const TC bc = k0 < LPP ? b[0] : b[1];
                     const TC bk = __shfl_sync(FULL, bc, k & (LPP - 1), LPP) * iv[u];
 #pragma unroll
                     for (int c = 0; c < C; ++c)
@@ -474,7 +463,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
             for (int c = 0; c < C; ++c) yv[c] = valid[c] ? (TC)y_ref[(int64_t)j[c] * a.ydim + o] : TC(0);
 #pragma unroll 4
             for (int k = 0; k < M; ++k) {
-                const TC yc = C == 1 || k < LPP ? yv[0] : yv[C - 1];
+                const TC yc = k < LPP ? yv[0] : yv[1];
                 const TC zk = __shfl_sync(FULL, yc, k & (LPP - 1), LPP) * idg[k];
 #pragma unroll
                 for (int c = 0; c < C; ++c)
@@ -663,7 +652,7 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_k
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using T1 = typename std::conditional<(M > 32), double, TIn>::type;  // the first attempt's precision
     constexpr bool F32 = std::is_same<T1, float>::value;
-    constexpr int LPP = lanes_per_point<T1>(M), GROUPS = 32 / LPP;
+    constexpr int LPP = lanes_per_point(M), GROUPS = 32 / LPP;
     const WarpLayout lay = WarpLayout::make<F32, !F32 || PRED>(M, a.d, a.n_theta, GRAD,
                                                               GRAD && !MATERN && M <= 32, GRAD && a.ard);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -685,19 +674,9 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_k
             if constexpr (!PRED) {
                 if (bad && sub == 0) atomicOr(a.redo_bits + (p >> 5), 1u << (p & 31));
             } else {
-                unsigned todo = __ballot_sync(0xffffffffu, bad && sub == 0);
-                constexpr int LPD = lanes_per_point<double>(M);
-                while (todo) {  // the marked groups' points, 32 / LPD at a time
-                    int src = -1;
-                    for (int g = 0; g < 32 / LPD; ++g) {
-                        const int b = todo ? __ffs(todo) - 1 : -1;
-                        if (todo) todo &= todo - 1;
-                        if (g == lane / LPD) src = b;
-                    }
-                    const int64_t pq = __shfl_sync(0xffffffffu, (long long)p, src < 0 ? 0 : src);
-                    solve_points<double, TIn, M, GRAD, PRED, MATERN>(a, src < 0 ? -1 : pq, lane, x_ref, y_ref, x_pt,
-                                                                     y_pt, nbr, wsm, gacc, ll_acc, mean, var, flags);
-                }
+                if (__any_sync(0xffffffffu, bad))
+                    solve_points<double, TIn, M, GRAD, PRED, MATERN>(a, bad ? p : -1, lane, x_ref, y_ref, x_pt, y_pt,
+                                                                     nbr, wsm, gacc, ll_acc, mean, var, flags);
             }
         }
     }
@@ -719,7 +698,7 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<double, M, false>)) local_re
                                                          const int32_t *__restrict__ nbr,
                                                          double *__restrict__ block_out, int32_t *__restrict__ flags) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int LPP = lanes_per_point<double>(M), GROUPS = 32 / LPP;
+    constexpr int LPP = lanes_per_point(M), GROUPS = 32 / LPP;
     const WarpLayout lay = WarpLayout::make<false, true>(M, a.d, a.n_theta, GRAD,
                                                         GRAD && !MATERN && M <= 32, GRAD && a.ard);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;

@@ -21,7 +21,7 @@ nngp_status launch_fit(const LocalArgs &a, bool grad, const TIn *x_ref, const TI
     auto fn = M == 16   ? pick(std::integral_constant<int, 16>{})
               : M == 32 ? pick(std::integral_constant<int, 32>{})
                         : pick(std::integral_constant<int, 64>{});
-    const int groups = 32 / lanes_per_point<TIn>(M);
+    const int groups = 32 / lanes_per_point(M);
     const bool keep_e = grad && rbf && M <= 32;
     const size_t bytes = (F32 && M <= 32 ? WarpLayout::make<true, false>(M, a.d, a.n_theta, grad, keep_e, grad && a.ard)
                                          : WarpLayout::make<false, true>(M, a.d, a.n_theta, grad, keep_e, grad && a.ard))
@@ -49,7 +49,7 @@ nngp_status launch_predict(const LocalArgs &a, const TIn *x_ref, const TIn *y_re
     auto fn = M == 16   ? pick(std::integral_constant<int, 16>{})
               : M == 32 ? pick(std::integral_constant<int, 32>{})
                         : pick(std::integral_constant<int, 64>{});
-    const int groups = 32 / lanes_per_point<TIn>(M);
+    const int groups = 32 / lanes_per_point(M);
     const size_t bytes = (F32 && M <= 32 ? WarpLayout::make<true, true>(M, a.d, 0, false, false, false)
                                          : WarpLayout::make<false, true>(M, a.d, 0, false, false, false))
                              .total;
