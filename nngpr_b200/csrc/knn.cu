@@ -557,8 +557,8 @@ size_t parts_room(int64_t n_ref, int64_t n_query, const tc::TcVariant &tv) {
 }
 
 // Lists of queries from the sorted lists of their parts (32 keys each: distance bits << 32 | index), one warp each.
-__global__ void __launch_bounds__(256) merge_parts_kernel(const unsigned long long *__restrict__ partial, int parts, int G,
-                                                          int64_t n_query, int m, int32_t *__restrict__ out) {
+__global__ void __launch_bounds__(256) merge_parts_kernel(const unsigned long long *__restrict__ partial, int parts,
+                                                          int G, int64_t n_query, int m, int32_t *__restrict__ out) {
     const int lane = threadIdx.x & 31;
     const int64_t q = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (q >= n_query) return;
@@ -896,11 +896,11 @@ nngp_status knn_impl(const T *ref, int64_t n_ref, const T *query, int64_t n_quer
                 if (p.needed + parts_bytes(groups * whole.parts, p.tv) > ws_bytes) whole.parts = 1;
                 whole.partial = reinterpret_cast<unsigned long long *>(base + p.off_parts);
                 const float *seeds_rows = seeds_c ? seeds_c + row_lo : nullptr;
-                lst = launch(tiles, groups * whole.parts, none, none, no_sizes, whole, none, none, none, ctr, seeds_rows, cut, 0,
-                             q_c);
+                lst = launch(tiles, groups * whole.parts, none, none, no_sizes, whole, none, none, none, ctr, seeds_rows,
+                             cut, 0, q_c);
                 if (lst == NNGP_OK && whole.parts > 1) {
-                    merge_parts_kernel<<<(int)((n_query + 7) / 8), 256, 0, stream>>>(whole.partial, whole.parts, G, n_query, m,
-                                                                                     out);
+                    merge_parts_kernel<<<(int)((n_query + 7) / 8), 256, 0, stream>>>(whole.partial, whole.parts, G,
+                                                                                     n_query, m, out);
                     NNGP_CUDA_TRY(cudaGetLastError());
                 }
             }

@@ -12,9 +12,10 @@
 //
 // In many dimensions boxes exclude little; from 9 features on the rows and refs are also kept in k-means
 // cells, and a tile is dropped as well when the slab between its cell and the group's is wider than the
-// bound allows (knn_cells.cu).  Inside a cell the rows are ordered by their seed first (16 steps of a
-// ninth of a factor of two in the squared distance, then the curve): a group reaches as far as its
-// largest seed, and the few rows in a cluster's tails would make every group reach far.  At d = 16, n = 1M (mixture of 64):
+// bound allows (knn_cells.cu).  Inside a cell the rows are ordered by their seed first (16 steps of a factor of
+// 2^(40 / 256) = 1.11 in the squared distance, then the curve): a group reaches as far as its
+// largest seed, and the few rows in a cluster's tails would make every group reach far.  At d = 16, n = 1M
+// (mixture of 64):
 // 3,282 listed tiles of 7,813 per group with boxes, 834 with cells, 443 with rows ordered by seed; search 68.5 ->
 // 38.9 -> 33.8 ms (32.2 with tile records written 16 bytes at a time).
 //
@@ -77,6 +78,10 @@ __device__ __forceinline__ int band_of(int64_t i, int64_t n, int shift) {
     while (b < shift && (i << (b + 1)) < n) ++b;  // i < n / 2^(b + 1)
     return b;
 }
+
+// Rows [0, early_rows(n, d)) = [0, n / 8), or [0, n / 64) where cells are used, always take the index-order
+// search: their prefixes are short, and the boxes of the sparse index classes they may use are large.
+int64_t early_rows(int64_t n, int d) { return n >> (cells::count(n, d) > 0 ? kEarlyShiftCells : kEarlyShift); }
 
 // log2 of a finite non-negative seed in units of 1/256, clamped below (zero seeds: duplicates)
 __device__ __forceinline__ long long log2q(float tau) {
@@ -172,7 +177,8 @@ __global__ void __launch_bounds__(kThreads) band_stats_kernel(int64_t n, int shi
 
 // Sort keys of the rows [row_lo, row_hi): pruned rows (band, cell, curve position), the others and the
 // rows outside the range (tag | index).  Counts of pruned rows per band and of the index-order rows.
-__global__ void __launch_bounds__(kThreads) classify_kernel(int64_t n, int shift, int by_seed, int64_t early, int64_t row_lo, int64_t row_hi,
+__global__ void __launch_bounds__(kThreads) classify_kernel(int64_t n, int shift, int by_seed, int64_t early,
+                                                            int64_t row_lo, int64_t row_hi,
                                                             const float *__restrict__ seeds,
                                                             const int32_t *__restrict__ pos0,
                                                             const uint8_t *__restrict__ cell,
@@ -517,7 +523,8 @@ __global__ void __launch_bounds__(kThreads) count_kernel(Boxes b, const DevSizes
                         const int tt = base + lane;
                         bool need = false, ov = false;
                         if (tt < nt && smin[tt] < q.lim)  // else every ref of the tile comes after every row
-                            tile_test(b, q, [&](int f) { return slo[f][tt]; }, [&](int f) { return shi[f][tt]; }, need, ov);
+                            tile_test(b, q, [&](int f) { return slo[f][tt]; }, [&](int f) { return shi[f][tt]; },
+                                      need, ov);
                         put((t0 + base) / 32, need, ov);
                     }
                 }
@@ -693,17 +700,17 @@ __global__ void uniform_groups_kernel(int64_t n_rows, int G, int64_t n_groups, i
 
 struct Layout {
     int64_t n_tiles, max_groups;
-    size_t tlo, thi, tmin, stats, keys_a, keys_b, vals_a, vals_b, rvals_a, rvals_b, headpos, seg_start, gh, gid, row_off, sizes, glo,
-        ghi, gtau, glim, counts, offsets, masks, list, cub, cub_bytes, cells_ws, cells_bytes, thome, ghome, treach, greach,
-        total;
+    size_t tlo, thi, tmin, stats, keys_a, keys_b, vals_a, vals_b, rvals_a, rvals_b, headpos, seg_start, gh, gid, row_off,
+        sizes, glo, ghi, gtau, glim, counts, offsets, masks, list, cub, cub_bytes, cells_ws, cells_bytes, thome, ghome,
+        treach, greach, total;
     int n_cells;  // 0: none
     int64_t maxg[2], max_items[2];
     size_t cnt[2], cbase[2], K[2], kbase[2], S[2], sbase[2], igroup[2], it0[2], it1[2], islot[2], okey_a[2], okey_b[2],
         oval_a[2], oval_b[2], partial[2];
 };
 
-// Groups: segments per band <= (pruned rows of the band) / 256 or 1, or K cells (at most n / 4,096, 32 from
-// 65,536 points on: kBands K <= n / 256), groups per segment <= rows / G + 1, so
+// Groups: segments per band <= (pruned rows of the band) / 256 or 1, or K cells (32 from cells::kMinPoints = 131,072
+// points on, then at most n / 4,096: kBands K <= n / 256), groups per segment <= rows / G + 1, so
 // max_groups = n / G + n / 256 + 2 kBands bounds the count.
 Layout layout(int64_t n, int d, int G) {
     Layout L{};
@@ -720,8 +727,8 @@ Layout layout(int64_t n, int d, int G) {
     L.thi = take((size_t)L.n_tiles * d * 4);
     L.tmin = take((size_t)L.n_tiles * 4);
     L.stats = take(kStats * 8);
-    L.keys_a = take((size_t)n * 8);
-    L.keys_b = take((size_t)n * 8);
+    L.keys_a = take((size_t)n * 4);
+    L.keys_b = take((size_t)n * 4);
     L.vals_a = take((size_t)n * 4);
     L.vals_b = take((size_t)n * 4);
     L.rvals_a = take((size_t)n * 4);
@@ -872,8 +879,6 @@ Layout layout_query(int64_t n_ref, int64_t n_query, int d, int G) {
 
 }  // namespace
 
-int64_t early_rows(int64_t n, int d) { return n >> (cells::count(n, d) > 0 ? kEarlyShiftCells : kEarlyShift); }
-
 bool enabled() {
     const char *env = std::getenv("NNGP_KNN_PRUNE");
     return !(env && env[0] == '0');
@@ -947,7 +952,8 @@ nngp_status build(const float *xs, int64_t n, int64_t row_lo, int64_t row_hi, in
     band_stats_kernel<<<grid_of(n - early), kThreads, 0, stream>>>(n, shift, std::max(early, row_lo), row_hi, seeds, sum,
                                                                    cnt);
     NNGP_CUDA_TRY(cudaGetLastError());
-    classify_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, shift, L.n_cells > 0 ? 1 : 0, early, row_lo, row_hi, seeds, pos0, cl.of, sum, cnt,
+    classify_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, shift, L.n_cells > 0 ? 1 : 0, early, row_lo, row_hi, seeds,
+                                                         pos0, cl.of, sum, cnt,
                                                          static_cast<uint32_t *>(at(L.keys_a)),
                                                          static_cast<int32_t *>(at(L.vals_a)), pcnt, icnt, isum);
     NNGP_CUDA_TRY(cudaGetLastError());
@@ -964,8 +970,8 @@ nngp_status build(const float *xs, int64_t n, int64_t row_lo, int64_t row_hi, in
     int32_t *rows = dv.Current();
 
     // groups: segments of one band and one octree cell, cut every G rows
-    segment_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, dk.Current(), L.n_cells > 0 ? 1 : 0, rows, pos0, keys0, pcnt, d, bits,
-                                                        seed::key_drop(d), headpos);
+    segment_kernel<<<grid_of(n), kThreads, 0, stream>>>(n, dk.Current(), L.n_cells > 0 ? 1 : 0, rows, pos0, keys0, pcnt,
+                                                        d, bits, seed::key_drop(d), headpos);
     NNGP_CUDA_TRY(cudaGetLastError());
     need = 0;
     NNGP_CUDA_TRY(cub::DeviceScan::InclusiveScan(nullptr, need, headpos, seg_start, cub::Max(), (int)n, stream));

@@ -17,10 +17,6 @@ constexpr int64_t kMaxPoints = 2000000;  // the tile lists' worst-case bound (gr
 constexpr int kMaxDim = 24;            // every shape of the tensor-core search (d <= 24)
 constexpr int kTileRefs = 128;         // refs per tile (the tensor-core search's ref tile)
 
-// Rows [0, early_rows(n, d)) = [0, n / 8), or [0, n / 64) where cells are used, always take the index-order
-// search: their prefixes are short, and the boxes of the sparse index classes they may use are large.
-int64_t early_rows(int64_t n, int d);
-
 // NNGP_KNN_PRUNE=0 turns pruning off (seeded index-order search only).
 bool enabled();
 
@@ -60,7 +56,7 @@ size_t workspace(int64_t n, int d, int rows_per_group);
 
 // Plans the prefix search of n scaled points xs (row stride dp, d <= kMaxDim features) over
 // itself, from the seeds and the curve order of knn_seed.cu (order0, pos0, keys0 with
-// bits_per_dim bits per dimension).  Rows below early_rows(n, d) and rows whose seed is more than
+// bits_per_dim bits per dimension).  Rows below n / 8 (n / 64 with cells) and rows whose seed is more than
 // 16 times the geometric mean of their band's seeds go to the index-order launch; the others
 // are sorted by (band = floor(log2(n / i)), curve position) and cut into groups of at most
 // rows_per_group rows that never straddle a band or an octree cell of the curve (a cell level
@@ -70,8 +66,8 @@ size_t workspace(int64_t n, int d, int rows_per_group);
 // the search's tiles in that order).  A ref tile is listed for a group unless (a) every point in it
 // has an index >= every row of the group, or (b) the distance between the two bounding boxes,
 // shrunk by the FP32 rounding bound, exceeds the largest seed of the group, or (c) the slab between their
-// cells does; tiles whose box meets the group's come first.  No rule excludes a neighbour of any row, so the search returns
-// the same lists.  No host synchronisation: sizes stay on the device.
+// cells does; tiles whose box meets the group's come first.  No rule excludes a neighbour of any row, so the
+// search returns the same lists.  No host synchronisation: sizes stay on the device.
 // Only the rows [row_lo, row_hi) are planned (a row shard of the multi-GPU fit step; [0, n) for
 // the whole search); the refs are all n points.
 nngp_status build(const float *xs, int64_t n, int64_t row_lo, int64_t row_hi, int d, int dp, int rows_per_group,
