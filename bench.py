@@ -529,14 +529,15 @@ def local_flops_per_point(m, d, n_theta):
 
 
 def our_launches_per_step(n, d, m):
-    """Kernels of this library one fit step launches (CUB's sort and scan kernels not counted):
-    scale, centre sums and tile build; per seed level (the prefixes n, n/8, ... of at least
-    8,192 points) bounds, Morton keys, places and coordinates, cross positions and the seed kernel; the pruned search's planning (21, the index-order fallback's two
-    included), a second tile build, two search
-    launches and two merges, or one search launch; the local systems and the final sum.  Below the
-    seeded sizes the direct search: scale and one launch."""
+    """Kernels of this library one fit step launches (CUB's sort and scan kernels not counted): of a
+    set that the library searches directly (nngp_knn_path), scale and one launch; else scale, centre
+    sums and tile build; per seed level (the prefixes n, n/8, ... of at least 8,192 points) bounds,
+    Morton keys, places and coordinates, cross positions and the seed kernel; the pruned search's
+    planning (21, the index-order fallback's two included), a second tile build, two search launches
+    and two merges, or one search launch; the local systems and the final sum."""
+    from nngpr_b200 import _lib
     seeded = n >= 8192
-    if not seeded:
+    if _lib.lib().nngp_knn_path(n, n, d, m, 1, 0, 0) == 3:
         return 2 + 2
     levels = 0
     p_ = n

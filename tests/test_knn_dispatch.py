@@ -75,3 +75,10 @@ def test_the_workspace_serves_the_search_with_and_without_a_cut(monkeypatch, f64
         monkeypatch.setenv('NNGP_KNN_KERNEL', ('tc', 'simt', 'generic', 'direct')[k])
         assert auto >= size(n_ref, n_query, d, m)
         monkeypatch.delenv('NNGP_KNN_KERNEL')
+
+
+def test_the_bench_counts_the_launches_of_the_search_it_runs():
+    import bench
+    for n, d in ((2000, 3), (8192, 16), (16384, 16)):
+        assert path(n, n, d, cut=0) == DIRECT and bench.our_launches_per_step(n, d, 32) == 4
+    assert bench.our_launches_per_step(16385, 16, 32) > 4
