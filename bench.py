@@ -528,17 +528,19 @@ def local_flops_per_point(m, d, n_theta):
     return 2.0 * k ** 3 / 3.0 + entries * (3 * d + 4) + 4.0 * entries * n_theta + 4.0 * k * k
 
 
-def our_launches_per_step(n, d, m):
+def our_launches_per_step(n, d, m, f32_systems=False):
     """Kernels of this library one fit step launches (CUB's sort and scan kernels not counted): of a
     set that the library searches directly (nngp_knn_path), scale and one launch; else scale, centre
     sums and tile build; per seed level (the prefixes n, n/8, ... of at least 8,192 points) bounds,
     Morton keys, places and coordinates, cross positions and the seed kernel; the pruned search's
     planning (21, the index-order fallback's two included), a second tile build, two search launches
-    and two merges, or one search launch; the local systems and the final sum."""
+    and two merges, or one search launch; the local systems (with FP32 ones the pass that re-solves
+    in FP64) and the final sum."""
     from nngpr_b200 import _lib
     seeded = n >= 8192
+    systems = 3 if f32_systems and m <= 32 else 2
     if _lib.lib().nngp_knn_path(n, n, d, m, 1, 0, 0) == 3:
-        return 2 + 2
+        return 2 + systems
     levels = 0
     p_ = n
     while seeded and p_ >= 8192:
@@ -549,7 +551,7 @@ def our_launches_per_step(n, d, m):
     search = (21 + 1 + 2 + 2) if pruned else 1
     if pruned and d >= 9 and n >= 131072:  # cells: k-means steps, directions, assignment, two reaches
         search += 10
-    return 3 + 5 * levels + search + 2
+    return 3 + 5 * levels + search + systems
 
 
 def run_plain(args, torch, x32, y64, xq32, p, flags, flush, lml_ours):
@@ -992,7 +994,9 @@ def run_ours(args):
         bf16_ops = D >= 12  # the search's operand type: BF16 x3 split from d = 12, TF32 split below
         kmma = 16 if bf16_ops else 8
         kp = (3 * (D + 1) + kmma - 1) // kmma * kmma  # split width of the tensor-core operands
-        issued = 2.0 * kp * pairs / (knn_avg_ms * 1e-3) / 1e12
+        # MMAs issued: 2 K' flops per pair, where every pair is screened (a pruned search's tile lists stay
+        # on the device)
+        issued = None if search_is_pruned(n, D) else 2.0 * kp * pairs / (knn_avg_ms * 1e-3) / 1e12
         local_avg_ms = float(np.mean([a - b for a, b in zip(step_ms, knn_ms)]))
         screen = 'BF16x3-split (kind::f16)' if bf16_ops else 'TF32-split (kind::tf32)'
         search = {'kernel': f'knn_tc_kernel<{D}> (prefix search: tcgen05 {screen} screen, exact FP32 rescoring; '
@@ -1015,7 +1019,8 @@ def run_ours(args):
             # the step's other kernel: the FP32 local systems (and the FP64 re-solve of marked points)
             lach = local_flops_per_point(M, D, p.n_theta) * (r1 - r0) / (local_avg_ms * 1e-3) / 1e12
             roof = {'bound': 'tensor', 'achieved': achieved, 'peak': tpk, 'unit': 'TFLOP/s', 'frac': achieved / tpk,
-                    'peak_source': tsrc, 'issued_mma_tflops': issued, 'issued_frac': issued / tpk,
+                    'peak_source': tsrc, 'issued_mma_tflops': issued,
+                    'issued_frac': None if issued is None else issued / tpk,
                     'fp32_fma_equivalent': {'peak': peak, 'frac': achieved / peak,
                                             'peak_source': 'FP32 FMA probe measured in this run'},
                     'local_systems': {'kernel': 'local_warp_kernel<float, grad> + local_redo_kernel',
@@ -1041,7 +1046,7 @@ def run_ours(args):
                 roof, traffic=read_profile_traffic(),
                 kernel=f'knn_tc_kernel<{D}> (prefix search: tcgen05 {screen} screen, exact FP32 rescoring)',
                 work='2*d flops per (query, ref) pair, n(n-1)/2 pairs, whichever pipe computes them; '
-                     'issued_mma = 2*K\' per pair with the split width K\'',
+                     'issued_mma = 2*K\' per pair with the split width K\', null for a pruned search',
                 pruned=search_is_pruned(n, D),
                 pruned_note='when pruned, the search screens only the pairs its tile lists keep, so achieved (and '
                             'frac) is the brute-force rate of the problem and can exceed the pipe\'s peak',
@@ -1054,7 +1059,7 @@ def run_ours(args):
             'serving': serving,
             'predict': None if pred_ms is None else {'value': N_PRED / (pred_ms * 1e-3), 'unit': 'points/s',
                                                      'ms': pred_ms, 'n_query': N_PRED},
-            'gpu_launches': args.steps * our_launches_per_step(n, D, M),  # row shards take the same path
+            'gpu_launches': args.steps * our_launches_per_step(n, D, M, LOCAL == 'f32'),  # shards alike
             'gpu_launches_note': 'kernels of libnngp_b200.so per step (see our_launches_per_step); CUB sort and '
                                  'scan kernels the planning launches are not counted',
             'clocks': clocks.summary(),
