@@ -12,11 +12,14 @@ namespace nngp {
 namespace cells {
 
 constexpr int kMaxCells = 128;
-// Cells are used from this many features and points on.  With fewer features boxes along the curve do as
-// well and cells cost partly filled groups (n = 434,874, with against without: uniform d = 5 12.9 / 10.8 ms, d = 6
-// 17.0 / 16.9, d = 8 26.8 / 26.4, d = 8 ARD 18.3 / 19.2); with fewer points the groups of a cell are too small
-// (mixture d = 10, n = 70,000 4.2 / 3.3 ms; n = 140,000 5.8 / 6.6; d = 16, n = 131,072 5.6 / 6.4, n = 200,000 7.1 /
-// 10.7; d = 24, n = 300,000 9.2 / 17.5).
+// Cells are used from this many features and points on.  With fewer features boxes along the curve do as well and
+// cells cost partly filled groups (n = 434,874, with against without: uniform d = 5 12.9 / 10.8 ms, d = 6 17.0 / 16.9,
+// d = 8 26.8 / 26.4, d = 8 ARD 18.3 / 19.2); with fewer points the groups of a cell are too small (mixture d = 10,
+// n = 70,000 4.2 / 3.3 ms; n = 140,000 5.8 / 6.6; d = 16, n = 131,072 5.6 / 6.4, n = 200,000 7.1 / 10.7; d = 24, n =
+// 300,000 9.2 / 17.5).  Points that are not clustered pay for the planning and gain little: uniform and normal, d = 9
+// to 24, with against without 3 % slower at n = 140,000 (d = 9 4.62 / 4.49 ms), 1 to 2 % at 434,874 and 1 % at 1M;
+// points near a 4-dimensional surface 4.67 / 4.17 ms at d = 9, n = 140,000, 30.1 / 35.7 at d = 16, n = 1M, 37.6 / 51.2
+// at d = 24, n = 1M.
 constexpr int kMinDim = 9;
 constexpr int64_t kMinPoints = 131072;
 

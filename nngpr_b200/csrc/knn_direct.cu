@@ -27,7 +27,7 @@
 //   3. kept refs within the bound go to a list in shared memory, normally m plus a few.  A list that is long
 //      (repeated points) is bounded again by its own m-th entry, in (distance, index) order, which ends the
 //      ties: a thread keeps its lowest indices.  A thread whose K-th kept ref lies before the
-//      bound may have dropped some that do, and goes through its refs again, for all queries of the CTA at once;
+//      bound may have dropped some that do: its refs are gone through again, spread over its warp;
 //   4. each listed ref's rank (entries before it in (distance, index) order) is its place.
 // A list that overflows in step 3 (near refs in few threads all the same) is bounded by its m-th entry as well and
 // filled again, every time with at least kCap - m refs fewer.
