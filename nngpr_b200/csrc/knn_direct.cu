@@ -9,15 +9,15 @@
 // 20,000 points over themselves d = 3 11,651 -> 564 us, d = 20 46.6 -> 1.6 ms.  The bound is the
 // FP32 (FP64) issue of the distances: about 0.8 ps a pair at d <= 4, 1.4 at 8, 3.0 at 20 in FP32.
 // Points on a grid and repeated points (with ref j in thread j mod 256, lists bounded by the minima alone and
-// ties bisected over all refs -> now; 1,000 queries, FP32): 256 x 64 grid 763 -> 46 us, 512 x 64 1,482 -> 67,
-// 256 x 1,024 12,114 -> 391, half of 100,000 points in 20 places 3,830 -> 187; 16,384 random points 48 -> 50.
+// ties bisected over all refs -> now; 1,000 queries, FP32): 256 x 64 grid 763 -> 46 us, 512 x 64 1,482 -> 65,
+// 256 x 1,024 12,114 -> 394, half of 100,000 points in 20 places 3,830 -> 198; 16,384 random points 48 -> 52.
 //
 // What it is for: searches that are short in queries (a prediction of a few hundred points, a small
 // model's fit step), where the other kernels give one thread or one TMEM lane to a query and
 // leave most of the chip idle, and the FP64 search, which has no screen.  Nothing of size
 // n_query x n_ref is stored; the work is the exact distances (3 d operations a pair) plus one
 // compare, and every ref is read once per CTA for its Q queries:
-//   1. each of the 256 threads takes one ref of every block of 256 and keeps its K = 3 nearest per query in
+//   1. each of the 256 threads takes one ref of every block of 256 and keeps its K = 3 or 4 nearest per query in
 //      registers.  Which one turns from block to block (ref_of): with ref j in thread j mod 256, points on a
 //      grid whose rows are 256 long, or any period that divides 256, put a whole column of near refs into one
 //      thread, and the bound of step 2 reached sixteen grid steps instead of three;
@@ -41,8 +41,12 @@ namespace direct {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kKeep = 3;
-constexpr int kCap = kKeep * kThreads;  // every thread's kept refs
+// Refs that a thread keeps per query.  Some thread has three of a query's 32 near ones in about one query of ten, and
+// its refs are gone through again; four in one of 300.  With one query per CTA the fourth is free (256 queries of
+// 16,599, d = 18, 56.9 -> 54.5 us; 1,000 of 8,000, d = 8, 35.3 -> 31.9); with four it costs registers and
+// shared memory (16,384 points over themselves, d = 3, 197 -> 237 us).
+template <int Q> constexpr int kKeep = Q == 1 ? 4 : 3;
+template <int Q> constexpr int kCap = kKeep<Q> * kThreads;  // every thread's kept refs
 constexpr int kLong = kThreads;         // a longer list is bounded by its own m-th entry first
 constexpr uint32_t kTol = 1u << 12;
 constexpr uint32_t kNone = 0xFFFFFFFFu;  // no finite distance
@@ -66,7 +70,7 @@ __device__ __forceinline__ double up_to(uint32_t h, double) {
 // Which ref of block k (refs 256 k .. 256 k + 255) a thread has: tid ^ ref_of(k).  The low 8 bits are a hash of k, so
 // that refs whose indices differ by a multiple of 256 share a thread for about one pair of blocks in 256.  A thread
 // that has G blocks in flight takes one hash for them, 64 refs apart (one query per CTA, 1,000 queries of 434,874
-// refs, d = 3: 660 us with a hash for each block, 597 so, 533 without any).
+// refs, d = 3: 660 us with a hash for each block, 593 so, 533 without any).
 __device__ __forceinline__ uint32_t turn(int g) {
     uint32_t h = (uint32_t)g * 0x9E3779B1u;
     h = (h ^ (h >> 15)) * 0x85EBCA6Bu;
@@ -184,8 +188,8 @@ __device__ __forceinline__ void mth_entry(const T *cd, const int32_t *cj, int c,
 // DP: row length when it is known at compile time (0: any).
 template <typename T, int DP, int Q> struct Shared {
     alignas(32) T q[Q][DP > 0 ? DP : 256];
-    alignas(16) T d[Q][kCap];
-    int32_t j[Q][kCap];
+    alignas(16) T d[Q][kCap<Q>];
+    int32_t j[Q][kCap<Q>];
     int count[Q];  // refs pushed; the first kCap of them are listed
     T bd[Q];
     int bj[Q];
@@ -194,29 +198,30 @@ template <typename T, int DP, int Q> struct Shared {
     __device__ __forceinline__ bool within(int i, T dist, int ref) const { return !before(bd[i], bj[i], dist, ref); }
     __device__ __forceinline__ void push(int i, T dist, int ref) {
         const int at = atomicAdd(&count[i], 1);
-        if (at < kCap) {
+        if (at < kCap<Q>) {
             d[i][at] = dist;
             j[i][at] = ref;
         }
     }
 };
 // A thread's nearest refs of a query, in (distance, index) order; j < 0: none.
-template <typename T> struct Kept {
-    T d[kKeep];
-    int j[kKeep];
+template <typename T, int K> struct Kept {
+    T d[K];
+    int j[K];
     // may the thread have dropped refs that lie before (bd, bj)?
     __device__ __forceinline__ bool dropped(T bd, int bj) const {
-        return j[kKeep - 1] >= 0 && before(d[kKeep - 1], j[kKeep - 1], bd, bj);
+        return j[K - 1] >= 0 && before(d[K - 1], j[K - 1], bd, bj);
     }
 };
 
 // Step 3 for the lists that are long, or whose threads may have dropped refs (todo: a bit per query, the same in
 // every thread): a call of its own, so that it holds no register of the distance loop.
 template <int G, typename T, int DP, int Q>
-__device__ __noinline__ void refine(Shared<T, DP, Q> &sh, const Kept<T> *kept, const int *lim, unsigned todo,
+__device__ __noinline__ void refine(Shared<T, DP, Q> &sh, const Kept<T, kKeep<Q>> *kept, const int *lim, unsigned todo,
                                     const T *__restrict__ refs, int n_ref, int blocks, int dp_any, int m) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     constexpr int R = 2;  // refs of a lane in flight
+    constexpr int K = kKeep<Q>;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dp = DP > 0 ? DP : dp_any;
     while (todo) {
@@ -227,7 +232,7 @@ __device__ __noinline__ void refine(Shared<T, DP, Q> &sh, const Kept<T> *kept, c
             if (warp < Q && ((again >> warp) & 1u)) {
                 T bd;
                 int bj;
-                mth_entry(sh.d[warp], sh.j[warp], min(sh.count[warp], kCap), m, lane, bd, bj);
+                mth_entry(sh.d[warp], sh.j[warp], min(sh.count[warp], kCap<Q>), m, lane, bd, bj);
                 __syncwarp();
                 if (lane == 0) {
                     sh.bd[warp] = bd;
@@ -237,7 +242,7 @@ __device__ __noinline__ void refine(Shared<T, DP, Q> &sh, const Kept<T> *kept, c
             }
             __syncthreads();
             for (int q = 0; q < Q; ++q)
-                for (int k = 0; ((again >> q) & 1u) && k < kKeep; ++k) {
+                for (int k = 0; ((again >> q) & 1u) && k < K; ++k) {
                     const T d = kept[q].d[k];
                     const int j = kept[q].j[k];
                     if (j >= 0 && sh.within(q, d, j)) sh.push(q, d, j);
@@ -254,8 +259,8 @@ __device__ __noinline__ void refine(Shared<T, DP, Q> &sh, const Kept<T> *kept, c
             int lj[Q];
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                ld[q] = __shfl_sync(FULL, kept[q].d[kKeep - 1], src);
-                lj[q] = __shfl_sync(FULL, kept[q].j[kKeep - 1], src);
+                ld[q] = __shfl_sync(FULL, kept[q].d[K - 1], src);
+                lj[q] = __shfl_sync(FULL, kept[q].j[K - 1], src);
             }
             for (int k0 = lane; k0 < blocks; k0 += 32 * R) {
                 int jr[R];
@@ -285,7 +290,7 @@ __device__ __noinline__ void refine(Shared<T, DP, Q> &sh, const Kept<T> *kept, c
         }
         __syncthreads();
         for (int q = 0; q < Q; ++q)
-            if (((todo >> q) & 1u) && sh.count[q] <= kCap) todo &= ~(1u << q);
+            if (((todo >> q) & 1u) && sh.count[q] <= kCap<Q>) todo &= ~(1u << q);
     }
 }
 
@@ -299,6 +304,7 @@ template <typename T, int DP, int Q, int R>
 __global__ void __launch_bounds__(kThreads, (kMinCtas<T, DP, Q>))
     knn_direct_kernel(const T *__restrict__ refs, const T *__restrict__ qs, int64_t n_query, int64_t n_ref, int dp_any,
                       int has_cut, int64_t cut, int m, int32_t *__restrict__ out) {
+    constexpr int K = kKeep<Q>;
     __shared__ Shared<T, DP, Q> sh;
     uint32_t(*smin)[kThreads] = reinterpret_cast<uint32_t(*)[kThreads]>(&sh.d[0][0]);  // in the lists' place
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -324,11 +330,11 @@ __global__ void __launch_bounds__(kThreads, (kMinCtas<T, DP, Q>))
     const int lim_max = limit_of(q0 + nq - 1);  // limits ascend
     __syncthreads();
 
-    Kept<T> kept[Q];
+    Kept<T, K> kept[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q)
 #pragma unroll
-        for (int k = 0; k < kKeep; ++k) {
+        for (int k = 0; k < K; ++k) {
             kept[q].d[k] = pos_inf<T>();
             kept[q].j[k] = -1;
         }
@@ -366,15 +372,28 @@ __global__ void __launch_bounds__(kThreads, (kMinCtas<T, DP, Q>))
             for (int r = 0; r < R; ++r) {
                 const int j = jr[r];
                 const T d = s[q][r];
-                if (d < kept[q].d[kKeep - 1] && j < lim[q]) {  // NaN and +inf never; ties keep the lower index
-                    Kept<T> &kp = kept[q];
-                    const bool b0 = d < kp.d[0], b1 = d < kp.d[1];
-                    kp.d[2] = b1 ? kp.d[1] : d;
-                    kp.j[2] = b1 ? kp.j[1] : j;
-                    kp.d[1] = b0 ? kp.d[0] : (b1 ? d : kp.d[1]);
-                    kp.j[1] = b0 ? kp.j[0] : (b1 ? j : kp.j[1]);
-                    kp.d[0] = b0 ? d : kp.d[0];
-                    kp.j[0] = b0 ? j : kp.j[0];
+                if (d < kept[q].d[K - 1] && j < lim[q]) {  // NaN and +inf never; ties keep the lower index
+                    Kept<T, K> &kp = kept[q];
+                    if constexpr (K == 3) {  // spelled out: the loops below cost the four-query form 1 to 5 %
+                        const bool b0 = d < kp.d[0], b1 = d < kp.d[1];
+                        kp.d[2] = b1 ? kp.d[1] : d;
+                        kp.j[2] = b1 ? kp.j[1] : j;
+                        kp.d[1] = b0 ? kp.d[0] : (b1 ? d : kp.d[1]);
+                        kp.j[1] = b0 ? kp.j[0] : (b1 ? j : kp.j[1]);
+                        kp.d[0] = b0 ? d : kp.d[0];
+                        kp.j[0] = b0 ? j : kp.j[0];
+                    } else {
+                        bool b[K];  // d lies before the k-th kept
+#pragma unroll
+                        for (int k = 0; k < K; ++k) b[k] = k == K - 1 || d < kp.d[k];
+#pragma unroll
+                        for (int k = K - 1; k > 0; --k) {
+                            kp.d[k] = b[k - 1] ? kp.d[k - 1] : (b[k] ? d : kp.d[k]);
+                            kp.j[k] = b[k - 1] ? kp.j[k - 1] : (b[k] ? j : kp.j[k]);
+                        }
+                        kp.d[0] = b[0] ? d : kp.d[0];
+                        kp.j[0] = b[0] ? j : kp.j[0];
+                    }
                 }
             }
     }
@@ -394,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, (kMinCtas<T, DP, Q>))
     for (int q = 0; q < Q; ++q) {
         const T bd = sh.bd[q];
 #pragma unroll
-        for (int k = 0; k < kKeep; ++k)
+        for (int k = 0; k < K; ++k)
             if (kept[q].j[k] >= 0 && kept[q].d[k] <= bd) sh.push(q, kept[q].d[k], kept[q].j[k]);
         if (kept[q].dropped(bd, INT32_MAX)) more |= 1u << q;
     }
@@ -404,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, (kMinCtas<T, DP, Q>))
 #pragma unroll
     for (int q = 0; q < Q; ++q) todo |= sh.count[q] > kLong ? 1u << q : 0u;
     if (todo) {
-        Kept<T> mine[Q];  // copies, so that only these are in memory
+        Kept<T, K> mine[Q];  // copies, so that only these are in memory
         int lims[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -438,8 +457,8 @@ cudaError_t launch(const T *refs, int64_t n_ref, const T *qs, int64_t n_query, i
         knn_direct_kernel<T, DP, 4, 1><<<(unsigned)((n_query + 3) / 4), kThreads, 0, stream>>>(
             refs, qs, n_query, n_ref, dp, has_cut, cut, m, out);
     else
-        knn_direct_kernel<T, DP, 1, 4><<<(unsigned)n_query, kThreads, 0, stream>>>(refs, qs, n_query, n_ref, dp, has_cut,
-                                                                                 cut, m, out);
+        knn_direct_kernel<T, DP, 1, 4><<<(unsigned)n_query, kThreads, 0, stream>>>(refs, qs, n_query, n_ref, dp,
+                                                                                 has_cut, cut, m, out);
     return cudaGetLastError();
 }
 
@@ -448,7 +467,7 @@ cudaError_t launch(const T *refs, int64_t n_ref, const T *qs, int64_t n_query, i
 template <typename T>
 nngp_status search(const T *refs, int64_t n_ref, const T *qs, int64_t n_query, int d, int m, int has_cut, int64_t cut,
                    int32_t *out, cudaStream_t stream) {
-    static_assert(kMaxNeighbours <= kCap && kMaxNeighbours <= kThreads, "the bound needs m thread minima");
+    static_assert(kMaxNeighbours <= kLong && kMaxNeighbours <= kThreads, "the bound needs m thread minima");
     if (m < 1 || m > kMaxNeighbours || n_ref < 1 || n_query < 1)
         return fail(NNGP_ERR_UNSUPPORTED, "knn: shape outside the direct search");
     const int dp = row_len(d);
