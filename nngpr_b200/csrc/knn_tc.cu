@@ -326,42 +326,63 @@ __device__ __forceinline__ bool warp_poll(int lane, const uint32_t *p, uint64_t 
 }
 
 // A row's m best so far, unordered: distances d[0 .. 31] (slots >= m: -inf), the largest of each four at
-// d[32 .. 39], indices, and the slot of the largest (distance, index).  Replaces that slot by (x, j) when (x, j)
-// is the smaller and finds the new largest through the four-maxima: about 50 instructions, the same in every
-// lane.  A binary heap's sift-down is five dependent steps whose lanes part (one search, n = 1M, d = 16
-// clustered: 33.3 ms with heaps, 32.1 sweeping all 32 slots, 30.1 with the four-maxima).  Returns the largest distance.
+// d[32 .. 39], indices, and a word: the slot of the largest (distance, index) in bits 0 .. 4, whether the list has held an
+// infinite distance in bit 5, and in bits 8 .. 23 the place of the largest in each group of four.  Replaces the
+// largest by (x, j) when (x, j) is the smaller and finds the new one through its group and the four-maxima: about
+// 50 instructions, the same in every lane.  A binary heap's sift-down is five dependent steps whose lanes part (one
+// search, n = 1M, d = 16 clustered: 33.3 ms with heaps, 32.1 sweeping all 32 slots, 30.1 with the four-maxima).
+// Equal distances cost up to 11 index reads, of the group and of the groups that share the maximum (without the places
+// up to 32: 5^3 places of 50,000 points 2.15 -> 1.40 ms, heaps 1.61; 20^4 grid 10.0 -> 6.5, heaps 6.5).  AT_ONCE: the
+// groups' indices are read together (1.53 and 7.05 ms one after the other); at d = 24 that spills (n = 300,000 8.6 ->
+// 9.4 ms).  Returns the largest distance.
+template <bool AT_ONCE>
 __device__ __forceinline__ float list_insert(float *d, uint32_t *idx, int32_t *largest, float x, uint32_t j) {
-    const int state = *largest, at = state & 31;  // bit 5: the list has held an infinite distance
+    uint32_t state = (uint32_t)*largest;
+    const int at = state & 31u, own_g = at >> 2;
     const float top = d[at];
     if (!(x < top || (x == top && j < idx[at]))) return top;
     d[at] = x;
     idx[at] = j;
+    if (!(x < pos_inf<float>())) state |= 32u;
+    const bool held_inf = (state & 32u) != 0u;  // else infinite distances are empty slots, of which any will do
     float4 *d4 = reinterpret_cast<float4 *>(d);
-    const float4 own = d4[at >> 2];
-    d[32 + (at >> 2)] = fmaxf(fmaxf(own.x, own.y), fmaxf(own.z, own.w));
+    const float4 own = d4[own_g];
+    const float gm = fmaxf(fmaxf(own.x, own.y), fmaxf(own.z, own.w));
+    d[32 + own_g] = gm;
+    uint32_t eq = (own.x == gm ? 1u : 0u) | (own.y == gm ? 2u : 0u) | (own.z == gm ? 4u : 0u) | (own.w == gm ? 8u : 0u);
+    uint32_t place = (uint32_t)__ffs((int)eq) - 1u;
+    eq &= eq - 1u;
+    if (eq != 0u && (gm < pos_inf<float>() || held_inf)) {  // equal distances: the largest index goes first
+        for (; eq; eq &= eq - 1u) {
+            const uint32_t k = (uint32_t)__ffs((int)eq) - 1u;
+            if (idx[4 * own_g + k] > idx[4 * own_g + place]) place = k;
+        }
+    }
+    state = (state & ~(3u << (8 + 2 * own_g))) | place << (8 + 2 * own_g);
     const float4 a = d4[8], b = d4[9];
     const float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
     uint32_t fours = (a.x == mx ? 1u : 0u) | (a.y == mx ? 2u : 0u) | (a.z == mx ? 4u : 0u) | (a.w == mx ? 8u : 0u) |
                      (b.x == mx ? 16u : 0u) | (b.y == mx ? 32u : 0u) | (b.z == mx ? 64u : 0u) | (b.w == mx ? 128u : 0u);
-    auto equal_in = [&](int g) {
-        const float4 t = d4[g];
-        return (t.x == mx ? 1u : 0u) | (t.y == mx ? 2u : 0u) | (t.z == mx ? 4u : 0u) | (t.w == mx ? 8u : 0u);
-    };
-    int g = __ffs((int)fours) - 1;
-    uint32_t eq = equal_in(g);
-    int pos = 4 * g + __ffs((int)eq) - 1;
-    const int held_inf = (state & 32) | (x < pos_inf<float>() ? 0 : 32);
-    // (any of the empty slots will do while there are some and nothing else is infinite)
-    if (((fours & (fours - 1)) | (eq & (eq - 1))) != 0u && (mx < pos_inf<float>() || held_inf)) {
-        for (; fours; fours &= fours - 1) {  // equal distances: the largest index goes first
-            g = __ffs((int)fours) - 1;
-            for (eq = equal_in(g); eq; eq &= eq - 1) {
-                const int k = 4 * g + __ffs((int)eq) - 1;
+    auto slot_of = [&](uint32_t g) -> uint32_t { return 4u * g + ((state >> (8 + 2 * g)) & 3u); };
+    uint32_t pos = slot_of((uint32_t)__ffs((int)fours) - 1u);
+    if ((fours & (fours - 1u)) != 0u && (mx < pos_inf<float>() || held_inf)) {
+        if constexpr (AT_ONCE) {
+            uint32_t best = 0u;
+#pragma unroll
+            for (uint32_t g = 0; g < 8; ++g) {
+                const uint32_t k = slot_of(g), v = idx[k];
+                const bool take = ((fours >> g) & 1u) != 0u && v >= best;
+                best = take ? v : best;
+                pos = take ? k : pos;
+            }
+        } else {
+            for (fours &= fours - 1u; fours; fours &= fours - 1u) {
+                const uint32_t k = slot_of((uint32_t)__ffs((int)fours) - 1u);
                 if (idx[k] > idx[pos]) pos = k;
             }
         }
     }
-    *largest = pos | held_inf;
+    *largest = (int32_t)((state & ~31u) | pos);
     return mx;
 }
 
@@ -504,7 +525,7 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
     float *row_norm = row_worst + C::ROWS, *row_eps = row_norm + C::ROWS;
     int32_t *row_limit = reinterpret_cast<int32_t *>(row_eps + C::ROWS);
     int32_t *row_point = row_limit + C::ROWS;            // -1: past the item's rows
-    int32_t *row_largest = row_point + C::ROWS;          // slot of its list's largest entry (list_insert)
+    int32_t *row_largest = row_point + C::ROWS;          // its list's largest entries (list_insert)
     uint64_t *bars = reinterpret_cast<uint64_t *>(row_largest + C::ROWS);
     static_assert((C::LIST_BYTES + C::A_BYTES) % 16 == 0 && (C::RING_BYTES + C::ROW_BYTES) % 8 == 0, "alignment");
     uint64_t *b_full = bars;                    // [S <= MAX_STAGES]
@@ -1038,7 +1059,8 @@ __global__ void __launch_bounds__(Cfg<D, QTILES>::THREADS, Cfg<D, QTILES>::CTAS_
                     while (todo) {
                         const unsigned grp = same_row & todo;
                         if (keep && (grp & (0u - grp)) == (1u << lane)) {
-                            const float top = list_insert(list_d + slot * DS, list_i + slot * IS, row_largest + slot, d2, jk);
+                            const float top = list_insert<(D < 24)>(list_d + slot * DS, list_i + slot * IS,
+                                                                    row_largest + slot, d2, jk);
                             if (top < row_worst[slot]) {
                                 row_worst[slot] = top;
                                 *reinterpret_cast<volatile float *>(row_thr + slot) = fminf((top - nq) + eps, pos_inf<float>());
