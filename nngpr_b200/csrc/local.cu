@@ -349,6 +349,13 @@ nngp_status resident_ctas(const void *fn, int threads, size_t smem, int *out) {
 }
 }  // namespace
 
+int rows_per_lane(int M, int d, int64_t n_points, bool f32, bool pred) {
+    if (M == 64) return 2;
+    if (n_points <= (int64_t)num_sms() * (M == 32 ? 7 : 22)) return 1;
+    const int bytes = d * (f32 && !pred ? 4 : 8);  // of a row (predict re-solves in FP64 in place)
+    return bytes >= (M == 16 || (pred && !f32) ? 224 : 288) ? 1 : 2;
+}
+
 nngp_status warp_launch(const void *fn, size_t warp_bytes, int64_t need_warps, int grid_limit, WarpLaunch *out) {
     if (warp_bytes > block_smem_limit())
         return fail(NNGP_ERR_UNSUPPORTED, "the local systems of this d and m need more shared memory than one CTA has");

@@ -14,7 +14,7 @@ nngp_status launch_redo(const LocalArgs &a, bool grad, const float *x_ref, const
                    : (grad ? local_redo_kernel<R, true, true> : local_redo_kernel<R, false, true>);
     };
     auto fn = M == 16 ? pick(std::integral_constant<int, 16>{}) : pick(std::integral_constant<int, 32>{});
-    const size_t bytes = WarpLayout::make<false, true>(M, a.d, a.n_theta, grad, grad && rbf, grad && a.ard).total;
+    const size_t bytes = WarpLayout::make<false, true>(M, 2, a.d, a.n_theta, grad, grad && rbf, grad && a.ard).total;
     WarpLaunch w;
     nngp_status st = warp_launch(reinterpret_cast<const void *>(fn), bytes, (a.n_points + 31) / 32, grid_limit, &w);
     if (st != NNGP_OK) return st;

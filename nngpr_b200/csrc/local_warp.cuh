@@ -1,19 +1,19 @@
 // Local systems of up to 64 neighbours: 32 / LPP points per warp, LPP lanes per point (local.cu
 // has the mathematics).
 //
-// Lane `sub` of a point's group owns the rows c * LPP + sub, c = 0, 1 (two rows per lane), of the
+// Lane `sub` of a point's group owns the rows c * LPP + sub, c = 0 .. C - 1 (C = M / LPP), of the
 // neighbour block, row i up to column (c + 1) * LPP - 1: with the rows of one class c equally long,
 // every loop bound is a compile-time constant and only the diagonal LPP x LPP blocks hold
 // entries above the diagonal.  M is the neighbour count rounded up to 16, 32 or 64; rows past it and
 // missing neighbours are identity rows.
 //
-// LPP is M / 2: one, two or four points per warp.  Why several
-// points per warp: with one row per lane a lane computes whole rows of a symmetric matrix, twice
-// the fill's and three times the factor's work, and the chain of each column (two shuffles, a
-// reciprocal square root, a trip through shared memory) is paid per point.  At M = 32 a warp issues 24
-// fill entries per point instead of 32 and 308 factor FMAs instead of 496, and one chain serves two
-// points.  Every value is formed by the same operations in the same order as with one row per
-// lane (sums over the rows by the same butterfly tree), so FP32 systems give the same bits.
+// LPP is M / 2, two rows per lane and one, two or four points per warp, or M, one row per lane (few
+// points, many features: rows_per_lane).  Why two rows: with one row per lane a lane computes whole
+// rows of a symmetric matrix, twice the fill's and three times the factor's work, and the chain of
+// each column (two shuffles, a reciprocal square root, a trip through shared memory) is paid per
+// point.  At M = 32 a warp issues 24 fill entries per point instead of 32 and 308 factor FMAs instead
+// of 496, and one chain serves two points.  Every value is formed by the same operations in the same
+// order with either (sums over the rows by the same butterfly tree), so FP32 systems give the same bits.
 //
 // Bound by latency: about 3,400 (FP32) and 4,500 (FP64) instructions per point at 2.5 to 3 warps per
 // scheduler, each waiting for fixed-latency chains, shared-memory round trips and the gather.
@@ -55,8 +55,8 @@ template <> struct Vec16<float> {
     __device__ static float4 make(const float *p) { return make_float4(p[0], p[1], p[2], p[3]); }
 };
 
-// Lanes per point of the systems with M rows: two rows per lane
-__host__ __device__ constexpr int lanes_per_point(int M) { return M / 2; }
+// C: rows per lane (1 or 2).  Lanes per point of the systems with M rows.
+__host__ __device__ constexpr int lanes_per_point(int M, int C) { return M / C; }
 
 // Resident CTAs (of two warps) per SM the registers are budgeted for: FP32 and the 16-row systems 168
 // registers, 12 warps per SM; the 32- and 64-row FP64 ones are held to 8 and 5 warps by shared memory, so
@@ -96,8 +96,9 @@ struct PtLayout {
 // both precisions), then one gradient accumulator per group.
 struct WarpLayout {
     size_t g, total;
-    template <bool F32, bool F64> __host__ __device__ static WarpLayout make(int M, int d, int n_theta, bool grad, bool keep_e, bool keep_x) {
-        const int groups = 32 / lanes_per_point(M);
+    template <bool F32, bool F64>
+    __host__ __device__ static WarpLayout make(int M, int C, int d, int n_theta, bool grad, bool keep_e, bool keep_x) {
+        const int groups = 32 / lanes_per_point(M, C);
         size_t b = 0;
         if (F32) b = groups * PtLayout::make<float>(M, d, grad, keep_e, keep_x).total;
         if (F64) {
@@ -114,14 +115,14 @@ struct WarpLayout {
 // Solves the system of point p for each group of LPP lanes (p < 0: the group has none; it runs along).
 // Returns false (and commits nothing) for the groups whose FP32 system has a pivot below the FP64
 // threshold.  ll_acc: the group's sum, held by its first lane; gacc: the group's gradient sums.
-template <typename TC, typename TIn, int M, bool GRAD, bool PRED, bool MATERN>
+template <typename TC, typename TIn, int M, int C, bool GRAD, bool PRED, bool MATERN>
 __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p, const int lane,
                                              const TIn *__restrict__ x_ref, const TIn *__restrict__ y_ref,
                                              const TIn *__restrict__ x_pt, const TIn *__restrict__ y_pt,
                                              const int32_t *__restrict__ nbr, unsigned char *wsm, double *gacc,
                                              double &ll_acc, TIn *__restrict__ mean, TIn *__restrict__ var,
                                              int32_t *__restrict__ flags) {
-    constexpr int LPP = lanes_per_point(M), C = 2;  // C: rows per lane
+    constexpr int LPP = lanes_per_point(M, C);
     using V = Vec16<TC>;
     using VT = typename V::T;
     constexpr int EV = V::N;
@@ -150,15 +151,20 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
         for (int o = LPP / 2; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
         return v;
     };
-    auto rows_sum = [&](const TC (&w)[C]) -> TC { return lanes_sum(add_rn(w[0], w[1])); };
+    auto rows_sum = [&](const TC (&w)[C]) -> TC {
+        if constexpr (C == 2) return lanes_sum(add_rn(w[0], w[1]));
+        else return lanes_sum(w[0]);
+    };
     // f(dc, k0) for every 4 columns k0 .. k0 + 3 of the lower triangle: dc is the class of their rows'
     // diagonal block (a constant once inlined), the rows of the classes c >= dc reach them.  Loops,
     // not unrolled code: a kernel of 4,000 straight instructions waits for its instructions.
     auto for_columns = [&](auto &&f) {
 #pragma unroll 1
         for (int k0 = 0; k0 < LPP; k0 += 4) f(0, k0);
+        if constexpr (C > 1) {
 #pragma unroll 1
-        for (int k0 = LPP; k0 < 2 * LPP; k0 += 4) f(1, k0);
+            for (int k0 = LPP; k0 < 2 * LPP; k0 += 4) f(1, k0);
+        }
     };
     auto store4 = [&](TC *at, const TC (&w)[4]) {
 #pragma unroll
@@ -397,7 +403,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
         }
     };
     factor_block(0);
-    factor_block(1);
+    if constexpr (C > 1) factor_block(1);
     const TC s2 = kpp - ss;
     bool ok = true;
     if constexpr (std::is_same<TC, float>::value)
@@ -422,7 +428,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
             for (int u = 3; u >= 0; --u) {
                 const int k = k0 + u;
                 auto step = [&](TC(&b)[C]) {
-                    const TC bc = k0 < LPP ? b[0] : b[1];
+                    const TC bc = k0 < LPP ? b[0] : b[C - 1];
                     const TC bk = __shfl_sync(FULL, bc, k & (LPP - 1), LPP) * iv[u];
 #pragma unroll
                     for (int c = 0; c < C; ++c)
@@ -463,7 +469,7 @@ __device__ __forceinline__ bool solve_points(const LocalArgs &a, const int64_t p
             for (int c = 0; c < C; ++c) yv[c] = valid[c] ? (TC)y_ref[(int64_t)j[c] * a.ydim + o] : TC(0);
 #pragma unroll 4
             for (int k = 0; k < M; ++k) {
-                const TC yc = k < LPP ? yv[0] : yv[1];
+                const TC yc = k < LPP ? yv[0] : yv[C - 1];
                 const TC zk = __shfl_sync(FULL, yc, k & (LPP - 1), LPP) * idg[k];
 #pragma unroll
                 for (int c = 0; c < C; ++c)
@@ -642,7 +648,7 @@ __device__ __forceinline__ void write_partials(const LocalArgs &a, bool grad, co
 
 // The fit step (PRED false) and predict.  Fit-step systems of FP32 inputs that need FP64 are marked
 // for local_redo_kernel; predict solves them in place.
-template <typename TIn, int M, bool GRAD, bool PRED, bool MATERN>
+template <typename TIn, int M, int C, bool GRAD, bool PRED, bool MATERN>
 __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_kernel(const __grid_constant__ LocalArgs a,
                                                          const TIn *__restrict__ x_ref, const TIn *__restrict__ y_ref,
                                                          const TIn *__restrict__ x_pt, const TIn *__restrict__ y_pt,
@@ -652,8 +658,8 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_k
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using T1 = typename std::conditional<(M > 32), double, TIn>::type;  // the first attempt's precision
     constexpr bool F32 = std::is_same<T1, float>::value;
-    constexpr int LPP = lanes_per_point(M), GROUPS = 32 / LPP;
-    const WarpLayout lay = WarpLayout::make<F32, !F32 || PRED>(M, a.d, a.n_theta, GRAD,
+    constexpr int LPP = lanes_per_point(M, C), GROUPS = 32 / LPP;
+    const WarpLayout lay = WarpLayout::make<F32, !F32 || PRED>(M, C, a.d, a.n_theta, GRAD,
                                                               GRAD && !MATERN && M <= 32, GRAD && a.ard);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int sub = lane & (LPP - 1), grp = lane / LPP;
@@ -666,7 +672,7 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_k
     const int64_t step = (int64_t)gridDim.x * warps * GROUPS;
     for (int64_t p0 = ((int64_t)blockIdx.x * warps + warp) * GROUPS; p0 < a.n_points; p0 += step) {
         const int64_t p = p0 + grp < a.n_points ? p0 + grp : -1;
-        const bool ok = solve_points<T1, TIn, M, GRAD, PRED, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm,
+        const bool ok = solve_points<T1, TIn, M, C, GRAD, PRED, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm,
                                                                      gacc, ll_acc, mean, var, flags);
         if constexpr (F32) {
             const bool bad = p >= 0 && !ok;
@@ -675,7 +681,7 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<TIn, M, PRED>)) local_warp_k
                 if (bad && sub == 0) atomicOr(a.redo_bits + (p >> 5), 1u << (p & 31));
             } else {
                 if (__any_sync(0xffffffffu, bad))
-                    solve_points<double, TIn, M, GRAD, PRED, MATERN>(a, bad ? p : -1, lane, x_ref, y_ref, x_pt, y_pt,
+                    solve_points<double, TIn, M, C, GRAD, PRED, MATERN>(a, bad ? p : -1, lane, x_ref, y_ref, x_pt, y_pt,
                                                                      nbr, wsm, gacc, ll_acc, mean, var, flags);
             }
         }
@@ -698,8 +704,8 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<double, M, false>)) local_re
                                                          const int32_t *__restrict__ nbr,
                                                          double *__restrict__ block_out, int32_t *__restrict__ flags) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int LPP = lanes_per_point(M), GROUPS = 32 / LPP;
-    const WarpLayout lay = WarpLayout::make<false, true>(M, a.d, a.n_theta, GRAD,
+    constexpr int C = 2, LPP = lanes_per_point(M, C), GROUPS = 32 / LPP;
+    const WarpLayout lay = WarpLayout::make<false, true>(M, C, a.d, a.n_theta, GRAD,
                                                         GRAD && !MATERN && M <= 32, GRAD && a.ard);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int sub = lane & (LPP - 1), grp = lane / LPP;
@@ -717,7 +723,7 @@ __global__ void __launch_bounds__(64, (kWarpMinCtas<double, M, false>)) local_re
                 if (g == grp) p = w * 32 + (__ffs(bits) - 1);
                 bits &= bits - 1;
             }
-            solve_points<double, float, M, GRAD, false, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm, gacc,
+            solve_points<double, float, M, C, GRAD, false, MATERN>(a, p, lane, x_ref, y_ref, x_pt, y_pt, nbr, wsm, gacc,
                                                                 ll_acc, static_cast<float *>(nullptr),
                                                                 static_cast<float *>(nullptr), flags);
         }
@@ -736,6 +742,18 @@ struct WarpLaunch {
 nngp_status warp_launch(const void *fn, size_t warp_bytes, int64_t need_warps, int grid_limit, WarpLaunch *out);
 
 inline int warp_rows(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : 64); }
+
+// Rows per lane of a launch: two, or one
+//   * for few points, where the length of a warp's program is the time: up to 7 points per SM at M = 32, 22 at M = 16,
+//     which one-row warps do in one wave (one against two, us: FP64 d = 18, m = 32 log-likelihood of 300 points
+//     25.5 / 31.5, of 1,000 28.7 / 30.9, of 1,200 39.9 / 33.8; FP32 d = 28 with gradient of 1,000 36.6 / 41.0; FP64
+//     d = 18, m = 16 log-likelihood of 3,300 24.6 / 28.6, of 4,000 32.8 / 28.8; FP64 gradients at m <= 16 gain nothing
+//     from 2,400 points on and lose up to 8 %);
+//   * for long rows, whose coordinates leave shared memory for few warps, so that a warp should hold few points: FP64
+//     log-likelihood of 30,000 points, m = 32, d = 128 2,049 / 3,413, d = 40 602 / 671, d = 28 496 / 469; FP32 with
+//     gradient d = 128 820 / 1,046, d = 64 1.04 times slower; m = 8 FP64 predict d = 28 0.86 of the time, d = 18 equal.
+// M = 64 has two.
+int rows_per_lane(int M, int d, int64_t n_points, bool f32, bool pred);
 
 // *parts: CTAs of the launch (the partial sums in block_out)
 template <typename TIn>
